@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "mg_common.cuh"
 #include "pdl.cuh"
 #include "pfgpu_kernels.h"
 
@@ -113,31 +114,6 @@ __device__ __forceinline__ void split_ijk(int t, int nx, int ny, int &i, int &j,
   j = r % ny;
   k = r / ny;
 }
-// A divisor with its float reciprocal: t / d from one multiplication and a
-// one-step correction (exact while the float product errs by less than one,
-// i.e. for t < 2^22; larger t take the integer division).  The single-block
-// tail splits a linear index per cell and phase, where integer division
-// would dominate its instruction count.
-struct FastDiv {
-  int d;
-  float inv;
-};
-__device__ __forceinline__ FastDiv fast_div(int d) { return FastDiv{d, 1.0f / (float)d}; }
-__device__ __forceinline__ int quot(int t, FastDiv f) {
-  if (t >= (1 << 22)) return t / f.d;
-  int q = (int)((float)t * f.inv);
-  if ((q + 1) * f.d <= t) q++;
-  if (q * f.d > t) q--;
-  return q;
-}
-__device__ __forceinline__ void split_ijk(int t, FastDiv fx, FastDiv fy, int &i, int &j,
-                                          int &k) {
-  const int r = quot(t, fx);
-  i = t - r * fx.d;
-  k = quot(r, fy);
-  j = r - k * fy.d;
-}
-
 // prolongation weights of one fine point (mg_semi.c:534-575): the
 // along-direction entries over the collapsed diagonal
 template <typename T>
@@ -286,17 +262,6 @@ template <typename T>
 constexpr bool kHasH16 = std::is_same<T, float>::value;
 
 // ---- scaled FP16 operator helpers (H mode) --------------------------------
-// 1/S for S = sqrt(|c|), 1 where c is 0 or not finite (hardware reciprocal
-// square root: the scaled values are stored as 11-bit FP16 significands)
-__device__ __forceinline__ float inv_scale_of(float c) {
-  const float a = fabsf(c);
-  return (a > 0.0f && isfinite(a)) ? rsqrtf(a) : 1.0f;
-}
-// S from c and 1/S without a division
-__device__ __forceinline__ float scale_from(float c, float inv) {
-  const float a = fabsf(c);
-  return (a > 0.0f && isfinite(a)) ? a * inv : 1.0f;
-}
 // scaled operator of fine cell c: off-diagonals E N U over S_c S_nb (a0 of
 // the +x, +y, +z neighbours, ignored where has_* is false), the diagonal
 // C / S^2 (raising *hflag when it is not +1) and, on level 0, 1/S; returns 1/S
@@ -346,12 +311,17 @@ __device__ __forceinline__ void gather7(const LV<T> &L, int i, int j, int k, T s
 // q1(2c+1), q2(2c-1) (all against its own coarse diagonal; q2(2c+1) comes
 // from the thread of c+1, or is 0 on the last coarse point), exactly as
 // h16_scale_cell computes them; the plain weights p1/p2 are not stored then.
+//
+// L holds the fine operator (F's own, or a copy of it in shared memory); the
+// coarse entries are returned for the caller to store.
+template <typename T>
+struct CoarseRow {
+  T c, e, n, u;
+};
 template <typename T, int D, bool H>
-__global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C) {
-  pdl_enter();
-  int ic, jc, kc;
-  thread_ijk(ic, jc, kc);
-  if (ic >= C.nx || jc >= C.ny || kc >= C.nz) return;
+__device__ __forceinline__ CoarseRow<T> setup_point(const LV<T> &L, const MGLevel<T> &F,
+                                                    const MGLevel<T> &C, int ic, int jc,
+                                                    int kc) {
   constexpr int ox = D == 0, oy = D == 1, oz = D == 2;
   constexpr int s0 = D == 0 ? 0 : D == 1 ? 0 : 0;
   constexpr int s1 = D == 0 ? 1 : D == 1 ? 3 : 5;  // along-D lower
@@ -361,7 +331,6 @@ __global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C)
   constexpr int s5 = D == 0 ? 5 : D == 1 ? 5 : 1;
   constexpr int s6 = D == 0 ? 6 : D == 1 ? 6 : 2;
   const int i = ox ? 2 * ic : ic, j = oy ? 2 * jc : jc, k = oz ? 2 * kc : kc;
-  LV<T> L = lv(F);
   T sm[7], sc[7], sp[7];  // fine cells f-1, f, f+1 along D
   gather7(L, i - ox, j - oy, k - oz, sm);
   gather7(L, i, j, k, sc);
@@ -387,7 +356,6 @@ __global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C)
     F.p2[f] = p2_2;
   }
   // coarse operator: coarse_op_core
-  const long long cc = ic + (long long)C.nx * (jc + (long long)C.ny * kc);
   const T ac3 = sc[s3] + T(0.5) * sm[s3] + T(0.5) * sp[s3];
   const T ac4 = sc[s4] + T(0.5) * sm[s4] + T(0.5) * sp[s4];
   const T ac5 = sc[s5] + T(0.5) * sm[s5] + T(0.5) * sp[s5];
@@ -401,17 +369,13 @@ __global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C)
   if (D == 0) { E = along_up; N = ac4; U = ac6; }
   else if (D == 1) { E = ac4; N = along_up; U = ac6; }
   else { E = ac6; N = ac4; U = along_up; }
-  C.a[1][cc] = E;
-  C.a[2][cc] = N;
-  C.a[3][cc] = U;
   const T cdiag = ac0 - (ac3 + ac4 + ac5 + ac6);
-  C.a[0][cc] = cdiag;
   // coarse ghost column (see coarse_op_core)
   if (ic == 0 && C.wg) C.wg[jc + C.ny * kc] = D == 1 ? ac3 : D == 2 ? ac5 : T(0);
   if constexpr (H) {
     const int nx = F.nx, ny = F.ny, nz = F.nz;
     const int sy = nx, sz = nx * ny;
-    const float *a0 = F.a[0];
+    const float *a0 = L.a0;
     const float ics = inv_scale_of(cdiag);
     // fine point 2c
     const int f0 = i + sy * j + sz * k;
@@ -440,6 +404,21 @@ __global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C)
       if (last) F.q2[f1] = 0.0f;
     }
   }
+  return CoarseRow<T>{cdiag, E, N, U};
+}
+
+template <typename T, int D, bool H>
+__global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C) {
+  pdl_enter();
+  int ic, jc, kc;
+  thread_ijk(ic, jc, kc);
+  if (ic >= C.nx || jc >= C.ny || kc >= C.nz) return;
+  const CoarseRow<T> r = setup_point<T, D, H>(lv(F), F, C, ic, jc, kc);
+  const long long cc = ic + (long long)C.nx * (jc + (long long)C.ny * kc);
+  C.a[0][cc] = r.c;
+  C.a[1][cc] = r.e;
+  C.a[2][cc] = r.n;
+  C.a[3][cc] = r.u;
 }
 
 template <typename T>
@@ -497,11 +476,17 @@ __device__ __forceinline__ float ldro_h(const __half *p) {
 // division.  Every array the sweep reads is read-only for the launch (it
 // writes one colour and reads only the other), so all loads take the
 // read-only data path.  Bitwise the same result as rb_cell.
-template <typename T, bool H>
+// EARLY: the operator, and b when b_early says that the kernel before this one
+// does not write it, are loaded ahead of the wait on that kernel.  On levels
+// whose blocks are all resident at once a sweep is a launch latency, and the
+// loads drop out of it (V-cycle of 64x64x32 in FP64: 103 us against 117); on
+// larger levels the loads kept in registers cost more than they hide (colour
+// sweep of 512x512x50, scaled FP16: 47 us against 31).
+template <typename T, bool H, bool EARLY>
 __global__ void __launch_bounds__(256) k_rb_sweep(MGLevel<T> L, T *__restrict__ x,
                                                   const T *__restrict__ b, int colour, int init,
-                                                  int flip) {
-  pdl_enter();
+                                                  int flip, int b_early) {
+  if (!EARLY) pdl_enter();
   const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = by * blockDim.y + threadIdx.y;
@@ -533,6 +518,7 @@ __global__ void __launch_bounds__(256) k_rb_sweep(MGLevel<T> L, T *__restrict__ 
     d = ldro(L.a[0] + c);
   }
   if (init) {
+    if (EARLY) pdl_enter();
     x[xo] = unit ? ldro(b + xo) : ldro(b + xo) / d;
     return;
   }
@@ -554,6 +540,8 @@ __global__ void __launch_bounds__(256) k_rb_sweep(MGLevel<T> L, T *__restrict__ 
     cl = hl ? ldro(L.a[3] + c - sz) : T(0);
     cu = ldro(L.a[3] + c);
   }
+  T bc = EARLY && b_early ? ldro(b + xo) : T(0);
+  if (EARLY) pdl_enter();
   const T *xr = x;  // the other colour: not written by this launch
   T acc = cw * (hw ? ldro(xr + xw) : T(0));
   acc = fma(ce, he ? ldro(xr + xe) : T(0), acc);
@@ -561,7 +549,7 @@ __global__ void __launch_bounds__(256) k_rb_sweep(MGLevel<T> L, T *__restrict__ 
   acc = fma(cn, hn ? ldro(xr + xn) : T(0), acc);
   acc = fma(cl, hl ? ldro(xr + xl) : T(0), acc);
   acc = fma(cu, hu ? ldro(xr + xu) : T(0), acc);
-  const T bc = ldro(b + xo);
+  if (!EARLY || !b_early) bc = ldro(b + xo);
   x[xo] = unit ? bc - acc : (bc - acc) / d;
 }
 
@@ -573,11 +561,11 @@ __global__ void __launch_bounds__(256) k_rb_sweep(MGLevel<T> L, T *__restrict__ 
 // from_b: the sweep that follows a zero-guess red sweep reads the red values
 // that sweep would have written, b / a0, straight from b (and the diagonal),
 // so the zero-guess sweep itself is not launched
-template <typename T, bool H, bool FROM_B = false>
+template <typename T, bool H, bool FROM_B, bool EARLY>
 __global__ void __launch_bounds__(256) k_rb_sweep2(MGLevel<T> L, T *__restrict__ x,
                                                    const T *__restrict__ b, int colour,
-                                                   int init, int flip) {
-  pdl_enter();
+                                                   int flip, int b_early) {
+  if (!EARLY) pdl_enter();
   const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   const int q0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int j = by * blockDim.y + threadIdx.y;
@@ -606,11 +594,6 @@ __global__ void __launch_bounds__(256) k_rb_sweep2(MGLevel<T> L, T *__restrict__
     d0 = ldro(L.a[0] + c0);
     if (two) d1 = ldro(L.a[0] + c1);
   }
-  if (init) {
-    x[xo] = unit ? ldro(b + xo) : ldro(b + xo) / d0;
-    if (two) x[xo + 1] = unit ? ldro(b + xo + 1) : ldro(b + xo + 1) / d1;
-    return;
-  }
   const bool hw = i0 > 0, he0 = i0 + 1 < nx, he1 = i0 + 3 < nx, hsj = j > 0, hn = j + 1 < ny,
              hl = k > 0, hu = k + 1 < nz;
   auto coef = [&](int s, int c) -> T {  // E / N / U entry s of cell c
@@ -619,6 +602,25 @@ __global__ void __launch_bounds__(256) k_rb_sweep2(MGLevel<T> L, T *__restrict__
     else
       return ldro(L.a[s + 1] + c);
   };
+  // w e s n l u of either cell (EARLY: loaded here, else where they are used)
+  auto row = [&](int c, bool w, T v[6]) {
+    v[0] = w ? coef(0, c - 1) : T(0);
+    v[1] = coef(0, c);
+    v[2] = hsj ? coef(1, c - sy) : T(0);
+    v[3] = coef(1, c);
+    v[4] = hl ? coef(2, c - sz) : T(0);
+    v[5] = coef(2, c);
+  };
+  T r0[6], r1[6], b0 = T(0), b1 = T(0);
+  if constexpr (EARLY) {
+    row(c0, hw, r0);
+    if (two) row(c1, true, r1);
+    if (b_early) {
+      b0 = ldro(b + xo);
+      if (two) b1 = ldro(b + xo + 1);
+    }
+    pdl_enter();
+  }
   const T *xr = x;  // the other colour: not written by this launch
   // the other colour's value at split index q (natural index cn)
   auto xv = [&](int q, int cn) -> T {
@@ -634,31 +636,27 @@ __global__ void __launch_bounds__(256) k_rb_sweep2(MGLevel<T> L, T *__restrict__
   };
   const T xm = he0 ? xv(ob + r, c0 + 1) : T(0);  // between the two cells
   {
-    const T cw = hw ? coef(0, c0 - 1) : T(0), ce = coef(0, c0);
-    const T cs = hsj ? coef(1, c0 - sy) : T(0), cn = coef(1, c0);
-    const T cl = hl ? coef(2, c0 - sz) : T(0), cu = coef(2, c0);
-    T acc = cw * (hw ? xv(ob - 1 + r, c0 - 1) : T(0));
-    acc = fma(ce, xm, acc);
-    acc = fma(cs, hsj ? xv(ob - hx, c0 - sy) : T(0), acc);
-    acc = fma(cn, hn ? xv(ob + hx, c0 + sy) : T(0), acc);
-    acc = fma(cl, hl ? xv(ob - hs, c0 - sz) : T(0), acc);
-    acc = fma(cu, hu ? xv(ob + hs, c0 + sz) : T(0), acc);
-    const T bc = ldro(b + xo);
-    x[xo] = unit ? bc - acc : (bc - acc) / d0;
+    if constexpr (!EARLY) row(c0, hw, r0);
+    T acc = r0[0] * (hw ? xv(ob - 1 + r, c0 - 1) : T(0));
+    acc = fma(r0[1], xm, acc);
+    acc = fma(r0[2], hsj ? xv(ob - hx, c0 - sy) : T(0), acc);
+    acc = fma(r0[3], hn ? xv(ob + hx, c0 + sy) : T(0), acc);
+    acc = fma(r0[4], hl ? xv(ob - hs, c0 - sz) : T(0), acc);
+    acc = fma(r0[5], hu ? xv(ob + hs, c0 + sz) : T(0), acc);
+    if (!EARLY || !b_early) b0 = ldro(b + xo);
+    x[xo] = unit ? b0 - acc : (b0 - acc) / d0;
   }
   if (two) {
     const int o1 = ob + 1;
-    const T cw = coef(0, c1 - 1), ce = coef(0, c1);
-    const T cs = hsj ? coef(1, c1 - sy) : T(0), cn = coef(1, c1);
-    const T cl = hl ? coef(2, c1 - sz) : T(0), cu = coef(2, c1);
-    T acc = cw * xm;
-    acc = fma(ce, he1 ? xv(o1 + r, c1 + 1) : T(0), acc);
-    acc = fma(cs, hsj ? xv(o1 - hx, c1 - sy) : T(0), acc);
-    acc = fma(cn, hn ? xv(o1 + hx, c1 + sy) : T(0), acc);
-    acc = fma(cl, hl ? xv(o1 - hs, c1 - sz) : T(0), acc);
-    acc = fma(cu, hu ? xv(o1 + hs, c1 + sz) : T(0), acc);
-    const T bc = ldro(b + xo + 1);
-    x[xo + 1] = unit ? bc - acc : (bc - acc) / d1;
+    if constexpr (!EARLY) row(c1, true, r1);
+    T acc = r1[0] * xm;
+    acc = fma(r1[1], he1 ? xv(o1 + r, c1 + 1) : T(0), acc);
+    acc = fma(r1[2], hsj ? xv(o1 - hx, c1 - sy) : T(0), acc);
+    acc = fma(r1[3], hn ? xv(o1 + hx, c1 + sy) : T(0), acc);
+    acc = fma(r1[4], hl ? xv(o1 - hs, c1 - sz) : T(0), acc);
+    acc = fma(r1[5], hu ? xv(o1 + hs, c1 + sz) : T(0), acc);
+    if (!EARLY || !b_early) b1 = ldro(b + xo + 1);
+    x[xo + 1] = unit ? b1 - acc : (b1 - acc) / d1;
   }
 }
 
@@ -720,64 +718,69 @@ __device__ __forceinline__ void mg_residual_cell(const MGLevel<T> &Lv, const T *
   const long long c = i + (long long)Lv.nx * (j + (long long)Lv.ny * k);
   const int nx = Lv.nx, ny = Lv.ny, nz = Lv.nz;
   LV<T> L = lv(Lv);
-  T y = -b[c];
-  y += diag<T, H>(L, c) * x[c];
-  y += coef<T, H>(L, 1, i, j, k) * vget(nx, ny, nz, x, i - 1, j, k);
-  y += coef<T, H>(L, 2, i, j, k) * vget(nx, ny, nz, x, i + 1, j, k);
-  y += coef<T, H>(L, 3, i, j, k) * vget(nx, ny, nz, x, i, j - 1, k);
-  y += coef<T, H>(L, 4, i, j, k) * vget(nx, ny, nz, x, i, j + 1, k);
-  y += coef<T, H>(L, 5, i, j, k) * vget(nx, ny, nz, x, i, j, k - 1);
-  y += coef<T, H>(L, 6, i, j, k) * vget(nx, ny, nz, x, i, j, k + 1);
-  r[c] = -y;
+  r[c] = residual_value<T>(
+      b[c], diag<T, H>(L, c), x[c], coef<T, H>(L, 1, i, j, k), vget(nx, ny, nz, x, i - 1, j, k),
+      coef<T, H>(L, 2, i, j, k), vget(nx, ny, nz, x, i + 1, j, k), coef<T, H>(L, 3, i, j, k),
+      vget(nx, ny, nz, x, i, j - 1, k), coef<T, H>(L, 4, i, j, k),
+      vget(nx, ny, nz, x, i, j + 1, k), coef<T, H>(L, 5, i, j, k),
+      vget(nx, ny, nz, x, i, j, k - 1), coef<T, H>(L, 6, i, j, k),
+      vget(nx, ny, nz, x, i, j, k + 1));
 }
 
-// grid form of mg_residual_cell (same operation order, lean indices)
-// r = b - A x of one cell (the grid residual kernels' shared arithmetic)
+// operator of one cell (zero towards missing lower neighbours), and the
+// residual r = b - A x there: the grid residual kernels' shared arithmetic
+template <typename T>
+struct PointOp {
+  T d, w, e, s, n, l, u;
+};
 template <typename T, bool H>
-__device__ __forceinline__ T mg_residual_cell(const MGLevel<T> &L, const T *__restrict__ x,
-                                              const T *__restrict__ b, int i, int j, int k) {
+__device__ __forceinline__ PointOp<T> point_op(const MGLevel<T> &L, int i, int j, int k) {
+  const int sy = L.nx, sz = L.nx * L.ny, c = i + sy * j + sz * k;
+  PointOp<T> p;
+  if constexpr (H) {
+    p.d = ldro(L.hflag) ? (T)ldro_h(L.h[3] + c) : T(1);
+    p.w = i > 0 ? (T)ldro_h(L.h[0] + c - 1) : T(0);
+    p.e = (T)ldro_h(L.h[0] + c);
+    p.s = j > 0 ? (T)ldro_h(L.h[1] + c - sy) : T(0);
+    p.n = (T)ldro_h(L.h[1] + c);
+    p.l = k > 0 ? (T)ldro_h(L.h[2] + c - sz) : T(0);
+    p.u = (T)ldro_h(L.h[2] + c);
+  } else {
+    p.d = ldro(L.a[0] + c);
+    p.w = i > 0 ? ldro(L.a[1] + c - 1) : T(0);
+    p.e = ldro(L.a[1] + c);
+    p.s = j > 0 ? ldro(L.a[2] + c - sy) : T(0);
+    p.n = ldro(L.a[2] + c);
+    p.l = k > 0 ? ldro(L.a[3] + c - sz) : T(0);
+    p.u = ldro(L.a[3] + c);
+  }
+  return p;
+}
+template <typename T>
+__device__ __forceinline__ T op_residual(const MGLevel<T> &L, const PointOp<T> &p,
+                                         const T *__restrict__ x, const T *__restrict__ b, int i,
+                                         int j, int k) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
-  const int sy = nx, sz = nx * ny;
-  const int c = i + sy * j + sz * k;
-  const bool hw = i > 0, he = i + 1 < nx, hs = j > 0, hn = j + 1 < ny, hl = k > 0,
-             hu = k + 1 < nz;
   int xo, xw, xe, xs, xn, xl, xu;  // x / b storage of the cell and its neighbours
   if (L.split) {
     const int hx = L.hx, hsl = hx * ny, half = hsl * nz;
-    const int p = (i + j + k) & 1, base = (i >> 1) + hx * j + hsl * k, r = i & 1;
-    xo = p * half + base;
-    const int ob = (p ^ 1) * half + base;
+    const int q = (i + j + k) & 1, base = (i >> 1) + hx * j + hsl * k, r = i & 1;
+    xo = q * half + base;
+    const int ob = (q ^ 1) * half + base;
     xw = ob - 1 + r; xe = ob + r; xs = ob - hx; xn = ob + hx; xl = ob - hsl; xu = ob + hsl;
   } else {
+    const int sy = nx, sz = nx * ny, c = i + sy * j + sz * k;
     xo = c; xw = c - 1; xe = c + 1; xs = c - sy; xn = c + sy; xl = c - sz; xu = c + sz;
   }
-  T d, cw, ce, cs, cn, cl, cu;
-  if constexpr (H) {
-    d = ldro(L.hflag) ? (T)ldro_h(L.h[3] + c) : T(1);
-    cw = hw ? (T)ldro_h(L.h[0] + c - 1) : T(0);
-    ce = (T)ldro_h(L.h[0] + c);
-    cs = hs ? (T)ldro_h(L.h[1] + c - sy) : T(0);
-    cn = (T)ldro_h(L.h[1] + c);
-    cl = hl ? (T)ldro_h(L.h[2] + c - sz) : T(0);
-    cu = (T)ldro_h(L.h[2] + c);
-  } else {
-    d = ldro(L.a[0] + c);
-    cw = hw ? ldro(L.a[1] + c - 1) : T(0);
-    ce = ldro(L.a[1] + c);
-    cs = hs ? ldro(L.a[2] + c - sy) : T(0);
-    cn = ldro(L.a[2] + c);
-    cl = hl ? ldro(L.a[3] + c - sz) : T(0);
-    cu = ldro(L.a[3] + c);
-  }
-  T y = -ldro(b + xo);
-  y += d * ldro(x + xo);
-  y += cw * (hw ? ldro(x + xw) : T(0));
-  y += ce * (he ? ldro(x + xe) : T(0));
-  y += cs * (hs ? ldro(x + xs) : T(0));
-  y += cn * (hn ? ldro(x + xn) : T(0));
-  y += cl * (hl ? ldro(x + xl) : T(0));
-  y += cu * (hu ? ldro(x + xu) : T(0));
-  return -y;
+  return residual_value<T>(ldro(b + xo), p.d, ldro(x + xo), p.w, i > 0 ? ldro(x + xw) : T(0), p.e,
+                           i + 1 < nx ? ldro(x + xe) : T(0), p.s, j > 0 ? ldro(x + xs) : T(0),
+                           p.n, j + 1 < ny ? ldro(x + xn) : T(0), p.l,
+                           k > 0 ? ldro(x + xl) : T(0), p.u, k + 1 < nz ? ldro(x + xu) : T(0));
+}
+template <typename T, bool H>
+__device__ __forceinline__ T point_residual(const MGLevel<T> &L, const T *__restrict__ x,
+                                            const T *__restrict__ b, int i, int j, int k) {
+  return op_residual<T>(L, point_op<T, H>(L, i, j, k), x, b, i, j, k);
 }
 
 template <typename T, bool H>
@@ -790,7 +793,7 @@ __global__ void __launch_bounds__(256) k_mg_residual(MGLevel<T> L, const T *__re
   const int j = by * blockDim.y + threadIdx.y;
   const int k = flip ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
   if (i >= L.nx || j >= L.ny) return;
-  r[i + L.nx * (j + L.ny * k)] = mg_residual_cell<T, H>(L, x, b, i, j, k);
+  r[i + L.nx * (j + L.ny * k)] = point_residual<T, H>(L, x, b, i, j, k);
 }
 
 // The residual right after a red/black sweep of colour zc: the cells of that
@@ -815,7 +818,72 @@ __global__ void __launch_bounds__(256) k_mg_residual_pair(MGLevel<T> L, const T 
   const int ic = iz == i0 ? i0 + 1 : i0;                     // the computed cell
   const int row = nx * (j + L.ny * k);
   if (iz < nx) r[iz + row] = T(0);
-  if (ic < nx) r[ic + row] = mg_residual_cell<T, H>(L, x, b, ic, j, k);
+  if (ic < nx) r[ic + row] = point_residual<T, H>(L, x, b, ic, j, k);
+}
+
+// Residual and restriction in one launch, right after a red/black sweep, on
+// levels where a launch costs more than its work.  The colour swept last
+// (parity zpar) was just solved against its current neighbours, so its
+// residual is taken as zero; and of a coarse point's three fine points f-1, f,
+// f+1 along D either f alone or f-1 and f+1 hold the other colour.  Every
+// thread evaluates a residual at f or f+1; the f-1 one comes from the
+// neighbouring lane (D = x) or is evaluated too (half the threads).  With the
+// operators loaded ahead of the wait a level's leg is one launch shorter: V-cycle
+// of 64x64x32 (FP64) 117 us against 123.  On the finest level of 512x512x50 the
+// second evaluation costs more than the stored residual: 107 us against 78.
+// init: the zero-guess red sweep x = b / a0 of the coarse level too.
+template <typename T, bool H, int D>
+__global__ void __launch_bounds__(256) k_resid_restrict(MGLevel<T> F, MGLevel<T> C,
+                                                        const T *__restrict__ x,
+                                                        const T *__restrict__ b,
+                                                        T *__restrict__ rc, T *__restrict__ xc,
+                                                        int flip, int zpar, int init) {
+  const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
+  const int kc = flip ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
+  const int ic = blockIdx.x * blockDim.x + threadIdx.x;
+  const int jc = by * blockDim.y + threadIdx.y;
+  const bool act = ic < C.nx && jc < C.ny;
+  if (D != 0 && !act) return;
+  constexpr int ox = D == 0, oy = D == 1, oz = D == 2;
+  const int nx = F.nx, so = D == 0 ? 1 : D == 1 ? nx : nx * F.ny;  // fine stride along D
+  const int nd = D == 0 ? nx : D == 1 ? F.ny : F.nz;
+  const T *w1p = H ? F.q1 : F.p1, *w2p = H ? F.q2 : F.p2;
+  const int i = ox ? 2 * ic : ic, j = oy ? 2 * jc : jc, k = oz ? 2 * kc : kc;
+  const bool comp = ((i + j + k) & 1) != zpar;  // f holds the other colour
+  const int off = comp ? 0 : 1, cd = D == 0 ? ic : D == 1 ? jc : kc;
+  const int f = i + nx * (j + F.ny * k);
+  const bool lo = act && !comp && cd > 0, hi = act && !comp && 2 * cd + 1 < nd;
+  const T w = H && act && comp ? ldro(w1p + f) : T(0);
+  const T w2m = lo ? ldro(w2p + f - so) : T(0), w1u = hi ? ldro(w1p + f + so) : T(0);
+  T d = T(1);
+  bool unit = false;
+  if (init && act) {
+    const int cc = ic + C.nx * (jc + C.ny * kc);
+    if constexpr (H) {
+      unit = ldro(C.hflag) == 0;
+      if (!unit) d = (T)ldro_h(C.h[3] + cc);
+    } else {
+      d = ldro(C.a[0] + cc);
+    }
+  }
+  const bool ev = act && (comp || hi);
+  const bool own = lo && (D != 0 || threadIdx.x == 0 || (threadIdx.x & 31) == 0);
+  PointOp<T> p{}, pm{};
+  if (ev) p = point_op<T, H>(F, i + ox * off, j + oy * off, k + oz * off);
+  if (own) pm = point_op<T, H>(F, i - ox, j - oy, k - oz);
+  pdl_enter();  // the operators and weights ahead of the wait
+  const T r = ev ? op_residual<T>(F, p, x, b, i + ox * off, j + oy * off, k + oz * off) : T(0);
+  T rm = T(0);
+  if constexpr (D == 0) {
+    rm = __shfl_up_sync(0xffffffffu, r, 1);
+    if (!lo) rm = T(0);
+  }
+  if (own) rm = op_residual<T>(F, pm, x, b, i - ox, j - oy, k - oz);
+  if (!act) return;
+  const T v = restrict_value<T, H>(w, comp ? r : T(0), w2m, rm, w1u, comp ? T(0) : r);
+  const int xi = xb_index(C, ic, jc, kc);
+  rc[xi] = v;
+  if (init && ((ic + jc + kc) & 1)) xc[xi] = unit ? v : v / d;
 }
 
 // r_c = r_f(c) + (p2(f-1) r_f(f-1) + p1(f+1) r_f(f+1)) (mg_semi_restrict.c:161-169)
@@ -834,12 +902,11 @@ __device__ __forceinline__ void restrict_cell(const MGLevel<T> &F, const MGLevel
   const T *w1 = H ? F.q1 : F.p1;
   const T *w2 = H ? F.q2 : F.p2;
   const long long f = i + (long long)nx * (j + (long long)ny * k);
-  T centre = rf[f];
-  if constexpr (H) centre = w1[f] * centre;
-  rc[cc] = centre + (vget(nx, ny, nz, w2, i - ox, j - oy, k - oz) *
-                         vget(nx, ny, nz, rf, i - ox, j - oy, k - oz) +
-                     vget(nx, ny, nz, w1, i + ox, j + oy, k + oz) *
-                         vget(nx, ny, nz, rf, i + ox, j + oy, k + oz));
+  rc[cc] = restrict_value<T, H>(H ? w1[f] : T(0), rf[f],
+                                vget(nx, ny, nz, w2, i - ox, j - oy, k - oz),
+                                vget(nx, ny, nz, rf, i - ox, j - oy, k - oz),
+                                vget(nx, ny, nz, w1, i + ox, j + oy, k + oz),
+                                vget(nx, ny, nz, rf, i + ox, j + oy, k + oz));
 }
 
 // grid form of restrict_cell with the direction D fixed at compile time and
@@ -847,7 +914,7 @@ __device__ __forceinline__ void restrict_cell(const MGLevel<T> &F, const MGLevel
 template <typename T, bool H, int D>
 __global__ void __launch_bounds__(256) k_restrict(MGLevel<T> F, MGLevel<T> C,
                                                   const T *__restrict__ rf, T *__restrict__ rc,
-                                                  int flip) {
+                                                  int flip, int init) {
   pdl_enter();
   const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   const int ic = blockIdx.x * blockDim.x + threadIdx.x;
@@ -864,11 +931,20 @@ __global__ void __launch_bounds__(256) k_restrict(MGLevel<T> F, MGLevel<T> C,
   const T *w1 = H ? F.q1 : F.p1;
   const T *w2 = H ? F.q2 : F.p2;
   const bool lo = cd > 0, hi = cd + 1 < nd;
-  T centre = ldro(rf + f);
-  if constexpr (H) centre = ldro(w1 + f) * centre;
-  rc[xb_index(C, ic, jc, kc)] =
-      centre + ((lo ? ldro(w2 + f - so) : T(0)) * (lo ? ldro(rf + f - so) : T(0)) +
-                (hi ? ldro(w1 + f + so) : T(0)) * (hi ? ldro(rf + f + so) : T(0)));
+  const T wc = H ? ldro(w1 + f) : T(0), wl = lo ? ldro(w2 + f - so) : T(0),
+          wh = hi ? ldro(w1 + f + so) : T(0);
+  const T v = restrict_value<T, H>(wc, ldro(rf + f), wl, lo ? ldro(rf + f - so) : T(0), wh,
+                                   hi ? ldro(rf + f + so) : T(0));
+  const int xi = xb_index(C, ic, jc, kc);
+  rc[xi] = v;
+  // the zero-guess red sweep of the coarse level
+  if (init && ((ic + jc + kc) & 1)) {
+    const int cc = ic + C.nx * (jc + C.ny * kc);
+    if constexpr (H)
+      C.x[xi] = ldro(C.hflag) == 0 ? v : v / (T)ldro_h(C.h[3] + cc);
+    else
+      C.x[xi] = v / ldro(C.a[0] + cc);
+  }
 }
 
 // x_f += P e_c: injection at coarse points, p1 e(f-1) + p2 e(f+1) at fine
@@ -885,64 +961,51 @@ __device__ __forceinline__ void prolong_add_cell(const MGLevel<T> &F, const MGLe
   const int ox = d == 0, oy = d == 1, oz = d == 2;
   const T *w1 = H ? F.q1 : F.p1;
   const T *w2 = H ? F.q2 : F.p2;
-  T e;
-  if (!(ci & 1)) {
-    e = ec[(ox ? i / 2 : i) + (long long)C.nx * ((oy ? j / 2 : j) + (long long)C.ny * (oz ? k / 2 : k))];
-    if constexpr (H) e = w1[c] * e;
-  } else {
-    int il = i - ox, jl = j - oy, kl = k - oz;  // coarse point below (even)
-    int ih = i + ox, jh = j + oy, kh = k + oz;  // coarse point above (even), may be outside
-    T el = ec[(ox ? il / 2 : il) + (long long)C.nx * ((oy ? jl / 2 : jl) + (long long)C.ny * (oz ? kl / 2 : kl))];
-    T eh = inside(F.nx, F.ny, F.nz, ih, jh, kh)
-               ? ec[(ox ? ih / 2 : ih) + (long long)C.nx * ((oy ? jh / 2 : jh) + (long long)C.ny * (oz ? kh / 2 : kh))]
-               : T(0);
-    e = (w1[c] * el + w2[c] * eh);
-  }
-  xf[c] = xf[c] + e;
+  const bool odd = ci & 1;
+  // coarse points at / below and (fine points, where it exists) above
+  const int il = i - (odd ? ox : 0), jl = j - (odd ? oy : 0), kl = k - (odd ? oz : 0);
+  const int ih = i + ox, jh = j + oy, kh = k + oz;
+  const T el = ec[(ox ? il / 2 : il) + (long long)C.nx * ((oy ? jl / 2 : jl) + (long long)C.ny * (oz ? kl / 2 : kl))];
+  const T eh = odd && inside(F.nx, F.ny, F.nz, ih, jh, kh)
+                   ? ec[(ox ? ih / 2 : ih) + (long long)C.nx * ((oy ? jh / 2 : jh) + (long long)C.ny * (oz ? kh / 2 : kh))]
+                   : T(0);
+  xf[c] = add_rn(xf[c], prolong_value<T, H>(odd, H || odd ? w1[c] : T(0), odd ? w2[c] : T(0), el, eh));
 }
 
-// grid form of prolong_add_cell with the direction D fixed at compile time:
-// one branch-free formula for both parities (at a coarse point the weights
-// are (1, 0), or (s_c, 0) in H mode, and both coarse neighbours coincide),
-// bitwise the same values as prolong_add_cell
-template <typename T, bool H, int D>
+// grid form of prolong_add_cell with the direction D fixed at compile time.
+// BLACK: a red/black post-smoother starts with a red sweep, which overwrites
+// the red cells without reading them, so only the black cells are corrected
+// (a thread per black cell of a row); else every cell.
+// 512x512x50, scaled FP16 operator, finest level: 32 us against 60 with a
+// thread per cell, half of them leaving at once.
+template <typename T, bool H, int D, bool BLACK>
 __global__ void __launch_bounds__(256) k_prolong_add(MGLevel<T> F, MGLevel<T> C,
                                                      const T *__restrict__ ec,
-                                                     T *__restrict__ xf, int flip, int skip_red) {
-  pdl_enter();
+                                                     T *__restrict__ xf, int flip) {
   const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = by * blockDim.y + threadIdx.y;
   const int k = flip ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
   const int nx = F.nx, ny = F.ny;
+  if (BLACK) i = 2 * i + ((j + k) & 1);
   if (i >= nx || j >= ny) return;
-  // a red/black post-smoother starts with a red sweep, which overwrites the
-  // red cells without reading them: only the black cells need the correction
-  if (skip_red && ((i + j + k) & 1)) return;
   const int c = i + nx * (j + ny * k);
   const int cd = D == 0 ? i : D == 1 ? j : k;
   const int nd = D == 0 ? nx : D == 1 ? ny : F.nz;
-  const int lo = cd >> 1, hi = (cd + 1) >> 1;  // coarse points at/below, at/above
-  const bool odd = cd & 1;
-  const bool has_hi = hi < (nd + 1) / 2;
+  const int lo = cd >> 1;  // coarse point at / below
+  const bool odd = cd & 1, has_hi = odd && cd + 1 < nd;
   const int clo = D == 0 ? xb_index(C, lo, j, k) : D == 1 ? xb_index(C, i, lo, k)
                                                          : xb_index(C, i, j, lo);
-  const int chi = D == 0 ? xb_index(C, hi, j, k) : D == 1 ? xb_index(C, i, hi, k)
-                                                         : xb_index(C, i, j, hi);
-  const T el = ldro(ec + clo);
-  const T eh = has_hi ? ldro(ec + chi) : T(0);
+  const int chi = D == 0 ? xb_index(C, lo + 1, j, k) : D == 1 ? xb_index(C, i, lo + 1, k)
+                                                             : xb_index(C, i, j, lo + 1);
   const T *w1p = H ? F.q1 : F.p1;
   const T *w2p = H ? F.q2 : F.p2;
-  T e;
-  if constexpr (H) {
-    // coarse points: q1 = s_c, q2 = 0
-    const T w1 = ldro(w1p + c);
-    e = odd ? (w1 * el + ldro(w2p + c) * eh) : w1 * el;
-  } else {
-    e = odd ? (ldro(w1p + c) * el + ldro(w2p + c) * eh) : el;
-  }
+  const T w1 = H || odd ? ldro(w1p + c) : T(0), w2 = odd ? ldro(w2p + c) : T(0);
   const int xc = xb_index(F, i, j, k);
-  xf[xc] = xf[xc] + e;
+  const T xv = xf[xc];  // (the kernel before this one works on the coarse level)
+  pdl_enter();
+  const T el = ldro(ec + clo), eh = has_hi ? ldro(ec + chi) : T(0);
+  xf[xc] = add_rn(xv, prolong_value<T, H>(odd, w1, w2, el, eh));
 }
 
 // ---------------------------------------------------------------------------
@@ -1466,33 +1529,58 @@ static bool rb_sweep_pairs(const MGLevel<T> &L, bool h16) {
   else
     return false;
 }
-template <typename T>
-static void rb_sweep(const MGLevel<T> &L, T *x, const T *b, int colour, int init,
-                     cudaStream_t st, int flip, bool h16, int from_b = 0) {
+// b_early: the kernel launched before this one does not write b
+constexpr long long EARLY_CELLS = 400000;
+template <typename T, bool H, bool EARLY>
+static void rb_sweep_t(const MGLevel<T> &L, T *x, const T *b, int colour, int init,
+                       cudaStream_t st, int flip, int b_early, int from_b) {
   // two cells per thread on colour-split levels of the FP16 operator (it is
   // bound by instruction issue there; the FP32 and FP64 sweeps, bound by
   // memory, are as fast or faster with one cell per thread and more threads)
-  if constexpr (kHasH16<T>) {
-    if (rb_sweep_pairs(L, h16)) {
+  if constexpr (H) {
+    if (rb_sweep_pairs(L, H) && !init) {
       Shape3 g2 = shape3((L.hx + 1) / 2, L.ny, L.nz);
       if (from_b)
-        launch_pdl(k_rb_sweep2<T, true, true>, dim3(g2.grid), dim3(g2.block), st, L, x, b,
-                   colour, init, flip);
+        launch_pdl(k_rb_sweep2<T, true, true, EARLY>, g2.grid, g2.block, st, L, x, b, colour,
+                   flip, b_early);
       else
-        launch_pdl(k_rb_sweep2<T, true>, dim3(g2.grid), dim3(g2.block), st, L, x, b, colour,
-                   init, flip);
+        launch_pdl(k_rb_sweep2<T, true, false, EARLY>, g2.grid, g2.block, st, L, x, b, colour,
+                   flip, b_early);
       return;
     }
   }
   Shape3 g = shape3((L.nx + 1) / 2, L.ny, L.nz);
+  launch_pdl(k_rb_sweep<T, H, EARLY>, g.grid, g.block, st, L, x, b, colour, init, flip, b_early);
+}
+template <typename T>
+static void rb_sweep(const MGLevel<T> &L, T *x, const T *b, int colour, int init,
+                     cudaStream_t st, int flip, bool h16, int b_early, int from_b = 0) {
+  const bool early = L.n <= EARLY_CELLS;
   if constexpr (kHasH16<T>) {
     if (h16) {
-      launch_pdl(k_rb_sweep<T, true>, dim3(g.grid), dim3(g.block), st, L, x, b, colour, init,
-                 flip);
+      if (early)
+        rb_sweep_t<T, true, true>(L, x, b, colour, init, st, flip, b_early, from_b);
+      else
+        rb_sweep_t<T, true, false>(L, x, b, colour, init, st, flip, b_early, from_b);
       return;
     }
   }
-  launch_pdl(k_rb_sweep<T, false>, dim3(g.grid), dim3(g.block), st, L, x, b, colour, init, flip);
+  if (early)
+    rb_sweep_t<T, false, true>(L, x, b, colour, init, st, flip, b_early, from_b);
+  else
+    rb_sweep_t<T, false, false>(L, x, b, colour, init, st, flip, b_early, from_b);
+}
+// the zero-guess red sweep of a pre-smoother is not launched: the black sweep
+// that follows reads its values from b, and the last red sweep writes them
+template <typename T>
+static bool zero_sweep_from_b(const MGLevel<T> &L, int smoother, bool h16) {
+  return smoother == 0 && rb_sweep_pairs(L, h16) && skip_zero_sweep();
+}
+// ... or it is left to the kernel that writes the level's right-hand side
+template <typename T>
+bool mg_wants_red_init(const MGLevel<T> &L, int smoother, bool h16) {
+  return (smoother == 0 || smoother == 2) && L.zc >= 0 && !L.lo[0] &&
+         !zero_sweep_from_b(L, smoother, h16);
 }
 // RedBlackGSPoint, MaxIter 1: red, black, red (Symmetric True, smoother 0)
 // or red, black (Symmetric False, smoother 2); a zero initial guess turns the
@@ -1518,28 +1606,33 @@ int launch_mg_smooth(const MGLevel<T> &L, T *x, const T *b, int zero, int smooth
     return 2;
   }
   if (smoother == 9) {  // a single red sweep (kernel timing)
-    rb_sweep(L, x, b, 0, 0, st, 0, h16);
+    rb_sweep(L, x, b, 0, 0, st, 0, h16, 1);
     return 1;
   }
-  if (smoother == 2) {
-    rb_sweep(L, x, b, 0, zero, st, f, h16);
-    rb_sweep(L, x, b, 1, 0, st, g, h16);
-    if (flip) *flip = f;
-    return 2;
-  }
-  if (zero && rb_sweep_pairs(L, h16) && skip_zero_sweep()) {
+  // zero: 1 zero initial guess, 2 the same with its red sweep already done by
+  // the kernel that wrote b.  With a zero guess the kernel before the first
+  // sweep is the one that writes b.
+  if (zero == 1 && zero_sweep_from_b(L, smoother, h16)) {
     // the black sweep reads the zero-guess red values from b; the last red
     // sweep writes x of the red cells
-    rb_sweep(L, x, b, 1, 0, st, g, h16, 1);
-    rb_sweep(L, x, b, 0, 0, st, f, h16);
+    rb_sweep(L, x, b, 1, 0, st, g, h16, 0, 1);
+    rb_sweep(L, x, b, 0, 0, st, f, h16, 1);
     if (flip) *flip = g;
     return 2;
   }
-  rb_sweep(L, x, b, 0, zero, st, f, h16);
-  rb_sweep(L, x, b, 1, 0, st, g, h16);
-  rb_sweep(L, x, b, 0, 0, st, f, h16);
+  int k = 0;
+  if (zero != 2) {
+    rb_sweep(L, x, b, 0, zero, st, f, h16, zero == 0);
+    k++;
+  }
+  rb_sweep(L, x, b, 1, 0, st, g, h16, zero != 2);
+  if (smoother == 2) {
+    if (flip) *flip = f;
+    return k + 1;
+  }
+  rb_sweep(L, x, b, 0, 0, st, f, h16, 1);
   if (flip) *flip = g;
-  return 3;
+  return k + 2;
 }
 template <typename K>
 static cudaError_t mid_prepare(K kern) {
@@ -1548,6 +1641,9 @@ static cudaError_t mid_prepare(K kern) {
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
+
+template <typename T, bool H>
+__global__ void k_setup_tail_smem(const MGLevel<T> *__restrict__ Ls, int first, int nl);
 
 // opt the fused smoother, the shared-memory tails and the cluster kernel into
 // their dynamic shared memory (> 48 KB) and cluster sizes above 8; called once
@@ -1566,6 +1662,17 @@ cudaError_t mg_prepare_kernels() {
   e = cudaFuncSetAttribute(k_vcycle_tail_smem<double, false>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM_MAX);
   if (e != cudaSuccess) return e;
+  e = tail_pairs_prepare<float>();
+  if (e != cudaSuccess) return e;
+  e = tail_pairs_prepare<double>();
+  if (e != cudaSuccess) return e;
+  for (const void *k : {(const void *)k_setup_tail_smem<float, false>,
+                        (const void *)k_setup_tail_smem<float, true>,
+                        (const void *)k_setup_tail_smem<double, false>}) {
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)SETUP_TAIL_SMEM_MAX);
+    if (e != cudaSuccess) return e;
+  }
   e = mid_prepare(k_vcycle_mid<float, false>);
   if (e != cudaSuccess) return e;
   e = mid_prepare(k_vcycle_mid<float, true>);
@@ -1620,50 +1727,80 @@ void launch_mg_residual(const MGLevel<T> &L, const T *x, const T *b, T *r, cudaS
 }
 template <typename T, bool H>
 static void restrict_d(const MGLevel<T> &F, const MGLevel<T> &C, const T *rf, T *rc,
-                       cudaStream_t st, int flip) {
+                       cudaStream_t st, int flip, int init) {
   Shape3 g = shape3(C.nx, C.ny, C.nz);
   if (F.dir == 0)
-    launch_pdl(k_restrict<T, H, 0>, dim3(g.grid), dim3(g.block), st, F, C, rf, rc, flip);
+    launch_pdl(k_restrict<T, H, 0>, g.grid, g.block, st, F, C, rf, rc, flip, init);
   else if (F.dir == 1)
-    launch_pdl(k_restrict<T, H, 1>, dim3(g.grid), dim3(g.block), st, F, C, rf, rc, flip);
+    launch_pdl(k_restrict<T, H, 1>, g.grid, g.block, st, F, C, rf, rc, flip, init);
   else
-    launch_pdl(k_restrict<T, H, 2>, dim3(g.grid), dim3(g.block), st, F, C, rf, rc, flip);
+    launch_pdl(k_restrict<T, H, 2>, g.grid, g.block, st, F, C, rf, rc, flip, init);
 }
-template <typename T, bool H>
+template <typename T, bool H, bool BLACK>
 static void prolong_d(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, T *xf,
-                      cudaStream_t st, int flip, int skip_red) {
-  Shape3 g = shape3(F.nx, F.ny, F.nz);
+                      cudaStream_t st, int flip) {
+  Shape3 g = shape3(BLACK ? (F.nx + 1) / 2 : F.nx, F.ny, F.nz);
   if (F.dir == 0)
-    launch_pdl(k_prolong_add<T, H, 0>, dim3(g.grid), dim3(g.block), st, F, C, ec, xf, flip,
-               skip_red);
+    launch_pdl(k_prolong_add<T, H, 0, BLACK>, g.grid, g.block, st, F, C, ec, xf, flip);
   else if (F.dir == 1)
-    launch_pdl(k_prolong_add<T, H, 1>, dim3(g.grid), dim3(g.block), st, F, C, ec, xf, flip,
-               skip_red);
+    launch_pdl(k_prolong_add<T, H, 1, BLACK>, g.grid, g.block, st, F, C, ec, xf, flip);
   else
-    launch_pdl(k_prolong_add<T, H, 2>, dim3(g.grid), dim3(g.block), st, F, C, ec, xf, flip,
-               skip_red);
+    launch_pdl(k_prolong_add<T, H, 2, BLACK>, g.grid, g.block, st, F, C, ec, xf, flip);
 }
 template <typename T>
 void launch_mg_restrict(const MGLevel<T> &F, const MGLevel<T> &C, const T *rf, T *rc,
-                        cudaStream_t st, int flip, bool h16) {
+                        cudaStream_t st, int flip, bool h16, int init) {
   if constexpr (kHasH16<T>) {
     if (h16) {
-      restrict_d<T, true>(F, C, rf, rc, st, flip);
+      restrict_d<T, true>(F, C, rf, rc, st, flip, init);
       return;
     }
   }
-  restrict_d<T, false>(F, C, rf, rc, st, flip);
+  restrict_d<T, false>(F, C, rf, rc, st, flip, init);
+}
+template <typename T, bool H>
+static void resid_restrict_d(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st, int flip,
+                             int init) {
+  const int zpar = F.zc == 0 ? 1 : 0;  // colour 0 (red) is parity 1 of i + j + k
+  const Shape3 g = shape3(C.nx, C.ny, C.nz);
+  const T *x = F.x, *b = F.b;
+  if (F.dir == 0)
+    launch_pdl(k_resid_restrict<T, H, 0>, g.grid, g.block, st, F, C, x, b, C.b, C.x, flip, zpar,
+               init);
+  else if (F.dir == 1)
+    launch_pdl(k_resid_restrict<T, H, 1>, g.grid, g.block, st, F, C, x, b, C.b, C.x, flip, zpar,
+               init);
+  else
+    launch_pdl(k_resid_restrict<T, H, 2>, g.grid, g.block, st, F, C, x, b, C.b, C.x, flip, zpar,
+               init);
+}
+template <typename T>
+void launch_mg_resid_restrict(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st, int flip,
+                              bool h16, int init) {
+  if constexpr (kHasH16<T>) {
+    if (h16) {
+      resid_restrict_d<T, true>(F, C, st, flip, init);
+      return;
+    }
+  }
+  resid_restrict_d<T, false>(F, C, st, flip, init);
 }
 template <typename T>
 void launch_mg_prolong_add(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, T *xf,
-                           cudaStream_t st, int flip, bool h16, int skip_red) {
+                           cudaStream_t st, int flip, bool h16, int black) {
   if constexpr (kHasH16<T>) {
     if (h16) {
-      prolong_d<T, true>(F, C, ec, xf, st, flip, skip_red);
+      if (black)
+        prolong_d<T, true, true>(F, C, ec, xf, st, flip);
+      else
+        prolong_d<T, true, false>(F, C, ec, xf, st, flip);
       return;
     }
   }
-  prolong_d<T, false>(F, C, ec, xf, st, flip, skip_red);
+  if (black)
+    prolong_d<T, false, true>(F, C, ec, xf, st, flip);
+  else
+    prolong_d<T, false, false>(F, C, ec, xf, st, flip);
 }
 template <typename T>
 void launch_vcycle_tail(const MGLevel<T> *levels_dev, int first, int nl, int smoother,
@@ -1780,10 +1917,6 @@ cudaError_t launch_vcycle_grid(const MGLevel<T> *levels_dev, int mid, int tail, 
                           smoother, w, tmp, ctl);
 }
 
-template <typename T>
-void launch_setup_tail(const MGLevel<T> *levels_dev, int first, int nl, cudaStream_t st) {
-  launch_pdl(k_setup_tail<T>, dim3(1), dim3(512), st, levels_dev, first, nl);
-}
 
 // ---------------------------------------------------------------------------
 // Scaled FP16 operator (H mode): from the plain FP32 operator of level F (and
@@ -1858,13 +1991,125 @@ __global__ void __launch_bounds__(512) k_h16_scale_tail(const MGLevel<float> *__
   }
 }
 
+// Setup of the tail levels in one block out of shared memory: the operators
+// of all tail levels live there, one phase per level (weights and coarse
+// operator as k_setup_level, the scaled operator with them in H mode, the
+// coarsest level's own scaling at the end), the results stored to global
+// memory as they come.  Bound by the chain of levels: 11 phases instead of
+// the 22 global-memory phases of k_setup_tail and the 11 of k_h16_scale_tail.
+template <typename T, int D, bool H>
+__device__ __forceinline__ void setup_tail_level(const MGLevel<T> &F, const MGLevel<T> &C, T *fs,
+                                                 T *cs) {
+  const int nf = (int)F.n, nc = (int)C.n;
+  LV<T> L;
+  L.nx = F.nx; L.ny = F.ny; L.nz = F.nz; L.n = nf;
+  L.a0 = fs; L.ae = fs + nf; L.an = fs + 2 * nf; L.au = fs + 3 * nf;
+  L.wg = F.wg;
+  const FastDiv fx = fast_div(C.nx), fy = fast_div(C.ny);
+  for (int t = threadIdx.x; t < nc; t += blockDim.x) {
+    int i, j, k;
+    split_ijk(t, fx, fy, i, j, k);
+    const CoarseRow<T> r = setup_point<T, D, H>(L, F, C, i, j, k);
+    cs[t] = r.c;
+    cs[nc + t] = r.e;
+    cs[2 * nc + t] = r.n;
+    cs[3 * nc + t] = r.u;
+    C.a[0][t] = r.c;
+    C.a[1][t] = r.e;
+    C.a[2][t] = r.n;
+    C.a[3][t] = r.u;
+  }
+}
+template <typename T, bool H>
+__global__ void __launch_bounds__(TAIL_THREADS, 1)
+    k_setup_tail_smem(const MGLevel<T> *__restrict__ Ls, int first, int nl) {
+  extern __shared__ __align__(16) unsigned char setup_raw[];
+  __shared__ __align__(16) unsigned char tab[TAIL_MAX_LEVELS * sizeof(MGLevel<T>)];
+  static_assert(sizeof(MGLevel<T>) % 4 == 0, "copied in words");
+  const int nt = nl - first;
+  // the level table is fixed at creation: copied ahead of the wait
+  for (int e = threadIdx.x; e < nt * (int)(sizeof(MGLevel<T>) / 4); e += blockDim.x)
+    reinterpret_cast<uint32_t *>(tab)[e] = reinterpret_cast<const uint32_t *>(Ls + first)[e];
+  __syncthreads();
+  pdl_enter();
+  const MGLevel<T> *S = reinterpret_cast<const MGLevel<T> *>(tab);
+  T *fs = reinterpret_cast<T *>(setup_raw);
+  {
+    const int n = (int)S[0].n;
+    const T *a0 = S[0].a[0], *a1 = S[0].a[1], *a2 = S[0].a[2], *a3 = S[0].a[3];
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+      const T v0 = a0[t], v1 = a1[t], v2 = a2[t], v3 = a3[t];
+      fs[t] = v0;
+      fs[n + t] = v1;
+      fs[2 * n + t] = v2;
+      fs[3 * n + t] = v3;
+    }
+  }
+  __syncthreads();
+  for (int l = 0; l + 1 < nt; l++) {
+    const MGLevel<T> &F = S[l], &C = S[l + 1];
+    T *cs = fs + 4 * (int)F.n;
+    if (F.dir == 0)
+      setup_tail_level<T, 0, H>(F, C, fs, cs);
+    else if (F.dir == 1)
+      setup_tail_level<T, 1, H>(F, C, fs, cs);
+    else
+      setup_tail_level<T, 2, H>(F, C, fs, cs);
+    fs = cs;
+    __syncthreads();  // (the coarse ghost column too, written to global memory)
+  }
+  if constexpr (H) {
+    // the coarsest level's scaling
+    const MGLevel<float> &F = S[nt - 1];
+    for (int t = threadIdx.x; t < (int)F.n; t += blockDim.x) {
+      int i, j, k;
+      split_ijk(t, F.nx, F.ny, i, j, k);
+      h16_scale_cell(F, F, 0, i, j, k);
+    }
+  }
+}
+
 void launch_h16_scale(const MGLevel<float> &F, const MGLevel<float> *C, cudaStream_t st) {
   Shape3 g = shape3(F.nx, F.ny, F.nz);
   launch_pdl(k_h16_scale, dim3(g.grid), dim3(g.block), st, F, C ? *C : F, C ? 1 : 0);
 }
-void launch_h16_scale_tail(const MGLevel<float> *levels_dev, int first, int nl,
-                           cudaStream_t st) {
-  launch_pdl(k_h16_scale_tail, dim3(1), dim3(512), st, levels_dev, first, nl);
+// the operators of all tail levels in shared memory
+template <typename T>
+static size_t setup_tail_bytes(const MGLevel<T> *L, int first, int nl) {
+  long long n = 0;
+  for (int q = first; q < nl; q++) n += L[q].n;
+  return (size_t)(4 * n * (long long)sizeof(T));
+}
+template <typename T>
+int launch_setup_tail(const MGLevel<T> *L, const MGLevel<T> *levels_dev, int first, int nl,
+                      cudaStream_t st, bool h16) {
+  const size_t smem = setup_tail_bytes(L, first, nl);
+  if (nl - first <= TAIL_MAX_LEVELS && smem <= SETUP_TAIL_SMEM_MAX) {
+    if constexpr (kHasH16<T>) {
+      if (h16) {
+        launch_pdl_smem(k_setup_tail_smem<T, true>, dim3(1), dim3(TAIL_THREADS), smem, st,
+                        levels_dev, first, nl);
+        return 1;
+      }
+    }
+    if (first + 1 < nl)
+      launch_pdl_smem(k_setup_tail_smem<T, false>, dim3(1), dim3(TAIL_THREADS), smem, st,
+                      levels_dev, first, nl);
+    return first + 1 < nl ? 1 : 0;
+  }
+  // tails that do not fit (a hierarchy cut short by MaxLevels)
+  int k = 0;
+  if (first + 1 < nl) {
+    launch_pdl(k_setup_tail<T>, dim3(1), dim3(512), st, levels_dev, first, nl);
+    k++;
+  }
+  if constexpr (kHasH16<T>) {
+    if (h16) {
+      launch_pdl(k_h16_scale_tail, dim3(1), dim3(512), st, levels_dev, first, nl);
+      k++;
+    }
+  }
+  return k;
 }
 
 // level-0 transfers of the preconditioner: a natural-layout FP64 vector into
@@ -1877,7 +2122,7 @@ constexpr int LEVEL_PLANES = 4;
 
 template <typename TO>
 __global__ void k_level_in(MGLevel<TO> L, const double *__restrict__ in, TO *__restrict__ out,
-                           const float *__restrict__ scale) {
+                           const float *__restrict__ scale, int init) {
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y, k0 = LEVEL_PLANES * blockIdx.z;
@@ -1888,8 +2133,13 @@ __global__ void k_level_in(MGLevel<TO> L, const double *__restrict__ in, TO *__r
   for (int u = 0; u < LEVEL_PLANES; u++) v[u] = k0 + u < L.nz ? in[c0 + u * sz] : 0.0;
 #pragma unroll
   for (int u = 0; u < LEVEL_PLANES; u++)
-    if (k0 + u < L.nz)
-      out[xb_index(L, i, j, k0 + u)] = cvt<double, TO>(v[u], scale, c0 + u * sz);
+    if (k0 + u < L.nz) {
+      const TO b = cvt<double, TO>(v[u], scale, c0 + u * sz);
+      const int o = xb_index(L, i, j, k0 + u);
+      out[o] = b;
+      // the zero-guess red sweep (plain operators)
+      if (init && ((i + j + k0 + u) & 1)) L.x[o] = b / L.a[0][c0 + u * sz];
+    }
 }
 template <typename TI>
 __global__ void k_level_out(MGLevel<TI> L, const TI *__restrict__ in, double *__restrict__ out,
@@ -1911,10 +2161,17 @@ __global__ void k_level_out(MGLevel<TI> L, const TI *__restrict__ in, double *__
 }
 
 template <typename T>
-int launch_level_in(const MGLevel<T> &L, const double *r, const float *scale, cudaStream_t st) {
+bool level_in_inits(const MGLevel<T> &L, int smoother, bool h16) {
+  return L.split && !h16 && mg_wants_red_init(L, smoother, h16);
+}
+template bool level_in_inits<float>(const MGLevel<float> &, int, bool);
+template bool level_in_inits<double>(const MGLevel<double> &, int, bool);
+template <typename T>
+int launch_level_in(const MGLevel<T> &L, const double *r, const float *scale, cudaStream_t st,
+                    int init) {
   if (L.split) {
     Shape3 g = shape3(L.nx, L.ny, (L.nz + LEVEL_PLANES - 1) / LEVEL_PLANES);
-    launch_pdl(k_level_in<T>, dim3(g.grid), dim3(g.block), st, L, r, L.b, scale);
+    launch_pdl(k_level_in<T>, dim3(g.grid), dim3(g.block), st, L, r, L.b, scale, init);
     return 1;
   }
   if (std::is_same<T, double>::value && !scale) {
@@ -1940,9 +2197,9 @@ int launch_level_out(const MGLevel<T> &L, const T *x, double *z, const float *sc
   return 1;
 }
 template int launch_level_in<float>(const MGLevel<float> &, const double *, const float *,
-                                    cudaStream_t);
+                                    cudaStream_t, int);
 template int launch_level_in<double>(const MGLevel<double> &, const double *, const float *,
-                                     cudaStream_t);
+                                     cudaStream_t, int);
 template int launch_level_out<float>(const MGLevel<float> &, const float *, double *,
                                      const float *, int, cudaStream_t);
 template int launch_level_out<double>(const MGLevel<double> &, const double *, double *,
@@ -1966,8 +2223,11 @@ void launch_convert(const TI *in, TO *out, long long n, cudaStream_t st, int fli
                                     cudaStream_t, int *, bool);                               \
   template void launch_mg_residual<T>(const MGLevel<T> &, const T *, const T *, T *,          \
                                       cudaStream_t, int, bool, int);                          \
+  template void launch_mg_resid_restrict<T>(const MGLevel<T> &, const MGLevel<T> &,            \
+                                            cudaStream_t, int, bool, int);                    \
+  template bool mg_wants_red_init<T>(const MGLevel<T> &, int, bool);                           \
   template void launch_mg_restrict<T>(const MGLevel<T> &, const MGLevel<T> &, const T *, T *, \
-                                      cudaStream_t, int, bool);                               \
+                                      cudaStream_t, int, bool, int);                               \
   template void launch_mg_prolong_add<T>(const MGLevel<T> &, const MGLevel<T> &, const T *,   \
                                          T *, cudaStream_t, int, bool, int);                  \
   template void launch_vcycle_mid<T>(const MGLevel<T> *, int, int, int, int, double, T *,       \
@@ -1979,7 +2239,8 @@ void launch_convert(const TI *in, TO *out, long long n, cudaStream_t st, int fli
   template void launch_vcycle_tail<T>(const MGLevel<T> *, int, int, int, double, T *, size_t, \
                                       cudaStream_t, bool);                                    \
   template size_t tail_smem_bytes<T>(const MGLevel<T> *, int, int, bool);                    \
-  template void launch_setup_tail<T>(const MGLevel<T> *, int, int, cudaStream_t);
+  template int launch_setup_tail<T>(const MGLevel<T> *, const MGLevel<T> *, int, int,         \
+                                    cudaStream_t, bool);
 INST(double)
 INST(float)
 template void launch_convert<double, float>(const double *, float *, long long, cudaStream_t, int,

@@ -14,6 +14,11 @@
 
 namespace pfgpu {
 
+// What a kernel may read before pdl_enter(): a kernel lets its successor start
+// only after its own wait, so when this kernel runs, everything up to the
+// kernel before its predecessor is complete and visible.  Arrays that the
+// predecessor itself writes (any element of them: a cached line would be stale
+// after the wait) must not be touched before pdl_enter().
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 #ifndef PFGPU_PDL_LATE_TRIGGER

@@ -74,10 +74,13 @@ struct MG {
   int grid_blocks = 0;         // levels mid .. tail-1 on cooperative grid kernels instead
   unsigned *gbar = nullptr;    // their barrier: counter, generation
   size_t tail_smem = 0;        // shared-memory bytes of the V-cycle tail (0: global)
+  void *tail_image = nullptr;  // packed tail levels of the pair kernel (red/black
+                               // smoothers), or null: the generic tail
   std::vector<char> waved;     // level smoothed by the wavefront kernel
   std::vector<WaveLevel> wave; // its control words
   bool h16 = false;            // scaled FP16 operator storage (float levels only)
   int *hflag = nullptr;        // some scaled diagonal is not +1 (set by the setup)
+  long long fuse_cells = 0;    // levels up to this size: residual and restriction in one launch
   int flip = 1;                // alternate the block order of consecutive launches
   int flip_out = 0;            // block order for the launch after a V-cycle
   T *wtmp = nullptr;           // Jacobi temp (finest size)
@@ -94,6 +97,10 @@ struct MG {
 //                     single-block tail kernels, as far as the tail fits in
 //                     shared memory (default 1024)
 //   PFGPU_TAIL_SMEM   0 runs the V-cycle tail from global memory
+//   PFGPU_FUSE_CELLS  grid levels at or below this many cells take residual
+//                     and restriction in one launch (default 400000: at
+//                     256x256x50 the V-cycle is 305 us there, 321 with none
+//                     and 311 with 1000000)
 //   PFGPU_MID_CELLS   grid levels at or below this many cells run, with the
 //                     tail, inside one thread-block-cluster kernel (default 0:
 //                     none; on B200 each of its phases waits about as long on
@@ -470,29 +477,38 @@ static void matvec(pfgpu_handle *h, const double *x, double *y) {
 }
 
 template <typename T>
-static long long mg_setup_T(MG<T> &mg, cudaStream_t st) {
+static long long mg_setup_T(MG<T> &mg, int smoother, cudaStream_t st) {
   long long k = 0;
   const int nl = (int)mg.L.size();
+  auto pack = [&]() {
+    if (!mg.tail_image) return;
+    launch_tail_pack<T>(mg.L.data(), mg.tail, nl, smoother, mg.tail_image, st, mg.h16);
+    k++;
+  };
   // FullJacobian: every level from the generic setup (mg_full.cu)
-  if (mg.L[0].lo[0]) return launch_mg_full_setup<T>(mg.L.data(), nl, st);
+  if (mg.L[0].lo[0]) {
+    k = launch_mg_full_setup<T>(mg.L.data(), nl, st);
+    pack();
+    return k;
+  }
   if (mg.h16) cudaMemsetAsync(mg.hflag, 0, sizeof(int), st);
-  for (int l = 0; l < mg.tail && l + 1 < nl; l++) {
-    launch_mg_setup_level<T>(mg.L[l], mg.L[l + 1], st, mg.h16);
+  // levels above 2048 cells on a grid each (their own scaling included), the
+  // rest in one block
+  int first = 0;
+  while (first < nl - 1 && mg.L[first].n > SETUP_TAIL_CELLS) {
+    launch_mg_setup_level<T>(mg.L[first], mg.L[first + 1], st, mg.h16);
+    first++;
     k++;
   }
-  if (mg.tail < nl - 1) {
-    launch_setup_tail<T>(mg.Ldev, mg.tail, nl, st);
-    k++;
-  }
-  if constexpr (std::is_same<T, float>::value) {
-    if (mg.h16) {
-      // the grid levels were scaled by their setup kernels; the tail levels
-      // once their operators are final
-      launch_h16_scale_tail(mg.Ldev, mg.tail, nl, st);
-      k++;
-    }
-  }
+  k += launch_setup_tail<T>(mg.L.data(), mg.Ldev, first, nl, st, mg.h16);
+  pack();
   return k;
+}
+
+// the input conversion of level 0 also does its zero-guess red sweep
+template <typename T>
+static bool level0_red_done(const MG<T> &mg, int smoother) {
+  return mg.mid > 0 && !mg.fused[0] && !mg.waved[0] && level_in_inits(mg.L[0], smoother, mg.h16);
 }
 
 // One V-cycle with zero initial guess on level-0 (b -> x)
@@ -523,6 +539,8 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
   // colour sweeps); the coarse levels start from zero in every cycle
   for (int cyc = 0; cyc < max_iter; cyc++) {
   const int zero0 = cyc == 0 ? 1 : 0;
+  // the level's zero-guess red sweep came with its right-hand side
+  bool red_done = level0_red_done(mg, smoother);
   for (int l = 0; l < first; l++) {
     MGLevel<T> &Ll = mg.L[l];
     const int zero = l == 0 ? zero0 : 1;
@@ -533,6 +551,7 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
       launch_mg_full_residual<T>(Ll, Ll.x, Ll.b, Ll.t, st);
       launch_mg_restrict<T>(Ll, mg.L[l + 1], Ll.t, mg.L[l + 1].b, st, next(), mg.h16);
       k += 2;
+      red_done = false;
       continue;
     }
     if (mg.fused[l]) {
@@ -543,12 +562,21 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
       f = mg.flip ? 1 : 0;  // the wave ends on the top planes
       k++;
     } else {
-      k += launch_mg_smooth<T>(Ll, Ll.x, Ll.b, zero, smoother, w, mg.wtmp, st, fp, mg.h16);
+      k += launch_mg_smooth<T>(Ll, Ll.x, Ll.b, zero && red_done ? 2 : zero, smoother, w, mg.wtmp,
+                               st, fp, mg.h16);
     }
-    // after the plain red/black pre-smoother the colour swept last (red, or
-    // black for the non-symmetric order) has a zero residual up to rounding
+    // after a red/black pre-smoother the colour swept last has a zero residual
+    // up to rounding
+    const MGLevel<T> &C = mg.L[l + 1];
+    red_done = Ll.zc >= 0 && l + 1 < first && !mg.fused[l + 1] && !mg.waved[l + 1] &&
+               mg_wants_red_init(C, smoother, mg.h16);
+    if (Ll.zc >= 0 && Ll.n <= mg.fuse_cells) {
+      launch_mg_resid_restrict<T>(Ll, C, st, next(), mg.h16, red_done ? 1 : 0);
+      k++;
+      continue;
+    }
     launch_mg_residual<T>(Ll, Ll.x, Ll.b, Ll.t, st, next(), mg.h16, Ll.zc);
-    launch_mg_restrict<T>(Ll, mg.L[l + 1], Ll.t, mg.L[l + 1].b, st, next(), mg.h16);
+    launch_mg_restrict<T>(Ll, C, Ll.t, C.b, st, next(), mg.h16, red_done ? 1 : 0);
     k += 2;
   }
   // levels first .. nl-1, coarse solve (RedBlackGSPoint, mg_semi.c:1276) included
@@ -563,6 +591,9 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
   } else if (mg.mid < mg.tail) {
     launch_vcycle_mid<T>(mg.Ldev, mg.mid, mg.tail, nl, smoother, w, mg.wtmp, mg.tail_smem,
                          mg.mid_cs, st, mg.h16);
+    k++;
+  } else if (mg.tail_image) {
+    launch_tail_pairs<T>(mg.L.data(), first, nl, smoother, mg.tail_image, st, mg.h16);
     k++;
   } else {
     launch_vcycle_tail<T>(mg.Ldev, first, nl, smoother, w, mg.wtmp, mg.tail_smem, st, mg.h16);
@@ -627,9 +658,11 @@ static int pc_apply_dense_impl(pfgpu_handle *h, const double *r, double *z) {
     return 0;
   }
   if (h->mixed)
-    k += launch_level_in<float>(h->mgf.L[0], r, h->h16 ? h->mgf.L[0].sinv : nullptr, h->st);
+    k += launch_level_in<float>(h->mgf.L[0], r, h->h16 ? h->mgf.L[0].sinv : nullptr, h->st,
+                                level0_red_done(h->mgf, h->d.mg_smoother));
   else
-    k += launch_level_in<double>(h->mgd.L[0], r, nullptr, h->st);
+    k += launch_level_in<double>(h->mgd.L[0], r, nullptr, h->st,
+                                 level0_red_done(h->mgd, h->d.mg_smoother));
   CK(cudaGetLastError());
   if (h->nk.capturing) {
     k += (int)vcycle_launch(h);  // inline in the solve's graph
@@ -658,9 +691,9 @@ static void pc_setup_dense_impl(pfgpu_handle *h, const double *u, double dt, boo
                                 bool reuse_vg) {
   assemble(h, u, dt, also_J, true, reuse_vg);
   if (h->mixed)
-    h->launches += mg_setup_T<float>(h->mgf, h->st);
+    h->launches += mg_setup_T<float>(h->mgf, h->d.mg_smoother, h->st);
   else
-    h->launches += mg_setup_T<double>(h->mgd, h->st);
+    h->launches += mg_setup_T<double>(h->mgd, h->d.mg_smoother, h->st);
   if (also_J) h->jac_valid = 1;
   h->pc_ready = true;
 }
@@ -1652,6 +1685,43 @@ static int newton(pfgpu_handle *h, double dt, pfgpu_stats *stats) {
 // ---------------------------------------------------------------------------
 // allocation
 // ---------------------------------------------------------------------------
+static void ens_forget(unsigned long long uid);
+// drops the handle's captured solves, its branches of ensemble graphs too
+// (nothing of the handle's may be running)
+static void solve_graphs_forget(pfgpu_handle *h) {
+  pfgpu_handle::NkGraph &G = h->nk;
+  if (G.exec) cudaGraphExecDestroy(G.exec);
+  G.exec = nullptr;
+  G.valid = false;
+  for (auto &kv : G.kept) cudaGraphExecDestroy(kv.exec);
+  G.kept.clear();
+  ens_forget(h->uid);
+}
+
+// red/black sweeps with the paired residual after them (MGLevel::zc >= 0)
+static bool mg_pairs_smoother(const pfgpu_handle *h) {
+  return (h->d.mg_smoother == PFGPU_SMOOTH_RBGS || h->d.mg_smoother == PFGPU_SMOOTH_RBGS_NONSYM) &&
+         env_ll("PFGPU_PAIR_RESIDUAL", 1) != 0;
+}
+
+// how the levels mg.tail .. run: the pair kernel, or the generic tail in
+// shared or global memory
+template <typename T>
+static int tail_form(const pfgpu_handle *h, MG<T> &mg) {
+  const int nl = (int)mg.L.size();
+  const size_t b = tail_smem_bytes<T>(mg.L.data(), mg.tail, nl, mg.h16);
+  const bool smem = env_ll("PFGPU_TAIL_SMEM", 1) != 0;
+  mg.tail_smem = b <= TAIL_SMEM_MAX && smem ? b : 0;
+  cudaFree(mg.tail_image);
+  mg.tail_image = nullptr;
+  if (smem && mg_pairs_smoother(h)) {
+    const size_t img = tail_image_bytes<T>(mg.L.data(), mg.tail, nl, mg.h16);
+    if (img > 0 && dalloc((unsigned char **)&mg.tail_image, (long long)img))
+      return PFGPU_ERR_NOMEM;
+  }
+  return 0;
+}
+
 template <typename T>
 static int alloc_mg(pfgpu_handle *h, MG<T> &mg) {
   double DX = h->d.dx, DY = h->d.dy, DZ = h->d.dz;
@@ -1718,18 +1788,20 @@ static int alloc_mg(pfgpu_handle *h, MG<T> &mg) {
   }
   if (dalloc(&mg.wtmp, mg.L[0].n)) return PFGPU_ERR_NOMEM;
   // first level of the single-block tail: the largest whose tail fits in
-  // shared memory (else the coarsest level alone, run from global memory)
+  // shared memory (else the coarsest level alone, run from global memory).
+  // Above 1024 cells one block walks a level slower than the grid kernels do.
   mg.tail = nl - 1;
+  const bool pairs = mg_pairs_smoother(h);
   const long long tail_cells = env_ll("PFGPU_TAIL_CELLS", 1024);
   for (int l = 0; l < nl; l++)
-    if (mg.L[l].n <= tail_cells && tail_smem_bytes<T>(mg.L.data(), l, nl, mg.h16) <= TAIL_SMEM_MAX) {
+    if (mg.L[l].n <= tail_cells &&
+        (pairs ? tail_image_bytes<T>(mg.L.data(), l, nl, mg.h16) > 0
+               : tail_smem_bytes<T>(mg.L.data(), l, nl, mg.h16) <= TAIL_SMEM_MAX)) {
       mg.tail = l;
       break;
     }
-  {
-    const size_t b = tail_smem_bytes<T>(mg.L.data(), mg.tail, nl, mg.h16);
-    mg.tail_smem = b <= TAIL_SMEM_MAX && env_ll("PFGPU_TAIL_SMEM", 1) ? b : 0;
-  }
+  if (tail_form<T>(h, mg)) return PFGPU_ERR_NOMEM;
+  mg.fuse_cells = env_ll("PFGPU_FUSE_CELLS", 400000);
   mg.flip = env_ll("PFGPU_FLIP", 1) != 0;
   // middle levels: the grid levels at or below PFGPU_MID_CELLS cells just
   // above the tail, when the device can co-schedule a cluster for them
@@ -1809,7 +1881,7 @@ static int alloc_mg(pfgpu_handle *h, MG<T> &mg) {
   // the residual after the pre-smoother: the colour swept last is solved
   // against its current neighbours, its residual zero up to rounding
   // (PFGPU_PAIR_RESIDUAL=0 computes it anyway)
-  const bool pair = env_ll("PFGPU_PAIR_RESIDUAL", 1) != 0;
+  const bool pair = mg_pairs_smoother(h);
   for (int l = 0; l < nl; l++) {
     const int sm = h->d.mg_smoother;
     // (the fused and wavefront smoothers run the same red/black/red sweeps)
@@ -1835,9 +1907,14 @@ static int mg_level0_on_grid(pfgpu_handle *h, MG<T> &mg) {
   MGLevel<T> &L0 = mg.L[0];
   if (nl > 1) {
     if (mg.tail < 1) {
+      // captured solves hold the old tail and its image
+      solve_graphs_forget(h);
       mg.tail = 1;
-      const size_t b = tail_smem_bytes<T>(mg.L.data(), 1, nl, mg.h16);
-      mg.tail_smem = b <= TAIL_SMEM_MAX && env_ll("PFGPU_TAIL_SMEM", 1) ? b : 0;
+      if (tail_form<T>(h, mg)) return PFGPU_ERR_NOMEM;
+      // the operators of an earlier setup, for a V-cycle before the next one
+      if (mg.tail_image)
+        launch_tail_pack<T>(mg.L.data(), mg.tail, nl, h->d.mg_smoother, mg.tail_image, h->st,
+                            mg.h16);
     }
     if (mg.mid < 1) mg.mid = 1;
   }
@@ -1900,6 +1977,8 @@ static void free_mg(MG<T> &mg) {
   mg.hflag = nullptr;
   cudaFree(mg.gbar);
   mg.gbar = nullptr;
+  cudaFree(mg.tail_image);
+  mg.tail_image = nullptr;
   mg.wave.clear();
   mg.L.clear();
 }
@@ -3560,7 +3639,7 @@ int pfgpu_time_kernel(pfgpu_handle *h, int kernel, int reps, double *ms, double 
         h->launches++;
         break;
       case PFGPU_KERNEL_MG_SETUP:
-        h->launches += h->mixed ? mg_setup_T<float>(h->mgf, h->st) : mg_setup_T<double>(h->mgd, h->st);
+        h->launches += h->mixed ? mg_setup_T<float>(h->mgf, h->d.mg_smoother, h->st) : mg_setup_T<double>(h->mgd, h->d.mg_smoother, h->st);
         break;
     }
   };

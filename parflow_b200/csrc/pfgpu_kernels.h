@@ -212,24 +212,31 @@ int launch_mg_smooth(const MGLevel<T> &L, T *x, const T *b, int zero, int smooth
                       bool h16 = false);
 cudaError_t mg_prepare_kernels();
 // h16: the level's scaled FP16 operator and weights (float levels only)
-template <typename T>
 // r = b - A x; zero_colour >= 0: right after a sweep of that colour, whose
 // cells' residual is written as zero
+template <typename T>
 void launch_mg_residual(const MGLevel<T> &L, const T *x, const T *b, T *r, cudaStream_t st,
                         int flip = 0, bool h16 = false, int zero_colour = -1);
+// init: also the zero-guess red sweep of C
 template <typename T>
 void launch_mg_restrict(const MGLevel<T> &F, const MGLevel<T> &C, const T *rf, T *rc,
-                        cudaStream_t st, int flip = 0, bool h16 = false);
+                        cudaStream_t st, int flip = 0, bool h16 = false, int init = 0);
+// both in one launch from F.x, F.b to C.b, after a red/black smoother (F.zc >= 0)
 template <typename T>
-// xf += P ec; skip_red: only the black cells (the next sweep is a red one)
+void launch_mg_resid_restrict(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st, int flip,
+                              bool h16, int init);
+// the level's pre-smoother takes a red sweep done by whoever writes its b
+// (launch_mg_smooth with zero = 2)
+template <typename T>
+bool mg_wants_red_init(const MGLevel<T> &L, int smoother, bool h16);
+// xf += P ec; black: only the black cells (the next sweep is a red one)
+template <typename T>
 void launch_mg_prolong_add(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, T *xf,
-                           cudaStream_t st, int flip = 0, bool h16 = false, int skip_red = 0);
+                           cudaStream_t st, int flip = 0, bool h16 = false, int black = 0);
 // scaled FP16 operator of level F from its FP32 operator and the diagonal of
 // the next coarser level C (null on the coarsest); sets *F.hflag when a
 // scaled diagonal is not +1 (the flag is cleared before the first level)
 void launch_h16_scale(const MGLevel<float> &F, const MGLevel<float> *C, cudaStream_t st);
-void launch_h16_scale_tail(const MGLevel<float> *levels_dev, int first, int nl,
-                           cudaStream_t st);
 // levels `first` .. nl-1 of a V-cycle / of the setup in one single-block
 // kernel; levels_dev is a device copy of the level table.  With smem > 0
 // (tail_smem_bytes of those levels, at most TAIL_SMEM_MAX) the V-cycle tail
@@ -271,13 +278,37 @@ cudaError_t launch_vcycle_grid(const MGLevel<T> *levels_dev, int mid, int tail, 
 // per SM (0 if the kernels cannot be launched cooperatively)
 template <typename T>
 int vcycle_grid_blocks(bool h16, int per_sm);
+// (mg_tail.cu) the same tail, a thread per pair of cells, for the red/black
+// smoothers with the paired residual (MGLevel::zc >= 0): it reads an image of
+// the tail levels' operators that launch_tail_pack fills after each setup.
+// tail_image_bytes: its size, 0 when these levels do not fit the kernel.
 template <typename T>
-void launch_setup_tail(const MGLevel<T> *levels_dev, int first, int nl, cudaStream_t st);
+size_t tail_image_bytes(const MGLevel<T> *levels_host, int first, int nl, bool h16);
+template <typename T>
+cudaError_t tail_pairs_prepare();
+template <typename T>
+void launch_tail_pack(const MGLevel<T> *levels_host, int first, int nl, int smoother, void *image,
+                      cudaStream_t st, bool h16);
+template <typename T>
+void launch_tail_pairs(const MGLevel<T> *levels_host, int first, int nl, int smoother, void *image,
+                       cudaStream_t st, bool h16);
+// setup of the tail levels (weights, coarse operators and, h16, their scaled
+// operators); returns the kernels launched
+constexpr size_t SETUP_TAIL_SMEM_MAX = 160 * 1024;
+constexpr long long SETUP_TAIL_CELLS = 2048;
+template <typename T>
+int launch_setup_tail(const MGLevel<T> *levels_host, const MGLevel<T> *levels_dev, int first,
+                      int nl, cudaStream_t st, bool h16);
 // a natural-layout FP64 vector r into b of level 0 / x of level 0 back into a
 // natural FP64 vector z, in the level's type and layout (times the FP16
 // scaling when scale is given); return the number of kernels launched
+// (init: with the zero-guess red sweep of the plain operator, where
+// level_in_inits says so)
 template <typename T>
-int launch_level_in(const MGLevel<T> &L, const double *r, const float *scale, cudaStream_t st);
+bool level_in_inits(const MGLevel<T> &L, int smoother, bool h16);
+template <typename T>
+int launch_level_in(const MGLevel<T> &L, const double *r, const float *scale, cudaStream_t st,
+                    int init);
 template <typename T>
 int launch_level_out(const MGLevel<T> &L, const T *x, double *z, const float *scale, int flip,
                      cudaStream_t st);

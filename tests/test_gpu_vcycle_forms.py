@@ -1,0 +1,83 @@
+"""The launch forms of one V-cycle give the same bits on grids where a form's
+index rules can go wrong: rows of one cell, odd and even rows, single planes,
+two-cell grids, levels around the sizes at which a form takes over.
+
+Default: the pair tail (levels of at most 1024 cells in one block), residual
+and restriction in one launch below PFGPU_FUSE_CELLS, the zero-guess red sweep
+done by whoever writes the right-hand side.  Compared with the generic tail in
+global memory (PFGPU_TAIL_SMEM=0), every level on the grid kernels
+(PFGPU_TAIL_CELLS=1), residual and restriction apart (PFGPU_FUSE_CELLS=0) and
+the natural layout of the iterates (PFGPU_SPLIT=0)."""
+
+import numpy as np
+import pytest
+
+from parflow_b200 import configs
+from parflow_b200.problem import SolverSettings
+
+pytestmark = pytest.mark.gpu
+
+ENV = ("PFGPU_TAIL_SMEM", "PFGPU_TAIL_CELLS", "PFGPU_FUSE_CELLS", "PFGPU_SPLIT")
+SHAPES = [(1, 1, 2), (2, 1, 1), (1, 37, 5), (2, 2, 2), (3, 5, 7), (16, 16, 4), (17, 15, 4),
+          (33, 31, 1), (1, 64, 33), (128, 3, 11), (65, 63, 9)]
+
+
+@pytest.fixture(scope="module")
+def solver():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for gpu tests")
+    from parflow_b200 import solver as s
+
+    return s
+
+
+def _pc(solver, prob, precision, monkeypatch, env):
+    for k in ENV:
+        monkeypatch.delenv(k, raising=False)
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    s = solver.RichardsGPU(prob, precision=precision)
+    rng = np.random.default_rng(11)
+    p = prob.initial_pressure() + 0.1 * rng.standard_normal(prob.shape)
+    s.pc_setup(p, prob.dt)
+    z = s.pc_apply(rng.standard_normal(prob.shape))
+    z2 = s.pc_apply(z)
+    s.close()
+    return np.concatenate([z.ravel(), z2.ravel()])
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed16"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_forms_bitwise_equal(solver, monkeypatch, shape, precision, symmetric):
+    nx, ny, nz = shape
+    prob = configs.box(nx=nx, ny=ny, nz=nz, nsteps=1,
+                       solver=SolverSettings(mg_smoother_symmetric=symmetric))
+    ref = _pc(solver, prob, precision, monkeypatch, {})
+    assert np.isfinite(ref).all() and np.abs(ref).max() > 0
+    for env in ({"PFGPU_TAIL_SMEM": "0"}, {"PFGPU_TAIL_CELLS": "1"}, {"PFGPU_FUSE_CELLS": "0"},
+                {"PFGPU_TAIL_CELLS": "1", "PFGPU_FUSE_CELLS": "0"}, {"PFGPU_SPLIT": "0"}):
+        z = _pc(solver, prob, precision, monkeypatch, env)
+        assert np.array_equal(z, ref), env
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed16"])
+def test_tail_moves_with_max_iter(solver, monkeypatch, precision):
+    """A grid that is all tail: MGSemi.MaxIter 2 takes level 0 out of it, back
+    to 1 leaves it out; the packed operators follow without a new setup."""
+    for k in ENV:
+        monkeypatch.delenv(k, raising=False)
+    prob = configs.box(nx=12, ny=10, nz=8, nsteps=1)
+    s = solver.RichardsGPU(prob, precision=precision)
+    rng = np.random.default_rng(12)
+    p = prob.initial_pressure() + 0.1 * rng.standard_normal(prob.shape)
+    r = rng.standard_normal(prob.shape)
+    s.pc_setup(p, prob.dt)
+    z = s.pc_apply(r)
+    assert s.lib.pfgpu_set_mg_max_iter(s.h, 2) == 0
+    s.pc_apply(r)
+    assert s.lib.pfgpu_set_mg_max_iter(s.h, 1) == 0
+    assert np.array_equal(s.pc_apply(r), z)
+    s.close()
