@@ -97,12 +97,27 @@ __device__ __forceinline__ void tfg_face_y(const DevProblem &P, int i, int j, do
   gc = 0.5 * (__ldg(P.tfg_yc + a) + (in ? __ldg(P.tfg_yc + a + P.nx) : g * 1.0));
 }
 
+// 1/x: the hardware's approximation (rcp.approx.ftz.f64, some 20 bits) and two
+// Newton-Raphson steps y += y (1 - x y), each squaring the relative error;
+// within 2 ulp of the division at a third of its instructions.  Operands near
+// the ends of the exponent range take the division.
+__device__ __forceinline__ double fast_rcp(double x) {
+  // exponent field outside 24 .. 2022: zero, tiny, huge, infinite, NaN
+  if (((unsigned)__double2hiint(x) >> 20 & 0x7ffu) - 24u > 1998u) return 1.0 / x;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(fma(-x, y, 1.0), y, y);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+
 // ParFlow's mean macros (pfsimulator/parflow_lib/solver.h:42-47)
 __device__ __forceinline__ double harmonic(double a, double b) {
-  return (a + b) ? (2.0 * a * b) / (a + b) : 0.0;
+  const double den = a + b;
+  return den ? __dmul_rn(__dmul_rn(__dmul_rn(2.0, a), b), fast_rcp(den)) : 0.0;
 }
 __device__ __forceinline__ double harmonic_dz(double a, double b, double c, double d) {
-  return ((c * b) + (a * d)) ? (((c + d) * a * b) / ((b * c) + (a * d))) : 0.0;
+  const double den = fma(b, c, __dmul_rn(a, d));
+  return den ? __dmul_rn(__dmul_rn(__dmul_rn(c + d, a), b), fast_rcp(den)) : 0.0;
 }
 __device__ __forceinline__ double upstream(double a, double b, double c, double d) {
   return ((a - b) >= 0) ? c : d;
@@ -185,17 +200,18 @@ __device__ __forceinline__ double vg_dkr(const DevProblem &P, double p, double a
          (coeff * coeff) * (m / 2) * pow(opahn, (-(m + 2) / 2)) * n * alpha * ahnm1;
 }
 
-// All four van Genuchten quantities of one cell from one log(alpha h) and one
-// log1p((alpha h)^n): every power of the reference formulas
+// All four van Genuchten quantities of one cell from log(alpha h) and
+// log(1 + (alpha h)^n): every power of the reference formulas
 // (problem_saturation.c:221-415, problem_phase_rel_perm.c:788, :981) comes
-// from two exponentials of these logarithms, one reciprocal of alpha h (for
-// the (alpha h)^(n-1), (alpha h)^(n-2) factors), one reciprocal of
-// 1 + (alpha h)^n and one square root ((1+A)^(-m/2) = sqrt((1+A)^(-m))).
+// from two exponentials of these logarithms ((1+A)^(-m/2), squared for
+// (1+A)^-m), a reciprocal of alpha h (for the (alpha h)^(n-1), (alpha h)^(n-2)
+// factors) and one of 1 + (alpha h)^n.  inv_rg = 1 / (density gravity), m = 1 - 1/n.
 struct VGAll {
   double kr, dkr, s, ds;
 };
 
-__device__ __forceinline__ VGAll vg_all(const DevProblem &P, double p, const VG &v) {
+__device__ __forceinline__ VGAll vg_all(const DevProblem &P, double p, const VG &v, double inv_rg,
+                                        double m) {
   VGAll r;
   const double s_dif = v.ssat - v.sres;
   if (p >= 0.0) {
@@ -206,24 +222,21 @@ __device__ __forceinline__ VGAll vg_all(const DevProblem &P, double p, const VG 
     return r;
   }
   const double n = v.n, alpha = v.alpha;
-  const double m = 1.0 - (1.0 / n);
-  const double head = fabs(p) / (P.density * P.gravity);
-  const double ah = alpha * head;
-  const double ahn = exp(n * log(ah));     // (alpha h)^n
-  const double inv_ah = 1.0 / ah;
-  const double ahnm1 = ahn * inv_ah;       // (alpha h)^(n-1)
-  const double ahnm2 = ahnm1 * inv_ah;     // (alpha h)^(n-2)
-  const double lop = log1p(ahn);           // log(1 + (alpha h)^n)
-  const double inv_opm = exp(-m * lop);    // opahn^-m
-  const double inv_opm2 = sqrt(inv_opm);   // opahn^(-m/2)
-  const double inv_op = 1.0 / (1.0 + ahn);
+  const double ah = alpha * (fabs(p) * inv_rg);
+  const double ahn = exp(n * log(ah));          // (alpha h)^n
+  const double inv_ah = fast_rcp(ah);
+  const double ahnm1 = ahn * inv_ah;            // (alpha h)^(n-1)
+  const double op = 1.0 + ahn;
+  const double inv_opm2 = exp(-0.5 * m * log(op));  // op^(-m/2)
+  const double inv_opm = inv_opm2 * inv_opm2;   // op^-m
+  const double inv_op = fast_rcp(op);
   const double t = 1.0 - ahnm1 * inv_opm;
+  const double na1 = n * alpha * ahnm1, mq = m * (inv_opm * inv_op) * na1;
   r.kr = (t * t) * inv_opm2;
-  r.dkr = 2.0 * (t * inv_opm2) *
-              ((n - 1) * ahnm2 * alpha * inv_opm - ahnm1 * m * (inv_opm * inv_op) * n * alpha * ahnm1) +
-          (t * t) * (m / 2) * (inv_opm2 * inv_op) * n * alpha * ahnm1;
+  r.dkr = 2.0 * (t * inv_opm2) * ((n - 1) * (ahnm1 * inv_ah) * alpha * inv_opm - ahnm1 * mq) +
+          (t * t) * (0.5 * m) * (inv_opm2 * inv_op) * na1;
   r.s = s_dif * inv_opm + v.sres;
-  r.ds = (m * n * alpha * ahnm1) * s_dif * (inv_opm * inv_op);
+  r.ds = s_dif * mq;
   return r;
 }
 
@@ -244,44 +257,36 @@ __device__ __forceinline__ double fb_z(const DevProblem &P, long long c) {
   return P.fbz ? __ldg(P.fbz + c) : 1.0;
 }
 
-__device__ __forceinline__ double flux_x(const DevProblem &P, double pa, double pb, double ka,
-                                         double kb, double kra, double krb, double zm,
-                                         double x_dir_g, double x_dir_g_c) {
-  double diff_l = pa - pb;
-  double updir = (diff_l * P.inv_dx) * x_dir_g_c - x_dir_g;
-  double km = harmonic(ka, kb);
-  double up = upstream(updir, 0.0, kra * P.density, krb * P.density);
-  double ffx = P.dy * P.dz;
-  double u = zm * ffx * 1.0 * km * (diff_l * P.inv_dx) * x_dir_g_c * up * P.inv_visc;
-  u += zm * ffx * 1.0 * km * (-x_dir_g) * up * P.inv_visc;
-  return u;
+// The driving gradient appears twice in the reference's expression, as the
+// upwind decision and as the sum of the pressure and gravity terms; here it is
+// formed once.  cx, cy, cz: the face's constant factor area rho / viscosity.
+struct FluxConst {
+  double cx, cy, cz;
+};
+__device__ __forceinline__ FluxConst flux_const(const DevProblem &P) {
+  const double q = P.density * P.inv_visc;
+  return FluxConst{P.dy * P.dz * q, P.dx * P.dz * q, P.dx * P.dy * q};
 }
-
-__device__ __forceinline__ double flux_y(const DevProblem &P, double pa, double pb, double ka,
-                                         double kb, double kra, double krb, double zm,
-                                         double y_dir_g, double y_dir_g_c) {
-  double diff_l = pa - pb;
-  double updir = (diff_l * P.inv_dy) * y_dir_g_c - y_dir_g;
-  double km = harmonic(ka, kb);
-  double up = upstream(updir, 0.0, kra * P.density, krb * P.density);
-  double ffy = P.dx * P.dz;
-  double u = zm * ffy * 1.0 * km * (diff_l * P.inv_dy) * y_dir_g_c * up * P.inv_visc;
-  u += zm * ffy * 1.0 * km * (-y_dir_g) * up * P.inv_visc;
-  return u;
+// x or y face with its spacing's reciprocal (inv_d) and constant (c)
+__device__ __forceinline__ double flux_xy(double inv_d, double c, double pa, double pb, double ka,
+                                          double kb, double kra, double krb, double zm,
+                                          double dir_g, double dir_g_c) {
+  const double drive = fma(__dmul_rn(pa - pb, inv_d), dir_g_c, -dir_g);
+  return __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(c, zm), harmonic(ka, kb)), drive),
+                   (drive >= 0.0) ? kra : krb);
 }
 
 // z face between layer k (a, below) and k+1 (b, above)
-__device__ __forceinline__ double flux_z(const DevProblem &P, double pa, double pb, double ka,
-                                         double kb, double kra, double krb, double za,
+__device__ __forceinline__ double flux_z(const DevProblem &P, double c, double pa, double pb,
+                                         double ka, double kb, double kra, double krb, double za,
                                          double zb, int k) {
-  const double g = P.gravity, rho = P.density;
+  const double rg = P.density * P.gravity;
   const double inv_sep = __ldg(P.zface + 3 * k);
-  double lower = pa * inv_sep - __ldg(P.zface + 3 * k + 1) * rho * g * 1.0;
-  double upper = pb * inv_sep + __ldg(P.zface + 3 * k + 2) * rho * g * 1.0;
-  double diff_l = lower - upper;
-  double ffz = P.dx * P.dy;
-  return ffz * 1.0 * 1.0 * harmonic_dz(ka, kb, za, zb) * diff_l *
-         upstream(lower, upper, kra * rho, krb * rho) * P.inv_visc;
+  const double lower = fma(pa, inv_sep, -__dmul_rn(__ldg(P.zface + 3 * k + 1), rg));
+  const double upper = fma(pb, inv_sep, __dmul_rn(__ldg(P.zface + 3 * k + 2), rg));
+  const double drive = lower - upper;
+  return __dmul_rn(__dmul_rn(__dmul_rn(c, harmonic_dz(ka, kb, za, zb)), drive),
+                   (drive >= 0.0) ? kra : krb);
 }
 
 // ---------------------------------------------------------------------------

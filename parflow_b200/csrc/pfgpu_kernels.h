@@ -39,6 +39,10 @@ struct PCOut {
 
 void launch_vg_all(const DevProblem &P, const double *p, double *kr, double *dkr, double *sat,
                    double *dsat, cudaStream_t st);
+// the same at unew = u + lam pp (lam from lam_p when given), which is written
+void launch_vg_step(const DevProblem &P, const double *u, const double *pp, const double *lam_p,
+                    double lam, double *unew, double *kr, double *dkr, double *sat, double *dsat,
+                    cudaStream_t st);
 void launch_saturation(const DevProblem &P, const double *p, double *s, cudaStream_t st);
 // vel: also write the face velocities and overland fluxes (null: F only)
 void launch_residual(const DevProblem &P, const double *p, const double *p_old,

@@ -1,9 +1,10 @@
 // Richards residual, analytic Jacobian assembly and stencil matvec.
 //
-// Gather form: every cell computes the fluxes (or flux derivatives) of its
-// own six faces; a face shared by two cells is evaluated by both with the
-// same operands in the same order, so both see identical bits and no atomics
-// are needed.  Per-cell relative permeabilities are produced by a first pass
+// Two launch forms, bitwise equal.  Gather: every cell computes the fluxes (or
+// flux derivatives) of its own six faces; a face shared by two cells is
+// evaluated by both with the same operands in the same order.  March: a warp
+// walks a strip of rows up through the planes and evaluates (almost) every
+// face once.  Neither needs atomics.  Per-cell relative permeabilities are produced by a first pass
 // (k_vg_all) so that each cell's van Genuchten state is evaluated once per
 // iterate and shared by the residual and the Jacobian.
 #include "pfgpu_device.cuh"
@@ -24,18 +25,34 @@ __device__ __forceinline__ bool launch_ijk(int nx, int ny, int nz, int &i, int &
 // Van Genuchten state of every cell at one pressure iterate: kr, dkr/dp, S,
 // dS/dp (problem_phase_rel_perm.c:1312-1361, problem_saturation.c:342-412).
 // The residual uses kr and S; the Jacobian at the same iterate reuses all four.
-// Launch bounds: these FP64 kernels are latency-bound at the occupancy their
-// natural register use allows; capping registers (a few spilled bytes stay in
-// L1) for 5 (8) resident blocks per SM cuts their time by about 30%.
-__global__ void __launch_bounds__(256, 5) k_vg_all(DevProblem P, const double *__restrict__ p, double *__restrict__ kr,
+// STEP: the iterate is formed here, pn = u + lam pp (lam from lam_p when
+// given), and written too, which is free: the pass is bound by instruction
+// issue (exp and log), not by memory.
+// 512x512x50: 136 us (memory floor 79 us) against 192 with the logarithms and
+// powers of the reference one by one, a division per reciprocal and per n.
+// q: 1/(rho g), and m = 1 - 1/n of a uniform n
+struct VGUniform {
+  double inv_rg, m;
+};
+template <bool STEP>
+__global__ void __launch_bounds__(256, 5) k_vg_all(DevProblem P, VGUniform q,
+                         const double *__restrict__ p, double *__restrict__ kr,
                          double *__restrict__ dkr, double *__restrict__ sat,
-                         double *__restrict__ dsat) {
-  pdl_enter();
-  long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+                         double *__restrict__ dsat, const double *__restrict__ pp,
+                         const double *lam_p, double lam, double *__restrict__ pn) {
+  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= P.n) return;
-  VGAll v = vg_all(P, p[c], vg_at(P, c));
+  const VG vg = vg_at(P, c);  // (fields: older than the kernel before this one)
+  const double m = P.vgn ? 1.0 - fast_rcp(vg.n) : q.m;
+  pdl_enter();
+  double pc = p[c];
+  if (STEP) {
+    const double a = lam_p ? *lam_p : lam;
+    if (a != 0.0) pc = pc + a * pp[c];
+    pn[c] = pc;
+  }
+  VGAll v = vg_all(P, pc, vg, q.inv_rg, m);
   if (P.krt) {  // relative permeability from the lookup table
-    const double pc = p[c];
     if (pc >= 0.0) {
       v.kr = 1.0;
       v.dkr = 0.0;
@@ -51,11 +68,14 @@ __global__ void __launch_bounds__(256, 5) k_vg_all(DevProblem P, const double *_
   dsat[c] = v.ds;
 }
 
-__global__ void k_saturation(DevProblem P, const double *__restrict__ p, double *__restrict__ s) {
-  pdl_enter();
-  long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void k_saturation(DevProblem P, VGUniform q, const double *__restrict__ p,
+                             double *__restrict__ s) {
+  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= P.n) return;
-  s[c] = vg_all(P, p[c], vg_at(P, c)).s;
+  const VG vg = vg_at(P, c);
+  const double m = P.vgn ? 1.0 - fast_rcp(vg.n) : q.m;
+  pdl_enter();
+  s[c] = vg_all(P, p[c], vg, q.inv_rg, m).s;
 }
 
 // Residual (nl_function_eval.c:167-2323).  Accumulation order per cell
@@ -74,33 +94,38 @@ __global__ void k_saturation(DevProblem P, const double *__restrict__ p, double 
 // (0 on the domain's upper faces).  Both launch forms below pass the values
 // of the same flux functions with the same operands, so their F is equal
 // bit for bit.
+// ponding and routing term of an overland top cell: the change of the ponded
+// depth and the divergence of the routed flux
+__device__ __forceinline__ double ponding(const DevProblem &P, double dt, double vol, double pc,
+                                          double po, double dqx, double dqy) {
+  const double div = __dadd_rn(dqx / P.dx, dqy / P.dy);
+  return __dadd_rn(__dmul_rn(vol, pmax0(pc) - pmax0(po)) / P.dz,
+                   __dmul_rn(__dmul_rn(dt, vol), div) / P.dz);
+}
+
 template <bool SURF, bool VEL>
 __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j, int k,
                                               long long c, const double *__restrict__ p,
-                                              const double *__restrict__ p_old,
-                                              const double *__restrict__ s_old,
-                                              const double *__restrict__ kr,
-                                              const double *__restrict__ satv, double dt,
+                                              const double *__restrict__ p_old, double dt,
                                               double *__restrict__ f, const VelOut &V,
-                                              double fl_z, double fl_y, double fl_x,
+                                              double pc, double krc, double sat, double so,
+                                              double po, double zm, double fl_z, double fl_y, double fl_x,
                                               double u_right, double u_front, double u_upper) {
   const long long sz = (long long)P.nx * P.ny;
   const double rho = P.density, g = P.gravity;
   const double vol = P.dx * P.dy * P.dz;
-  const double zm = __ldg(P.zmult + k);
-  const double pc = p[c];
-  const double sat = satv[c];
-  const double so = s_old[c];
-  double fc = (sat * rho - so * rho) * P.porosity * vol * 1.0 * 1.0 * zm;
-  fc += P.sstorage * vol * 1.0 * 1.0 * zm * (pc * sat * rho - p_old[c] * so * rho);
-  fc -= vol * 1.0 * 1.0 * zm * dt * (0.0 + (P.et ? __ldg(P.et + c) : 0.0));
-  const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
-  const double krc = kr[c];
+  // (multiply-adds written out here and in the fluxes, so that every launch
+  // form rounds alike)
+  const double vz = vol * zm;
+  double fc = __dmul_rn(__dmul_rn(__dmul_rn(sat, rho) - __dmul_rn(so, rho), P.porosity), vz);
+  fc = fma(__dmul_rn(P.sstorage, vz),
+           __dmul_rn(__dmul_rn(pc, sat), rho) - __dmul_rn(__dmul_rn(po, so), rho), fc);
+  if (P.et) fc = fma(-__dmul_rn(vz, dt), __ldg(P.et + c), fc);
   // neighbours' scatter (reference loop order: plane k-1, row j-1, cell i-1)
-  if (k > 0) fc += -dt * fl_z;
-  if (j > 0) fc += -dt * fl_y;
-  if (i > 0) fc += -dt * fl_x;
-  fc += dt * (u_right + u_front + u_upper);
+  fc = fma(-dt, fl_z, fc);
+  fc = fma(-dt, fl_y, fc);
+  fc = fma(-dt, fl_x, fc);
+  fc = fma(dt, u_right + u_front + u_upper, fc);
   if (VEL) {
     const long long fx1 = (long long)(P.nx + 1), cyz = (long long)P.nx * (P.ny + 1);
     if (V.vx && i + 1 < P.nx)
@@ -150,8 +175,7 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
       } else if (o.sfy > 0.0) {  // outflow through the lower y edge
         ks = -(o.sfy / (o.sq * o.n)) * pow(pmax0(pc), (5.0 / 3.0));
       }
-      const double q_ov = vol * (pmax0(pc) - pmax0(p_old[c])) / P.dz +
-                          dt * vol * ((ke - kw) / P.dx + (kn - ks) / P.dy) / P.dz;
+      const double q_ov = ponding(P, dt, vol, pc, po, ke - kw, kn - ks);
       fc += q_ov;
       u_new = ffz * value;
       if (VEL) {
@@ -170,11 +194,10 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
       const double qs = ovf_q<false>(P, p, i, j - 1), qm = ovf_q<false>(P, p, i, j),
                    qn = ovf_q<false>(P, p, i, j + 1);
       const double ks = pmax0(qs) - pmax0(-qm), kn = pmax0(qm) - pmax0(-qn);
-      double q_ov = vol * (pmax0(pc) - pmax0(p_old[c])) / P.dz +
-                    dt * vol * ((ke - kw) / P.dx + (kn - ks) / P.dy) / P.dz;
+      double q_ov = ponding(P, dt, vol, pc, po, ke - kw, kn - ks);
       if (P.ov_p2 != 0.0 || P.ov_spinup == 1) {
         const double damp = exp(fmin(pc, 0.0) * P.ov_p1) * P.ov_p2;
-        q_ov = q_ov + vol * dt / P.dz * damp;
+        q_ov = fma(vol * dt / P.dz, damp, q_ov);
         if (P.ov_spinup == 1) q_ov = (vol / P.dz) * dt * ((pmax0(pc) - 0.0) + damp);
       }
       fc += q_ov;
@@ -193,8 +216,7 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
       const double ke = ovd_qx(o), kn = ovd_qy(o);
       const double kw = i > 0 ? ovd_qx(ovd_col(P, p, i - 1, j)) : qxw;
       const double ks = j > 0 ? ovd_qy(ovd_col(P, p, i, j - 1)) : qys;
-      const double q_ov = vol * (pmax0(pc) - pmax0(p_old[c])) / P.dz +
-                          dt * vol * ((ke - kw) / P.dx + (kn - ks) / P.dy) / P.dz;
+      const double q_ov = ponding(P, dt, vol, pc, po, ke - kw, kn - ks);
       fc += q_ov;
       u_new = ffz * value;
       if (VEL) {
@@ -207,7 +229,7 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
       double krg = vg_kr(P, value, v.alpha, v.n);
       if (face < 4) {
         double h = (face < 2) ? ffx * zm : ffy * zm;
-        double kk = (face < 2) ? kxc : kyc;
+        double kk = __ldg((face < 2 ? P.kx : P.ky) + c);
         double dd = (face < 2) ? P.dx : P.dy;
         if (dir < 0) {
           double diff = value - pc;
@@ -230,12 +252,12 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
           upper = (value / sep) + 0.25 * rho * g * 1.0;
           u_new = upstream(lower, upper, krc * rho, krg * rho);
         }
-        u_new = u_new * ffz * (kzc * P.inv_visc) * 2.0 * (lower - upper);
+        u_new = u_new * ffz * (__ldg(P.kz + c) * P.inv_visc) * 2.0 * (lower - upper);
       }
       // DirichletBC: u_new / h (nl_function_eval.c:1227-1230)
       if (VEL) vel = u_new / ((face < 2) ? ffx * zm : (face < 4) ? ffy * zm : ffz);
     }
-    fc += dt * dir * u_new;
+    fc = fma(dt * dir, u_new, fc);
     if (VEL) {
       const int up = face & 1;
       if (face < 2 && V.vx)
@@ -264,6 +286,7 @@ __global__ void __launch_bounds__(256, 5) k_residual(DevProblem P, const double 
   const long long c = i + (long long)P.nx * (j + (long long)P.ny * k);
   const long long sy = P.nx, sz = (long long)P.nx * P.ny;
   const double g = P.gravity;
+  const FluxConst A = flux_const(P);
   const double zm = __ldg(P.zmult + k);
   const double pc = p[c];
   const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
@@ -272,123 +295,136 @@ __global__ void __launch_bounds__(256, 5) k_residual(DevProblem P, const double 
   if (k > 0) {
     long long l = c - sz;
     double zl = __ldg(P.zmult + k - 1);
-    fl_z = flux_z(P, p[l], pc, __ldg(P.kz + l), kzc, kr[l], krc, zl, zm, k - 1);
+    fl_z = flux_z(P, A.cz, p[l], pc, __ldg(P.kz + l), kzc, kr[l], krc, zl, zm, k - 1);
     if (P.fbz) fl_z = fl_z * fb_z(P, l);
   }
-  double gs = 0.5 * (g * 0.0 + g * 0.0), gc = 0.5 * (g * 1.0 + g * 1.0);
+  double gs = 0.0, gc = g;
   if (j > 0) {
     long long s = c - sy;
     if (SURF) tfg_face_y(P, i, j - 1, gs, gc);
-    fl_y = flux_y(P, p[s], pc, __ldg(P.ky + s), kyc, kr[s], krc, zm, gs, gc);
+    fl_y = flux_xy(P.inv_dy, A.cy, p[s], pc, __ldg(P.ky + s), kyc, kr[s], krc, zm, gs, gc);
     if (P.fby) fl_y = fl_y * fb_y(P, s);
   }
   if (i > 0) {
     long long w = c - 1;
     if (SURF) tfg_face_x(P, i - 1, j, gs, gc);
-    fl_x = flux_x(P, p[w], pc, __ldg(P.kx + w), kxc, kr[w], krc, zm, gs, gc);
+    fl_x = flux_xy(P.inv_dx, A.cx, p[w], pc, __ldg(P.kx + w), kxc, kr[w], krc, zm, gs, gc);
     if (P.fbx) fl_x = fl_x * fb_x(P, w);
   }
   double u_right = 0.0, u_front = 0.0, u_upper = 0.0;
   if (i + 1 < P.nx) {
     long long e = c + 1;
     if (SURF) tfg_face_x(P, i, j, gs, gc);
-    u_right = flux_x(P, pc, p[e], kxc, __ldg(P.kx + e), krc, kr[e], zm, gs, gc);
+    u_right = flux_xy(P.inv_dx, A.cx, pc, p[e], kxc, __ldg(P.kx + e), krc, kr[e], zm, gs, gc);
     if (P.fbx) u_right = u_right * fb_x(P, c);
   }
   if (j + 1 < P.ny) {
     long long nn = c + sy;
     if (SURF) tfg_face_y(P, i, j, gs, gc);
-    u_front = flux_y(P, pc, p[nn], kyc, __ldg(P.ky + nn), krc, kr[nn], zm, gs, gc);
+    u_front = flux_xy(P.inv_dy, A.cy, pc, p[nn], kyc, __ldg(P.ky + nn), krc, kr[nn], zm, gs, gc);
     if (P.fby) u_front = u_front * fb_y(P, c);
   }
   if (k + 1 < P.nz) {
     long long u = c + sz;
-    u_upper = flux_z(P, pc, p[u], kzc, __ldg(P.kz + u), krc, kr[u], zm,
+    u_upper = flux_z(P, A.cz, pc, p[u], kzc, __ldg(P.kz + u), krc, kr[u], zm,
                      __ldg(P.zmult + k + 1), k);
     if (P.fbz) u_upper = u_upper * fb_z(P, c);
   }
-  residual_cell<SURF, VEL>(P, i, j, k, c, p, p_old, s_old, kr, satv, dt, f, V, fl_z, fl_y, fl_x,
-                           u_right, u_front, u_upper);
+  residual_cell<SURF, VEL>(P, i, j, k, c, p, p_old, dt, f, V, pc, krc, satv[c], s_old[c],
+                           p_old[c], zm, fl_z, fl_y, fl_x, u_right, u_front, u_upper);
 }
 
-// Face-once form: a block owns a (blockDim.x x blockDim.y) column tile of
-// planes k0 .. k0+kchunk-1 and walks up through them.  Each cell evaluates
-// only its right, front and upper faces; the right / front fluxes go to shared
-// memory for the neighbour in the tile, the upper flux stays in a register as
-// the lower flux of the next plane.  The tile's west / south edge faces and
-// the chunk's first lower faces are evaluated by the cells on those edges.
-// Every flux is the same function of the same operands as in the gather form.
-// Shared memory: blockDim.y x (blockDim.x + 1) right fluxes and
-// (blockDim.y + 1) x blockDim.x front fluxes.
-template <bool SURF, bool VEL = false>
-__global__ void __launch_bounds__(256) k_residual_zm(DevProblem P, const double *__restrict__ p,
-                           const double *__restrict__ p_old, const double *__restrict__ s_old,
-                           const double *__restrict__ kr, const double *__restrict__ satv,
-                           double dt, double *__restrict__ f, VelOut V, int kchunk) {
-  extern __shared__ double zm_smem[];
-  const int bx = blockDim.x, by = blockDim.y, tx = threadIdx.x, ty = threadIdx.y;
-  double *sE = zm_smem;                    // [by][bx + 1]: sE[ty][tx + 1] = right face of (tx, ty)
-  double *sN = zm_smem + by * (bx + 1);    // [by + 1][bx]: sN[ty + 1][tx] = front face
+// March form (one permeability field for the three directions, no face
+// velocities): a warp owns 32 columns of a row and walks up through planes
+// k0 .. k0 + kchunk - 1.  Lane l holds column i = 31 w + l - 1; it evaluates the
+// east face of its column, which the next lane takes by a shuffle as its west
+// face (lane 0 only provides), both y faces, and the upper z face, which stays
+// in a register as the lower one of the next plane: four faces per cell instead
+// of six and half the loads, with no barrier and no shared memory.  Every flux
+// is the same function of the same operands as in the gather form.
+// The gather form is bound by instruction issue and the latency its occupancy
+// leaves; 512x512x50: 232 us against 311 (memory floor 112 us, 56 B per cell).
+// Four blocks of 64 registers per SM; three (five) give 267 (250) us; with the
+// slopes of a terrain-following grid, which need more registers, three give 45
+// us at 256x256x20, four 51, gather 54.  Two rows per warp (3.6 faces per cell,
+// 96 registers) were slower than gather: 20 warps per SM hide too little.
+constexpr int MARCH_WARPS = 8, MARCH_COLS = 31;
+constexpr long long MARCH_MIN_CELLS = 600000;
+
+// a column's value of one plane
+struct MCell {
+  double p, k, kr;
+};
+__device__ __forceinline__ MCell mcell(const DevProblem &P, const double *__restrict__ p,
+                                       const double *__restrict__ kr, int c) {
+  return MCell{p[c], __ldg(P.kx + c), kr[c]};
+}
+
+template <bool SURF>
+__global__ void __launch_bounds__(32 * MARCH_WARPS, SURF ? 3 : 4) k_residual_march(
+    DevProblem P, const double *__restrict__ p, const double *__restrict__ p_old,
+    const double *__restrict__ s_old, const double *__restrict__ kr,
+    const double *__restrict__ satv, double dt, double *__restrict__ f, int kchunk) {
   pdl_enter();
   if (P.dtp) dt = *P.dtp;
-  const int i = blockIdx.x * bx + tx, j = blockIdx.y * by + ty;
-  const int k0 = blockIdx.z * kchunk, k1 = min(P.nz, k0 + kchunk);
-  const bool in = i < P.nx && j < P.ny;
-  const long long sy = P.nx, sz = (long long)P.nx * P.ny;
-  const double g = P.gravity;
-  // gravity terms of this column's faces (constant through the planes)
-  double gsw = 0.5 * (g * 0.0 + g * 0.0), gcw = 0.5 * (g * 1.0 + g * 1.0);
-  double gss = gsw, gcs = gcw, gse = gsw, gce = gcw, gsn = gsw, gcn = gcw;
-  if (SURF && in) {
-    if (i > 0) tfg_face_x(P, i - 1, j, gsw, gcw);
-    if (j > 0) tfg_face_y(P, i, j - 1, gss, gcs);
-    if (i + 1 < P.nx) tfg_face_x(P, i, j, gse, gce);
-    if (j + 1 < P.ny) tfg_face_y(P, i, j, gsn, gcn);
+  const int lane = threadIdx.x, nx = P.nx, ny = P.ny, nz = P.nz;
+  const int j = blockIdx.y * MARCH_WARPS + threadIdx.y;
+  if (j >= ny) return;
+  const int i = blockIdx.x * MARCH_COLS + lane - 1;
+  const int k0 = blockIdx.z * kchunk, k1 = min(nz, k0 + kchunk);
+  const bool in = i >= 0 && i < nx, out = in && lane > 0, east = in && i + 1 < nx;
+  const bool south = j > 0, north = j + 1 < ny;
+  const int ii = in ? i : (i < 0 ? 0 : nx - 1), sz = nx * ny;
+  const FluxConst A = flux_const(P);
+  const VelOut V{};
+  // gravity terms of the column's faces (constant through the planes)
+  double gse = 0.0, gce = P.gravity, gss = 0.0, gcs = P.gravity, gsn = 0.0, gcn = P.gravity;
+  if (SURF) {
+    if (east) tfg_face_x(P, ii, j, gse, gce);
+    if (south) tfg_face_y(P, ii, j - 1, gss, gcs);
+    if (north) tfg_face_y(P, ii, j, gsn, gcn);
   }
-  long long c = i + (long long)P.nx * (j + (long long)P.ny * k0);
-  double fl_z = 0.0;
-  if (in && k0 > 0 && k0 < k1)
-    fl_z = flux_z(P, p[c - sz], p[c], __ldg(P.kz + c - sz), __ldg(P.kz + c), kr[c - sz], kr[c],
-                  __ldg(P.zmult + k0 - 1), __ldg(P.zmult + k0), k0 - 1) *
-           fb_z(P, c - sz);
+  int c = ii + nx * (j + ny * k0);
+  MCell q = mcell(P, p, kr, c);
+  double lz = 0.0, zm = __ldg(P.zmult + k0);
+  if (k0 > 0) {
+    const MCell a = mcell(P, p, kr, c - sz);
+    lz = flux_z(P, A.cz, a.p, q.p, a.k, q.k, a.kr, q.kr, __ldg(P.zmult + k0 - 1), zm, k0 - 1);
+    if (P.fbz) lz = lz * fb_z(P, c - sz);
+  }
   for (int k = k0; k < k1; k++, c += sz) {
-    double u_right = 0.0, u_front = 0.0, u_upper = 0.0;
-    if (in) {
-      const double zm = __ldg(P.zmult + k);
-      const double pc = p[c];
-      const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
-      const double krc = kr[c];
-      if (i + 1 < P.nx)
-        u_right = flux_x(P, pc, p[c + 1], kxc, __ldg(P.kx + c + 1), krc, kr[c + 1], zm, gse,
-                         gce) *
-                  fb_x(P, c);
-      if (j + 1 < P.ny)
-        u_front = flux_y(P, pc, p[c + sy], kyc, __ldg(P.ky + c + sy), krc, kr[c + sy], zm, gsn,
-                         gcn) *
-                  fb_y(P, c);
-      if (k + 1 < P.nz)
-        u_upper = flux_z(P, pc, p[c + sz], kzc, __ldg(P.kz + c + sz), krc, kr[c + sz], zm,
-                         __ldg(P.zmult + k + 1), k) *
-                  fb_z(P, c);
-      // the tile's west and south edge faces
-      if (tx == 0 && i > 0)
-        sE[ty * (bx + 1)] = flux_x(P, p[c - 1], pc, __ldg(P.kx + c - 1), kxc, kr[c - 1], krc, zm,
-                                   gsw, gcw) *
-                            fb_x(P, c - 1);
-      if (ty == 0 && j > 0)
-        sN[tx] = flux_y(P, p[c - sy], pc, __ldg(P.ky + c - sy), kyc, kr[c - sy], krc, zm, gss,
-                        gcs) *
-                 fb_y(P, c - sy);
+    const bool up = k + 1 < nz;
+    const double zu = up ? __ldg(P.zmult + k + 1) : zm;
+    // every operand first
+    const MCell n = mcell(P, p, kr, up ? c + sz : c);
+    const MCell e = mcell(P, p, kr, east ? c + 1 : c);
+    const MCell s = mcell(P, p, kr, south ? c - nx : c);
+    const MCell t = mcell(P, p, kr, north ? c + nx : c);
+    const double sat = satv[c], so = s_old[c], po = p_old[c];
+    double ux = 0.0, us = 0.0, un = 0.0, uz = 0.0;
+    if (east) {
+      ux = flux_xy(P.inv_dx, A.cx, q.p, e.p, q.k, e.k, q.kr, e.kr, zm, gse, gce);
+      if (P.fbx) ux = ux * fb_x(P, c);
     }
-    sE[ty * (bx + 1) + tx + 1] = u_right;
-    sN[(ty + 1) * bx + tx] = u_front;
-    __syncthreads();
-    if (in)
-      residual_cell<SURF, VEL>(P, i, j, k, c, p, p_old, s_old, kr, satv, dt, f, V, fl_z,
-                               sN[ty * bx + tx], sE[ty * (bx + 1) + tx], u_right, u_front,
-                               u_upper);
-    fl_z = u_upper;
-    __syncthreads();
+    const double wx = __shfl_up_sync(0xffffffffu, ux, 1);
+    if (south) {
+      us = flux_xy(P.inv_dy, A.cy, s.p, q.p, s.k, q.k, s.kr, q.kr, zm, gss, gcs);
+      if (P.fby) us = us * fb_y(P, c - nx);
+    }
+    if (north) {
+      un = flux_xy(P.inv_dy, A.cy, q.p, t.p, q.k, t.k, q.kr, t.kr, zm, gsn, gcn);
+      if (P.fby) un = un * fb_y(P, c);
+    }
+    if (up) {
+      uz = flux_z(P, A.cz, q.p, n.p, q.k, n.k, q.kr, n.kr, zm, zu, k);
+      if (P.fbz) uz = uz * fb_z(P, c);
+    }
+    if (out)
+      residual_cell<SURF, false>(P, i, j, k, c, p, p_old, dt, f, V, q.p, q.kr, sat, so, po, zm, lz,
+                                 us, i > 0 ? wx : 0.0, ux, un, uz);
+    lz = uz;
+    q = n;
+    zm = zu;
   }
 }
 
@@ -397,79 +433,86 @@ __global__ void __launch_bounds__(256) k_residual_zm(DevProblem P, const double 
 // TA is the arithmetic of the face terms: double for the FP64 Jacobian; for
 // a Jacobian stored in FP32 the face terms are formed in FP32 too (their
 // products round no worse than the storage), while the upwind decisions, the
-// pressure differences they come from and the row sums stay FP64.  With TA =
-// double the operations are those of the reference macros, in their order.
+// pressure differences they come from and the row sums stay FP64.
 template <typename TA>
 struct FaceDer {
   TA lo, hi, sym;  // d/dp of the face flux w.r.t. lower cell (negated), upper cell; sym part
 };
 
+__device__ __forceinline__ float quotient(float a, float b) { return a / b; }
+__device__ __forceinline__ double quotient(double a, double b) { return a * fast_rcp(b); }
 template <typename TA>
 __device__ __forceinline__ TA harmonic_t(TA a, TA b) {
-  return (a + b) ? (TA(2) * a * b) / (a + b) : TA(0);
+  return (a + b) ? quotient(TA(2) * a * b, a + b) : TA(0);
 }
 template <typename TA>
 __device__ __forceinline__ TA harmonic_dz_t(TA a, TA b, TA c, TA d) {
-  return ((c * b) + (a * d)) ? (((c + d) * a * b) / ((b * c) + (a * d))) : TA(0);
-}
-// upstream() with the decision taken in FP64 and the values in TA
-template <typename TA>
-__device__ __forceinline__ TA pick(double a, double b, TA c, TA d) {
-  return ((a - b) >= 0) ? c : d;
+  const TA den = (b * c) + (a * d);
+  return den ? quotient((c + d) * a * b, den) : TA(0);
 }
 
+// What a face term needs of a cell: the pressure in FP64 (its differences take
+// the upwind decision), K, kr rho and dkr rho in the face arithmetic,
+// converted once per cell
 template <typename TA>
-__device__ __forceinline__ FaceDer<TA> face_der_xy(const DevProblem &P, double dt, double fb,
-                                                   double h_ff,
-                                                   double dd, double inv_dd, double pa,
-                                                   double pb, double ka, double kb, double prod,
-                                                   double prod_der, double prod_rt,
-                                                   double prod_rt_der, double zm, double dir_g,
-                                                   double dir_g_c) {
-  const double diff64 = pa - pb;
-  const double updir = (diff64 * inv_dd) * dir_g_c - dir_g;
-  const TA diff = (TA)diff64;
-  // x_coeff / y_coeff (richards_jacobian_eval.c:662, 692): FB * dt * ...
-  const TA coeff = (TA)fb * (TA)dt * (TA)h_ff * (TA)inv_dd * (TA)zm *
-                   harmonic_t<TA>((TA)ka, (TA)kb) * (TA)P.inv_visc;
-  const TA dgc = (TA)dir_g_c, dg = (TA)dir_g, tdd = (TA)dd;
+struct JCell {
+  double p;
+  TA k, prod, prod_der;
+};
+template <typename TA>
+__device__ __forceinline__ JCell<TA> jcell(const double *__restrict__ p, const double *kk,
+                                           const double *__restrict__ kr,
+                                           const double *__restrict__ dkr, double rho,
+                                           long long c) {
+  return JCell<TA>{p[c], (TA)__ldg(kk + c), (TA)(kr[c] * rho), (TA)(dkr[c] * rho)};
+}
+// constants of the x / y faces: area dt / (spacing viscosity), and the
+// spacing and its reciprocal
+template <typename TA>
+struct JFace {
+  TA c, d;
+  double inv_d;
+};
+
+// x_coeff / y_coeff (richards_jacobian_eval.c:662, 692): FB * dt * ...; the
+// upwinded terms of the reference's macros with their common factors formed once
+template <typename TA>
+__device__ __forceinline__ FaceDer<TA> face_der_xy(const JFace<TA> &F, double fb,
+                                                   const JCell<TA> &a, const JCell<TA> &b,
+                                                   TA zm, double dir_g, double dir_g_c) {
+  const double diff64 = a.p - b.p;
+  const bool lower = ((diff64 * F.inv_d) * dir_g_c - dir_g) >= 0.0;  // flow from a to b
+  const TA diff = (TA)diff64, dgc = (TA)dir_g_c, dg = (TA)dir_g;
+  const TA coeff = (TA)fb * F.c * zm * harmonic_t<TA>(a.k, b.k);
+  // derivative of the upwind cell's mobility times the driving difference
+  const TA drive = coeff * (diff * dgc - F.d * dg);
+  const TA sym = (-coeff * (lower ? a.prod : b.prod)) * dgc;
   FaceDer<TA> r;
-  TA sym_lo = (-coeff * pick<TA>(updir, 0.0, (TA)prod, (TA)prod_rt)) * dgc;
-  r.lo = (-coeff * diff * pick<TA>(updir, 0.0, (TA)prod_der, TA(0.0))) * dgc + sym_lo;
-  r.lo += (coeff * tdd * pick<TA>(updir, 0.0, (TA)prod_der, TA(0.0))) * dg;
-  r.sym = (-coeff * pick<TA>(updir, 0.0, (TA)prod, (TA)prod_rt)) * dgc;
-  r.hi = (coeff * diff * pick<TA>(updir, 0.0, TA(0.0), (TA)prod_rt_der)) * dgc + r.sym;
-  r.hi += -(coeff * tdd * pick<TA>(updir, 0.0, TA(0.0), (TA)prod_rt_der)) * dg;
+  r.sym = sym;
+  r.lo = lower ? sym - drive * a.prod_der : sym;
+  r.hi = lower ? sym : sym + drive * b.prod_der;
   return r;
 }
 
-// z face between a (lower) and b (upper) (richards_jacobian_eval.c:697-745)
+// z face between a (lower) and b (upper) (richards_jacobian_eval.c:697-745);
+// the terms with the density's derivative are zero (constant density)
 template <typename TA>
-__device__ __forceinline__ FaceDer<TA> face_der_z(const DevProblem &P, double dt, double fb,
-                                                  double pa,
-                                                  double pb, double ka, double kb, double prod,
-                                                  double prod_der, double prod_up,
-                                                  double prod_up_der, double za, double zb,
-                                                  int k) {
-  const double g = P.gravity, rho = P.density, drho = 0.0;
-  const double dz = P.dz;
+__device__ __forceinline__ FaceDer<TA> face_der_z(const DevProblem &P, TA cz, double fb,
+                                                  const JCell<TA> &a, const JCell<TA> &b,
+                                                  double za, double zb, int k) {
+  const double rg = P.density * P.gravity;
   const double inv_sep = __ldg(P.zface + 3 * k);
-  double lower_cond = pa * inv_sep - __ldg(P.zface + 3 * k + 1) * rho * g;
-  double upper_cond = pb * inv_sep + __ldg(P.zface + 3 * k + 2) * rho * g;
-  const TA diff = (TA)(lower_cond - upper_cond);
-  const TA z_coeff = (TA)fb * (TA)dt * ((TA)P.dx * (TA)P.dy) *
-                     harmonic_dz_t<TA>((TA)ka, (TA)kb, (TA)za, (TA)zb) * (TA)P.inv_visc;
-  const TA up = pick<TA>(lower_cond, upper_cond, (TA)prod, (TA)prod_up);
-  const TA grav = (TA)(-g * 0.5 * dz * (amean(za, zb)) * drho);
-  const TA sym_lower = -z_coeff * (TA)inv_sep * up;
+  const double lower_cond = a.p * inv_sep - __ldg(P.zface + 3 * k + 1) * rg;
+  const double upper_cond = b.p * inv_sep + __ldg(P.zface + 3 * k + 2) * rg;
+  const double diff64 = lower_cond - upper_cond;
+  const bool lower = diff64 >= 0.0;
+  const TA coeff = (TA)fb * cz * harmonic_dz_t<TA>(a.k, b.k, (TA)za, (TA)zb);
+  const TA drive = coeff * (TA)diff64;
+  const TA sym = -coeff * (TA)inv_sep * (lower ? a.prod : b.prod);
   FaceDer<TA> r;
-  r.lo = -z_coeff * (diff * pick<TA>(lower_cond, upper_cond, (TA)prod_der, TA(0.0)) +
-                     (grav * up)) +
-         sym_lower;
-  r.sym = z_coeff * (TA)inv_sep * -up;
-  r.hi = z_coeff * (diff * pick<TA>(lower_cond, upper_cond, TA(0.0), (TA)prod_up_der) +
-                    (grav * up)) +
-         r.sym;
+  r.sym = sym;
+  r.lo = lower ? sym - drive * a.prod_der : sym;
+  r.hi = lower ? sym : sym + drive * b.prod_der;
   return r;
 }
 
@@ -493,10 +536,9 @@ template <typename TJ, typename TP, bool SURF>
 __device__ __forceinline__ void jacobian_cell(const DevProblem &P, int i, int j, int k,
                                               long long c, const double *__restrict__ p,
                                               const double *__restrict__ kr,
-                                              const double *__restrict__ dkr,
-                                              const double *__restrict__ satv,
-                                              const double *__restrict__ dsatv, double dt,
+                                              const double *__restrict__ dkr, double dt,
                                               const JacOut<TJ> &J, const PCOut<TP> &M,
+                                              double pc, double sat, double dsat, double zm,
                                               FaceLH<TJ> dl_z, FaceLH<TJ> dl_y, FaceLH<TJ> dl_x,
                                               const FaceDer<TJ> &de, const FaceDer<TJ> &dn,
                                               const FaceDer<TJ> &du) {
@@ -504,13 +546,6 @@ __device__ __forceinline__ void jacobian_cell(const DevProblem &P, int i, int j,
   const double rho = P.density, g = P.gravity, drho = 0.0;
   const double vol = P.dx * P.dy * P.dz;
   const double ffx = P.dy * P.dz, ffy = P.dx * P.dz, ffz = P.dx * P.dy;
-  const double zm = __ldg(P.zmult + k);
-  const double pc = p[c];
-  const double sat = satv[c], dsat = dsatv[c];
-  const double prod = kr[c] * rho, prod_der = dkr[c] * rho + kr[c] * drho;
-  const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
-  (void)g;
-  (void)kzc;
 
   double vol2 = vol * zm;
   double cp = 0.0;
@@ -557,6 +592,8 @@ __device__ __forceinline__ void jacobian_cell(const DevProblem &P, int i, int j,
     if (!onf[face] || P.bc_type[face] != 1) continue;
     const double value = __ldg(P.bc_val[face] + face_slot(P, face, i, j, k));
     const double den_d = rho;
+    const double prod = kr[c] * rho, prod_der = dkr[c] * rho + kr[c] * drho;
+    const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
     const VG v = vg_at(P, c);
     const double prod_val = vg_kr(P, value, v.alpha, v.n) * den_d;
     // above the top layer the z_mult ghost keeps the 1 it was initialised
@@ -755,8 +792,20 @@ __device__ __forceinline__ void jacobian_cell(const DevProblem &P, int i, int j,
   }
 }
 
+template <typename TA>
+struct JConst {
+  JFace<TA> x, y;
+  TA cz;
+  __device__ __forceinline__ JConst(const DevProblem &P, double dt) {
+    const TA q = (TA)dt * (TA)P.inv_visc;
+    x = JFace<TA>{q * (TA)(P.dy * P.dz) * (TA)P.inv_dx, (TA)P.dx, P.inv_dx};
+    y = JFace<TA>{q * (TA)(P.dx * P.dz) * (TA)P.inv_dy, (TA)P.dy, P.inv_dy};
+    cz = q * ((TA)P.dx * (TA)P.dy);
+  }
+};
+
 // Gather form: every cell evaluates the derivative parts of all six of its
-// faces.  The default launch form (see residual_gather).
+// faces.
 template <typename TJ, typename TP, bool SURF>
 __global__ void __launch_bounds__(128, 8) k_jacobian(DevProblem P, const double *__restrict__ p,
                            const double *__restrict__ kr, const double *__restrict__ dkr,
@@ -769,150 +818,117 @@ __global__ void __launch_bounds__(128, 8) k_jacobian(DevProblem P, const double 
   if (!launch_ijk(P.nx, P.ny, P.nz, i, j, k)) return;
   const long long c = i + (long long)P.nx * (j + (long long)P.ny * k);
   const long long sy = P.nx, sz = (long long)P.nx * P.ny;
-  const double rho = P.density, g = P.gravity, drho = 0.0;
-  const double ffx = P.dy * P.dz, ffy = P.dx * P.dz;
+  const double rho = P.density, g = P.gravity;
+  const JConst<TA> A(P, dt);
   const double zm = __ldg(P.zmult + k);
-  const double pc = p[c];
-  const double prod = kr[c] * rho, prod_der = dkr[c] * rho + kr[c] * drho;
-  const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
+  const JCell<TA> q = jcell<TA>(p, P.kx, kr, dkr, rho, c);
+  const TA kyc = P.ky == P.kx ? q.k : (TA)__ldg(P.ky + c);
+  const TA kzc = P.kz == P.kx ? q.k : (TA)__ldg(P.kz + c);
+  const JCell<TA> qy{q.p, kyc, q.prod, q.prod_der}, qz{q.p, kzc, q.prod, q.prod_der};
   FaceLH<TA> dl_z{}, dl_y{}, dl_x{};
   FaceDer<TA> de{}, dn{}, du{};
   if (k > 0) {
-    long long q = c - sz;
-    FaceDer<TA> d = face_der_z<TA>(P, dt, fb_z(P, q), p[q], pc, __ldg(P.kz + q), kzc,
-                                   kr[q] * rho, dkr[q] * rho + kr[q] * drho, prod, prod_der,
-                                   __ldg(P.zmult + k - 1), zm, k - 1);
+    const FaceDer<TA> d = face_der_z<TA>(P, A.cz, fb_z(P, c - sz),
+                                         jcell<TA>(p, P.kz, kr, dkr, rho, c - sz), qz,
+                                         __ldg(P.zmult + k - 1), zm, k - 1);
     dl_z = {d.lo, d.hi};
   }
-  double gs = 0.5 * (g * 0.0 + g * 0.0), gc = 0.5 * (g * 1.0 + g * 1.0);
+  double gs = 0.0, gc = g;
   if (j > 0) {
-    long long q = c - sy;
     if (SURF) tfg_face_y(P, i, j - 1, gs, gc);
-    FaceDer<TA> d = face_der_xy<TA>(P, dt, fb_y(P, q), ffy, P.dy, P.inv_dy, p[q], pc,
-                                    __ldg(P.ky + q), kyc, kr[q] * rho,
-                                    dkr[q] * rho + kr[q] * drho, prod, prod_der, zm, gs, gc);
+    const FaceDer<TA> d = face_der_xy<TA>(A.y, fb_y(P, c - sy),
+                                          jcell<TA>(p, P.ky, kr, dkr, rho, c - sy), qy, (TA)zm, gs,
+                                          gc);
     dl_y = {d.lo, d.hi};
   }
   if (i > 0) {
-    long long q = c - 1;
     if (SURF) tfg_face_x(P, i - 1, j, gs, gc);
-    FaceDer<TA> d = face_der_xy<TA>(P, dt, fb_x(P, q), ffx, P.dx, P.inv_dx, p[q], pc,
-                                    __ldg(P.kx + q), kxc, kr[q] * rho,
-                                    dkr[q] * rho + kr[q] * drho, prod, prod_der, zm, gs, gc);
+    const FaceDer<TA> d = face_der_xy<TA>(A.x, fb_x(P, c - 1),
+                                          jcell<TA>(p, P.kx, kr, dkr, rho, c - 1), q, (TA)zm, gs,
+                                          gc);
     dl_x = {d.lo, d.hi};
   }
   if (i + 1 < P.nx) {
-    long long q = c + 1;
     if (SURF) tfg_face_x(P, i, j, gs, gc);
-    de = face_der_xy<TA>(P, dt, fb_x(P, c), ffx, P.dx, P.inv_dx, pc, p[q], kxc, __ldg(P.kx + q),
-                         prod, prod_der, kr[q] * rho, dkr[q] * rho + kr[q] * drho, zm, gs, gc);
+    de = face_der_xy<TA>(A.x, fb_x(P, c), q, jcell<TA>(p, P.kx, kr, dkr, rho, c + 1), (TA)zm, gs,
+                         gc);
   }
   if (j + 1 < P.ny) {
-    long long q = c + sy;
     if (SURF) tfg_face_y(P, i, j, gs, gc);
-    dn = face_der_xy<TA>(P, dt, fb_y(P, c), ffy, P.dy, P.inv_dy, pc, p[q], kyc, __ldg(P.ky + q),
-                         prod, prod_der, kr[q] * rho, dkr[q] * rho + kr[q] * drho, zm, gs, gc);
+    dn = face_der_xy<TA>(A.y, fb_y(P, c), qy, jcell<TA>(p, P.ky, kr, dkr, rho, c + sy), (TA)zm,
+                         gs, gc);
   }
-  if (k + 1 < P.nz) {
-    long long q = c + sz;
-    du = face_der_z<TA>(P, dt, fb_z(P, c), pc, p[q], kzc, __ldg(P.kz + q), prod, prod_der,
-                        kr[q] * rho, dkr[q] * rho + kr[q] * drho, zm, __ldg(P.zmult + k + 1), k);
-  }
-  jacobian_cell<TJ, TP, SURF>(P, i, j, k, c, p, kr, dkr, satv, dsatv, dt, J, M, dl_z, dl_y,
-                              dl_x, de, dn, du);
+  if (k + 1 < P.nz)
+    du = face_der_z<TA>(P, A.cz, fb_z(P, c), qz, jcell<TA>(p, P.kz, kr, dkr, rho, c + sz), zm,
+                        __ldg(P.zmult + k + 1), k);
+  jacobian_cell<TJ, TP, SURF>(P, i, j, k, c, p, kr, dkr, dt, J, M, q.p, satv[c], dsatv[c], zm,
+                              dl_z, dl_y, dl_x, de, dn, du);
 }
 
-// Face-once form (as k_residual_zm): each cell evaluates the derivative
-// parts of its right, front and upper faces; the (lo, hi) parts the
-// neighbour needs go through shared memory (x, y) or a register (z).
-// Shared memory: blockDim.y x (blockDim.x + 1) and (blockDim.y + 1) x
-// blockDim.x pairs of TJ.
+// March form (as k_residual_march): a face's (lo, hi) parts go to the lane of
+// the next column by shuffles and to the next plane in registers.
+// The gather form converts every operand of every face to the face arithmetic
+// (103 conversions and reciprocals per cell on a pipe of 16 lanes), this one a
+// cell's values once per thread that needs them.  512x512x50, FP32: 347 us
+// against 449; FP64: 503 against 516.
 template <typename TJ, typename TP, bool SURF>
-__global__ void __launch_bounds__(256, 3) k_jacobian_zm(DevProblem P, const double *__restrict__ p,
-                           const double *__restrict__ kr, const double *__restrict__ dkr,
-                           const double *__restrict__ satv, const double *__restrict__ dsatv,
-                           double dt, JacOut<TJ> J, PCOut<TP> M, int kchunk) {
+__global__ void __launch_bounds__(32 * MARCH_WARPS, sizeof(TJ) == 8 ? 2 : SURF ? 3 : 4)
+    k_jacobian_march(
+    DevProblem P, const double *__restrict__ p, const double *__restrict__ kr,
+    const double *__restrict__ dkr, const double *__restrict__ satv,
+    const double *__restrict__ dsatv, double dt, JacOut<TJ> J, PCOut<TP> M, int kchunk) {
   using TA = TJ;
-  extern __shared__ __align__(16) unsigned char jz_smem[];
-  const int bx = blockDim.x, by = blockDim.y, tx = threadIdx.x, ty = threadIdx.y;
-  FaceLH<TA> *sE = reinterpret_cast<FaceLH<TA> *>(jz_smem);  // [by][bx + 1]
-  FaceLH<TA> *sN = sE + by * (bx + 1);                         // [by + 1][bx]
   pdl_enter();
   if (P.dtp) dt = *P.dtp;
-  const int i = blockIdx.x * bx + tx, j = blockIdx.y * by + ty;
-  const int k0 = blockIdx.z * kchunk, k1 = min(P.nz, k0 + kchunk);
-  const bool in = i < P.nx && j < P.ny;
-  const long long sy = P.nx, sz = (long long)P.nx * P.ny;
-  const double rho = P.density, g = P.gravity, drho = 0.0;
-  const double ffx = P.dy * P.dz, ffy = P.dx * P.dz;
-  double gsw = 0.5 * (g * 0.0 + g * 0.0), gcw = 0.5 * (g * 1.0 + g * 1.0);
-  double gss = gsw, gcs = gcw, gse = gsw, gce = gcw, gsn = gsw, gcn = gcw;
-  if (SURF && in) {
-    if (i > 0) tfg_face_x(P, i - 1, j, gsw, gcw);
-    if (j > 0) tfg_face_y(P, i, j - 1, gss, gcs);
-    if (i + 1 < P.nx) tfg_face_x(P, i, j, gse, gce);
-    if (j + 1 < P.ny) tfg_face_y(P, i, j, gsn, gcn);
+  const int lane = threadIdx.x, nx = P.nx, ny = P.ny, nz = P.nz;
+  const int j = blockIdx.y * MARCH_WARPS + threadIdx.y;
+  if (j >= ny) return;
+  const int i = blockIdx.x * MARCH_COLS + lane - 1;
+  const int k0 = blockIdx.z * kchunk, k1 = min(nz, k0 + kchunk);
+  const bool in = i >= 0 && i < nx, out = in && lane > 0, east = in && i + 1 < nx;
+  const bool south = j > 0, north = j + 1 < ny;
+  const int ii = in ? i : (i < 0 ? 0 : nx - 1), sz = nx * ny;
+  const double rho = P.density;
+  const JConst<TA> A(P, dt);
+  double gse = 0.0, gce = P.gravity, gss = 0.0, gcs = P.gravity, gsn = 0.0, gcn = P.gravity;
+  if (SURF) {
+    if (east) tfg_face_x(P, ii, j, gse, gce);
+    if (south) tfg_face_y(P, ii, j - 1, gss, gcs);
+    if (north) tfg_face_y(P, ii, j, gsn, gcn);
   }
-  long long c = i + (long long)P.nx * (j + (long long)P.ny * k0);
-  FaceLH<TA> dl_z{};
-  if (in && k0 > 0 && k0 < k1) {
-    const long long q = c - sz;
-    FaceDer<TA> d = face_der_z<TA>(P, dt, fb_z(P, q), p[q], p[c], __ldg(P.kz + q), __ldg(P.kz + c),
-                                   kr[q] * rho, dkr[q] * rho + kr[q] * drho, kr[c] * rho,
-                                   dkr[c] * rho + kr[c] * drho, __ldg(P.zmult + k0 - 1),
-                                   __ldg(P.zmult + k0), k0 - 1);
-    dl_z = {d.lo, d.hi};
+  int c = ii + nx * (j + ny * k0);
+  auto cell = [&](int q) { return jcell<TA>(p, P.kx, kr, dkr, rho, q); };
+  JCell<TA> q = cell(c);
+  FaceLH<TA> lz = {};
+  double zm = __ldg(P.zmult + k0);
+  if (k0 > 0) {
+    const FaceDer<TA> d = face_der_z<TA>(P, A.cz, fb_z(P, c - sz), cell(c - sz), q,
+                                         __ldg(P.zmult + k0 - 1), zm, k0 - 1);
+    lz = {d.lo, d.hi};
   }
   for (int k = k0; k < k1; k++, c += sz) {
-    FaceDer<TA> de{}, dn{}, du{};
-    if (in) {
-      const double zm = __ldg(P.zmult + k);
-      const double pc = p[c];
-      const double prod = kr[c] * rho, prod_der = dkr[c] * rho + kr[c] * drho;
-      const double kxc = __ldg(P.kx + c), kyc = __ldg(P.ky + c), kzc = __ldg(P.kz + c);
-      if (i + 1 < P.nx) {
-        const long long q = c + 1;
-        de = face_der_xy<TA>(P, dt, fb_x(P, c), ffx, P.dx, P.inv_dx, pc, p[q], kxc,
-                             __ldg(P.kx + q), prod, prod_der, kr[q] * rho,
-                             dkr[q] * rho + kr[q] * drho, zm, gse, gce);
-      }
-      if (j + 1 < P.ny) {
-        const long long q = c + sy;
-        dn = face_der_xy<TA>(P, dt, fb_y(P, c), ffy, P.dy, P.inv_dy, pc, p[q], kyc,
-                             __ldg(P.ky + q), prod, prod_der, kr[q] * rho,
-                             dkr[q] * rho + kr[q] * drho, zm, gsn, gcn);
-      }
-      if (k + 1 < P.nz) {
-        const long long q = c + sz;
-        du = face_der_z<TA>(P, dt, fb_z(P, c), pc, p[q], kzc, __ldg(P.kz + q), prod, prod_der,
-                            kr[q] * rho, dkr[q] * rho + kr[q] * drho, zm,
-                            __ldg(P.zmult + k + 1), k);
-      }
-      if (tx == 0 && i > 0) {
-        const long long q = c - 1;
-        FaceDer<TA> d = face_der_xy<TA>(P, dt, fb_x(P, q), ffx, P.dx, P.inv_dx, p[q], pc,
-                                        __ldg(P.kx + q), kxc, kr[q] * rho,
-                                        dkr[q] * rho + kr[q] * drho, prod,
-                                        prod_der, zm, gsw, gcw);
-        sE[ty * (bx + 1)] = {d.lo, d.hi};
-      }
-      if (ty == 0 && j > 0) {
-        const long long q = c - sy;
-        FaceDer<TA> d = face_der_xy<TA>(P, dt, fb_y(P, q), ffy, P.dy, P.inv_dy, p[q], pc,
-                                        __ldg(P.ky + q), kyc, kr[q] * rho,
-                                        dkr[q] * rho + kr[q] * drho, prod,
-                                        prod_der, zm, gss, gcs);
-        sN[tx] = {d.lo, d.hi};
-      }
+    const bool up = k + 1 < nz;
+    const double zu = up ? __ldg(P.zmult + k + 1) : zm;
+    const JCell<TA> n = cell(up ? c + sz : c), e = cell(east ? c + 1 : c);
+    const JCell<TA> s = cell(south ? c - nx : c), t = cell(north ? c + nx : c);
+    const double sat = satv[c], dsat = dsatv[c];
+    FaceDer<TA> dx = {}, dn = {}, dz = {};
+    FaceLH<TA> wx, dsl = {};
+    if (east) dx = face_der_xy<TA>(A.x, fb_x(P, c), q, e, (TA)zm, gse, gce);
+    wx.lo = __shfl_up_sync(0xffffffffu, dx.lo, 1);
+    wx.hi = __shfl_up_sync(0xffffffffu, dx.hi, 1);
+    if (south) {
+      const FaceDer<TA> d = face_der_xy<TA>(A.y, fb_y(P, c - nx), s, q, (TA)zm, gss, gcs);
+      dsl = {d.lo, d.hi};
     }
-    sE[ty * (bx + 1) + tx + 1] = {de.lo, de.hi};
-    sN[(ty + 1) * bx + tx] = {dn.lo, dn.hi};
-    __syncthreads();
-    if (in)
-      jacobian_cell<TJ, TP, SURF>(P, i, j, k, c, p, kr, dkr, satv, dsatv, dt, J, M, dl_z,
-                                  sN[ty * bx + tx], sE[ty * (bx + 1) + tx], de, dn, du);
-    dl_z = {du.lo, du.hi};
-    __syncthreads();
+    if (north) dn = face_der_xy<TA>(A.y, fb_y(P, c), q, t, (TA)zm, gsn, gcn);
+    if (up) dz = face_der_z<TA>(P, A.cz, fb_z(P, c), q, n, zm, zu, k);
+    if (out)
+      jacobian_cell<TJ, TP, SURF>(P, i, j, k, c, p, kr, dkr, dt, J, M, q.p, sat, dsat, zm, lz, dsl,
+                                  wx, dx, dn, dz);
+    lz = {dz.lo, dz.hi};
+    q = n;
+    zm = zu;
   }
 }
 
@@ -962,68 +978,73 @@ static inline void shape_tuned(int nx, int ny, int nz, int threads, const int ti
   grid = dim3((nx + tile[0] - 1) / tile[0], (ny + tile[1] - 1) / tile[1], nz);
 }
 
+static VGUniform vg_uniform(const DevProblem &P) {
+  return VGUniform{1.0 / (P.density * P.gravity), 1.0 - 1.0 / P.vgn0};
+}
 void launch_vg_all(const DevProblem &P, const double *p, double *kr, double *dkr, double *sat,
                    double *dsat, cudaStream_t st) {
-  launch_pdl(k_vg_all, dim3(blocks_for(P.n, 256)), dim3(256), st, P, p, kr, dkr, sat, dsat);
+  launch_pdl(k_vg_all<false>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), p, kr,
+             dkr, sat, dsat, nullptr, nullptr, 0.0, nullptr);
+}
+void launch_vg_step(const DevProblem &P, const double *u, const double *pp, const double *lam_p,
+                    double lam, double *unew, double *kr, double *dkr, double *sat, double *dsat,
+                    cudaStream_t st) {
+  launch_pdl(k_vg_all<true>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), u, kr,
+             dkr, sat, dsat, pp, lam_p, lam, unew);
 }
 
 void launch_saturation(const DevProblem &P, const double *p, double *s, cudaStream_t st) {
-  launch_pdl(k_saturation, dim3(blocks_for(P.n, 256)), dim3(256), st, P, p, s);
+  launch_pdl(k_saturation, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), p, s);
 }
 
-// The gather form is the default: on B200 the face-once form runs slower at
-// 512x512x50 (0.566 against 0.524 ms for the VG pass plus the residual,
-// 0.730 against 0.649 ms for the Jacobian with its VG pass): the shared
-// fluxes cost registers and a barrier per plane, and the kernels are bound
-// by latency at the occupancy they leave.  PFGPU_RESIDUAL_FACE_ONCE=1 selects
-// the face-once form (bitwise the same results).
-static bool residual_gather() {
-  static const bool on = [] {
-    const char *v = getenv("PFGPU_RESIDUAL_FACE_ONCE");
-    return !(v && *v == '1');
+// March or gather: the march form reads one permeability field and has a
+// warp per 31 columns and chunk of planes, so it needs a grid that fills the
+// GPU several times over.  Residual with its VG pass, march against gather:
+// 350k cells 20 us against 14, 900k 27 against 34, 3.3M 97 against 111, 13.1M
+// 357 against 430.  PFGPU_RESIDUAL_FACE_ONCE=1 / 0 forces march / gather
+// (bitwise the same results).
+static int face_once_env() {
+  static const int v = [] {
+    const char *e = getenv("PFGPU_RESIDUAL_FACE_ONCE");
+    return e && *e ? (*e == '1' ? 1 : 0) : -1;
   }();
-  return on;
+  return v;
 }
-
-// planes per block of the face-once kernels: enough blocks for about eight
-// per SM while each block walks as many planes as that allows
-static inline int zm_chunk(const dim3 &g2, int nz) {
-  const long long tiles = (long long)g2.x * g2.y;
-  long long chunks = (8LL * 148 + tiles - 1) / tiles;
-  if (chunks < 1) chunks = 1;
-  if (chunks > nz) chunks = nz;
-  return (int)((nz + chunks - 1) / chunks);
+// planes per chunk of the march form, 0: gather
+static int march_chunk(const DevProblem &P) {
+  const int env = face_once_env();
+  if (env == 0 || P.ky != P.kx || P.kz != P.kx) return 0;
+  const long long strips = (long long)((P.nx + MARCH_COLS - 1) / MARCH_COLS) *
+                           P.ny;
+  // chunks of at least eight planes (one more z face per chunk), four waves
+  // of 32 warps per SM where the planes allow it
+  const long long want = 4LL * 32 * 148;
+  long long chunks = (want + strips - 1) / strips;
+  const long long most = (P.nz + 7) / 8;
+  if (chunks > most) chunks = most;
+  if (env < 0 && P.n < MARCH_MIN_CELLS) return 0;
+  return (int)((P.nz + chunks - 1) / chunks);
 }
-
-// tile of the face-once kernels: a tuned shape when one is set, else 32 x 8
-// (one extra x face per 32 cells and one extra y face per 8)
-static inline void zm_shape(int nx, int ny, const int tile[2], dim3 &grid, dim3 &block) {
-  int bx = 32, by = 8;
-  if (tile && tile[0] > 0 && tile[1] > 0 && tile[0] * tile[1] <= 256) {
-    bx = tile[0];
-    by = tile[1];
-  }
-  block = dim3(bx, by, 1);
-  grid = dim3((nx + bx - 1) / bx, (ny + by - 1) / by, 1);
+static dim3 march_grid(const DevProblem &P, int kchunk) {
+  return dim3((P.nx + MARCH_COLS - 1) / MARCH_COLS,
+              (P.ny + MARCH_WARPS - 1) / MARCH_WARPS,
+              (P.nz + kchunk - 1) / kchunk);
 }
 
 template <bool SURF, bool VEL>
 static void launch_residual_t(const DevProblem &P, const double *p, const double *p_old,
                               const double *s_old, const double *kr, const double *sat,
                               double dt, double *f, cudaStream_t st, const VelOut &vel) {
-  dim3 g, b;
-  if (residual_gather()) {
-    shape_tuned(P.nx, P.ny, P.nz, 256, P.tile[0], g, b);
-    launch_pdl(k_residual<SURF, VEL>, dim3(g), dim3(b), st, P, p, p_old, s_old, kr, sat, dt, f,
-               vel);
-    return;
+  if constexpr (!VEL) {
+    if (const int kchunk = march_chunk(P)) {
+      launch_pdl(k_residual_march<SURF>, march_grid(P, kchunk), dim3(32, MARCH_WARPS), st, P, p,
+                 p_old, s_old, kr, sat, dt, f, kchunk);
+      return;
+    }
   }
-  zm_shape(P.nx, P.ny, P.tile[0], g, b);
-  const int kchunk = zm_chunk(g, P.nz);
-  const dim3 gz(g.x, g.y, (P.nz + kchunk - 1) / kchunk);
-  const size_t smem = sizeof(double) * ((size_t)b.y * (b.x + 1) + (size_t)(b.y + 1) * b.x);
-  launch_pdl_smem(k_residual_zm<SURF, VEL>, gz, b, smem, st, P, p, p_old, s_old, kr, sat, dt, f,
-                  vel, kchunk);
+  dim3 g, b;
+  shape_tuned(P.nx, P.ny, P.nz, 256, P.tile[0], g, b);
+  launch_pdl(k_residual<SURF, VEL>, dim3(g), dim3(b), st, P, p, p_old, s_old, kr, sat, dt, f, vel);
 }
 
 void launch_residual(const DevProblem &P, const double *p, const double *p_old,
@@ -1047,28 +1068,25 @@ template <typename TJ, typename TP>
 void launch_jacobian(const DevProblem &P, const double *p, const double *kr,
                      const double *dkr, const double *sat, const double *dsat, double dt,
                      JacOut<TJ> J, PCOut<TP> M, cudaStream_t st) {
-  dim3 g, b;
   const bool surf = P.tfg_xs || P.bc_type[5] == 2 || P.bc_type[5] == 3 || P.bc_type[5] == 4;
-  if (residual_gather()) {
-    shape_tuned(P.nx, P.ny, P.nz, 128, P.tile[1], g, b);
+  const int kchunk = march_chunk(P);
+  if (kchunk && !(surf && sizeof(TJ) == 8 && face_once_env() < 0)) {
+    // (FP64 with slopes: gather, 71 us against 75 at 256x256x20)
     if (surf)
-      launch_pdl(k_jacobian<TJ, TP, true>, dim3(g), dim3(b), st, P, p, kr, dkr, sat, dsat, dt, J,
-                 M);
+      launch_pdl(k_jacobian_march<TJ, TP, true>, march_grid(P, kchunk), dim3(32, MARCH_WARPS), st,
+                 P, p, kr, dkr, sat, dsat, dt, J, M, kchunk);
     else
-      launch_pdl(k_jacobian<TJ, TP, false>, dim3(g), dim3(b), st, P, p, kr, dkr, sat, dsat, dt,
-                 J, M);
+      launch_pdl(k_jacobian_march<TJ, TP, false>, march_grid(P, kchunk), dim3(32, MARCH_WARPS), st,
+                 P, p, kr, dkr, sat, dsat, dt, J, M, kchunk);
     return;
   }
-  zm_shape(P.nx, P.ny, P.tile[1], g, b);
-  const int kchunk = zm_chunk(g, P.nz);
-  const dim3 gz(g.x, g.y, (P.nz + kchunk - 1) / kchunk);
-  const size_t smem = sizeof(FaceLH<TJ>) * ((size_t)b.y * (b.x + 1) + (size_t)(b.y + 1) * b.x);
+  dim3 g, b;
+  shape_tuned(P.nx, P.ny, P.nz, 128, P.tile[1], g, b);
   if (surf)
-    launch_pdl_smem(k_jacobian_zm<TJ, TP, true>, gz, b, smem, st, P, p, kr, dkr, sat, dsat, dt,
-                    J, M, kchunk);
+    launch_pdl(k_jacobian<TJ, TP, true>, dim3(g), dim3(b), st, P, p, kr, dkr, sat, dsat, dt, J, M);
   else
-    launch_pdl_smem(k_jacobian_zm<TJ, TP, false>, gz, b, smem, st, P, p, kr, dkr, sat, dsat, dt,
-                    J, M, kchunk);
+    launch_pdl(k_jacobian<TJ, TP, false>, dim3(g), dim3(b), st, P, p, kr, dkr, sat, dsat, dt, J,
+               M);
 }
 
 template <typename TJ>
