@@ -12,8 +12,18 @@
 
 namespace pfgpu {
 
+// Four blocks per SM and four elements in flight per thread keep enough bytes
+// in flight to stream at HBM bandwidth (projection with the next dot product at
+// 512x512x50: 58 us against 76 with one element); short vectors take
+// no more blocks than give each thread its four elements, since every block
+// adds an atomic to the serial end of the reduction.
 static const int RED_THREADS = 256;
 static const int RED_BLOCKS = 592;  // 4 x 148 SMs
+static const int RED_UNROLL = 4;
+static int red_grid(long long n, int most) {
+  const long long per = (long long)RED_THREADS * RED_UNROLL, need = (n + per - 1) / per;
+  return (int)(need < 1 ? 1 : need < most ? need : most);
+}
 
 int reduce_blocks() { return RED_BLOCKS; }
 
@@ -47,16 +57,21 @@ struct OpStepDiff {  // |a - b| / (1 + |a|)  (KINStop, kinsol.c:1541-1544)
 
 template <typename Op>
 __global__ void __launch_bounds__(RED_THREADS) k_reduce(Op op, long long n, double *partial,
-                                                        double *dst, unsigned int *ticket,
-                                                        const double *gate) {
+                                                        double *dst, unsigned int *ticket) {
   pdl_enter();
   __shared__ double sh[RED_THREADS / 32];
   __shared__ bool last;
-  if (gate && *gate == 0.0) return;  // reduction not needed this time
   double acc = Op::init();
-  for (long long i = blockIdx.x * (long long)RED_THREADS + threadIdx.x; i < n;
-       i += (long long)gridDim.x * RED_THREADS)
-    acc = Op::comb(acc, op(i));
+  const long long stride = (long long)gridDim.x * RED_THREADS;
+  long long i = blockIdx.x * (long long)RED_THREADS + threadIdx.x;
+  for (; i + (RED_UNROLL - 1) * stride < n; i += RED_UNROLL * stride) {
+    double v[RED_UNROLL];
+#pragma unroll
+    for (int u = 0; u < RED_UNROLL; u++) v[u] = op(i + u * stride);
+#pragma unroll
+    for (int u = 0; u < RED_UNROLL; u++) acc = Op::comb(acc, v[u]);
+  }
+  for (; i < n; i += stride) acc = Op::comb(acc, op(i));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc = Op::comb(acc, __shfl_down_sync(0xffffffffu, acc, o));
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
@@ -92,23 +107,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce(Op op, long long n, doub
 }
 
 template <typename Op>
-static void reduce(Op op, long long n, double *dst, ReduceBuf rb, cudaStream_t st,
-                   const double *gate = nullptr) {
-  long long need = (n + RED_THREADS - 1) / RED_THREADS;
-  int blocks = (int)(need < rb.blocks ? need : rb.blocks);
-  if (blocks < 1) blocks = 1;
-  launch_pdl(k_reduce<Op>, dim3(blocks), dim3(RED_THREADS), st, op, n, rb.partial, dst, rb.ticket, gate);
+static void reduce(Op op, long long n, double *dst, ReduceBuf rb, cudaStream_t st) {
+  launch_pdl(k_reduce<Op>, dim3(red_grid(n, rb.blocks)), dim3(RED_THREADS), st, op, n, rb.partial, dst, rb.ticket);
 }
 
 void launch_dot(const double *a, const double *b, long long n, double *dst, ReduceBuf rb,
                 cudaStream_t st) {
   OpDot op{a, b};
   reduce(op, n, dst, rb, st);
-}
-void launch_dot_gated(const double *a, const double *b, long long n, double *dst,
-                      const double *gate, ReduceBuf rb, cudaStream_t st) {
-  OpDot op{a, b};
-  reduce(op, n, dst, rb, st, gate);
 }
 void launch_maxabs(const double *a, long long n, double *dst, ReduceBuf rb, cudaStream_t st) {
   OpMaxAbs op{a};
@@ -145,9 +151,16 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_multi(Op op, long long n
   double acc[K];
 #pragma unroll
   for (int q = 0; q < K; q++) acc[q] = 0.0;
-  for (long long i = blockIdx.x * (long long)RED_THREADS + threadIdx.x; i < n;
-       i += (long long)gridDim.x * RED_THREADS)
-    o.acc(i, acc);
+  const long long stride = (long long)gridDim.x * RED_THREADS;
+  long long i = blockIdx.x * (long long)RED_THREADS + threadIdx.x;
+  for (; i + (RED_UNROLL - 1) * stride < n; i += RED_UNROLL * stride) {
+    typename Op::In in[RED_UNROLL];
+#pragma unroll
+    for (int u = 0; u < RED_UNROLL; u++) in[u] = o.load(i + u * stride);
+#pragma unroll
+    for (int u = 0; u < RED_UNROLL; u++) o.acc(i + u * stride, in[u], acc);
+  }
+  for (; i < n; i += stride) o.acc(i, o.load(i), acc);
 #pragma unroll
   for (int q = 0; q < K; q++) {
     double a = acc[q];
@@ -202,11 +215,14 @@ struct OpMgsFirst {
   static constexpr int K = 2;
   const double *vk, *v0;
   double *dst[K];
+  struct In {
+    double a, v;
+  };
   __device__ void setup() {}
-  __device__ void acc(long long i, double *v) const {
-    const double a = vk[i];
-    v[0] = v[0] + a * a;
-    v[1] = v[1] + v0[i] * a;
+  __device__ In load(long long i) const { return In{vk[i], v0[i]}; }
+  __device__ void acc(long long, const In &q, double *v) const {
+    v[0] = v[0] + q.a * q.a;
+    v[1] = v[1] + q.v * q.a;
   }
   __device__ static double comb(int, double x, double y) { return comb_sum(x, y); }
 };
@@ -218,11 +234,15 @@ struct OpAxpyDot {
   const double *x, *s, *z;
   double sign, a;
   double *dst[K];
+  struct In {
+    double y, x, z;
+  };
   __device__ void setup() { a = sign * (*s); }
-  __device__ void acc(long long i, double *v) {
-    const double yn = y[i] + a * x[i];
+  __device__ In load(long long i) const { return In{y[i], x[i], z ? z[i] : 0.0}; }
+  __device__ void acc(long long i, const In &q, double *v) {
+    const double yn = q.y + a * q.x;
     y[i] = yn;
-    const double zi = z ? z[i] : yn;
+    const double zi = z ? q.z : yn;
     v[0] = v[0] + zi * yn;
   }
   __device__ static double comb(int, double x, double y) { return comb_sum(x, y); }
@@ -233,13 +253,16 @@ struct OpLineSearchIn {
   static constexpr int K = 4;
   const double *jp, *f, *p, *u;
   double *dst[K];
+  struct In {
+    double j, p, f, u;
+  };
   __device__ void setup() {}
-  __device__ void acc(long long i, double *v) const {
-    const double j = jp[i], pi = p[i];
-    v[0] = v[0] + j * j;
-    v[1] = v[1] + f[i] * j;
-    v[2] = v[2] + pi * pi;
-    v[3] = comb_max(v[3], fabs(pi / (1.0 / 1.0 + fabs(u[i]))));
+  __device__ In load(long long i) const { return In{jp[i], p[i], f[i], u[i]}; }
+  __device__ void acc(long long, const In &q, double *v) const {
+    v[0] = v[0] + q.j * q.j;
+    v[1] = v[1] + q.f * q.j;
+    v[2] = v[2] + q.p * q.p;
+    v[3] = comb_max(v[3], fabs(q.p / (1.0 / 1.0 + fabs(q.u))));
   }
   __device__ static double comb(int q, double x, double y) {
     return q == 3 ? comb_max(x, y) : comb_sum(x, y);
@@ -250,11 +273,14 @@ struct OpStepNorms {
   static constexpr int K = 2;
   const double *f;
   double *dst[K];
+  struct In {
+    double f;
+  };
   __device__ void setup() {}
-  __device__ void acc(long long i, double *v) const {
-    const double fi = f[i];
-    v[0] = v[0] + fi * fi;
-    v[1] = comb_max(v[1], fabs(fi));
+  __device__ In load(long long i) const { return In{f[i]}; }
+  __device__ void acc(long long, const In &q, double *v) const {
+    v[0] = v[0] + q.f * q.f;
+    v[1] = comb_max(v[1], fabs(q.f));
   }
   __device__ static double comb(int q, double x, double y) {
     return q == 0 ? comb_sum(x, y) : comb_max(x, y);
@@ -265,12 +291,15 @@ struct OpInitNorms {
   static constexpr int K = 3;
   const double *u, *f;
   double *dst[K];
+  struct In {
+    double u, f;
+  };
   __device__ void setup() {}
-  __device__ void acc(long long i, double *v) const {
-    const double ui = u[i], fi = f[i];
-    v[0] = v[0] + ui * ui;
-    v[1] = comb_max(v[1], fabs(fi));
-    v[2] = v[2] + fi * fi;
+  __device__ In load(long long i) const { return In{u[i], f[i]}; }
+  __device__ void acc(long long, const In &q, double *v) const {
+    v[0] = v[0] + q.u * q.u;
+    v[1] = comb_max(v[1], fabs(q.f));
+    v[2] = v[2] + q.f * q.f;
   }
   __device__ static double comb(int q, double x, double y) {
     return q == 1 ? comb_max(x, y) : comb_sum(x, y);
@@ -282,22 +311,22 @@ struct OpDQ {
   static constexpr int K = 3;
   const double *u, *v;
   double *dst[K];
+  struct In {
+    double u, v;
+  };
   __device__ void setup() {}
-  __device__ void acc(long long i, double *s) const {
-    const double ui = u[i], vi = v[i];
-    s[0] = s[0] + ui * vi;
-    s[1] = s[1] + vi * vi;
-    s[2] = s[2] + fabs(vi);
+  __device__ In load(long long i) const { return In{u[i], v[i]}; }
+  __device__ void acc(long long, const In &q, double *s) const {
+    s[0] = s[0] + q.u * q.v;
+    s[1] = s[1] + q.v * q.v;
+    s[2] = s[2] + fabs(q.v);
   }
   __device__ static double comb(int, double x, double y) { return comb_sum(x, y); }
 };
 
 template <typename Op>
 static void reduce_multi(Op op, long long n, ReduceBuf rb, cudaStream_t st) {
-  long long need = (n + RED_THREADS - 1) / RED_THREADS;
-  int blocks = (int)(need < rb.blocks ? need : rb.blocks);
-  if (blocks < 1) blocks = 1;
-  launch_pdl(k_reduce_multi<Op>, dim3(blocks), dim3(RED_THREADS), st, op, n, rb.partial,
+  launch_pdl(k_reduce_multi<Op>, dim3(red_grid(n, rb.blocks)), dim3(RED_THREADS), st, op, n, rb.partial,
              rb.ticket);
 }
 
@@ -546,16 +575,6 @@ __global__ void k_fill_if(double *__restrict__ x, double v, const int *flag, lon
        i += (long long)gridDim.x * blockDim.x)
     x[i] = v;
 }
-// a trial step: z = x + lam y, or z = x when lam == 0 (the copy of KINSOL's
-// N_VScale(ONE, uu, unew))
-__global__ void k_xpay_lam(double *__restrict__ z, const double *__restrict__ x,
-                           const double *lam, const double *__restrict__ y, long long n) {
-  pdl_enter();
-  const double a = *lam;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    z[i] = (a == 0.0) ? x[i] : x[i] + a * y[i];
-}
 __global__ void k_scale_by(double *__restrict__ x, const double *a_p, long long n) {
   pdl_enter();
   const double a = *a_p;
@@ -595,10 +614,6 @@ void launch_scale_inv_dev_unless(double *x, const double *s, const int *skip, lo
 void launch_fill_if(double *x, double v, const int *flag, long long n, cudaStream_t st) {
   launch_pdl(k_fill_if, dim3(grid_for(n)), dim3(256), st, x, v, flag, n);
 }
-void launch_xpay_lam(double *z, const double *x, const double *lam, const double *y, long long n,
-                     cudaStream_t st) {
-  launch_pdl(k_xpay_lam, dim3(grid_for(n)), dim3(256), st, z, x, lam, y, n);
-}
 void launch_scale_by(double *x, const double *a, long long n, cudaStream_t st) {
   launch_pdl(k_scale_by, dim3(grid_for(n)), dim3(256), st, x, a, n);
 }
@@ -615,8 +630,7 @@ struct GS {
   int lmax;
   __device__ double &h(int i, int j) { return H[i * lmax + j]; }
 };
-enum { SC_RNORM = 0, SC_ROT, SC_RHO, SC_VKNORM2, SC_NEWNORM2, SC_FLAG, SC_NN2, SC_NP, SC_GATE,
-       SC_COEF, SC_HLL, SC_BETA, SC_QRFAIL };
+enum { SC_RNORM = 0, SC_ROT, SC_RHO, SC_VKNORM2, SC_NEWNORM2, SC_HLL, SC_BETA, SC_QRFAIL };
 
 __device__ GS gs_view(double *S, int lmax) {
   GS g;
@@ -648,49 +662,13 @@ __device__ __forceinline__ void gmres_scalar_op(int op, double *S, int l, int lm
   double *sc = g.sc;
   switch (op) {
     case 0: {  // start: r_norm = sqrt(<V0,V0>) already in SC_RNORM as squared
+      for (int i = threadIdx.x; i < (lmax + 1) * lmax; i += blockDim.x) g.H[i] = 0.0;
+      if (threadIdx.x != 0) break;
       double r = sqrt(sc[SC_RNORM]);
       sc[SC_RNORM] = r;
       sc[SC_BETA] = r;
       sc[SC_ROT] = 1.0;
       sc[SC_RHO] = r;
-      for (int i = 0; i < (lmax + 1) * lmax; i++) g.H[i] = 0.0;
-      break;
-    }
-    case 1: {  // after GS: H(i, k-1) stored by dots; compute new norm & reorth flag
-      int k = l + 1;
-      double vk_norm = sqrt(sc[SC_VKNORM2]);
-      double new_norm = sqrt(sc[SC_NEWNORM2]);
-      double temp = 1000.0 * vk_norm;
-      sc[SC_FLAG] = ((temp + new_norm) != temp) ? 0.0 : 1.0;
-      sc[SC_NN2] = 0.0;
-      g.h(k, k - 1) = new_norm;
-      break;
-    }
-    case 3: {  // QR update for column l and residual estimate (iterativ.c:205-250)
-      int n = l + 1;
-      if (l == 0) {
-        double t1 = g.h(0, 0), t2 = g.h(1, 0), c, s;
-        givens(t1, t2, c, s);
-        g.giv[0] = c;
-        g.giv[1] = s;
-        g.h(0, 0) = c * t1 - s * t2;
-      } else {
-        int nm1 = n - 1;
-        for (int k = 0; k < nm1; k++) {
-          double t1 = g.h(k, nm1), t2 = g.h(k + 1, nm1);
-          double c = g.giv[2 * k], s = g.giv[2 * k + 1];
-          g.h(k, nm1) = c * t1 - s * t2;
-          g.h(k + 1, nm1) = s * t1 + c * t2;
-        }
-        double t1 = g.h(nm1, nm1), t2 = g.h(n, nm1), c, s;
-        givens(t1, t2, c, s);
-        g.giv[2 * nm1] = c;
-        g.giv[2 * nm1 + 1] = s;
-        g.h(nm1, nm1) = c * t1 - s * t2;
-      }
-      sc[SC_ROT] *= g.giv[2 * l + 1];
-      sc[SC_RHO] = fabs(sc[SC_ROT] * sc[SC_RNORM]);
-      sc[SC_HLL] = g.h(l + 1, l);
       break;
     }
     case 4: {  // QRsol with krydim = l (iterativ.c:253-286)
@@ -729,18 +707,8 @@ __device__ __forceinline__ void gmres_scalar_op(int op, double *S, int l, int lm
       break;
     }
     case 7: {  // next restart cycle: Hessenberg cleared, rotation product 1
-      sc[SC_ROT] = 1.0;
-      for (int i = 0; i < (lmax + 1) * lmax; i++) g.H[i] = 0.0;
-      break;
-    }
-    case 5: {  // finish reorthogonalisation: corrected new norm (iterativ.c:79-84)
-      int k = l + 1;
-      if (sc[SC_FLAG] != 0.0 && sc[SC_NN2] != 0.0) {
-        double nn = g.h(k, k - 1);
-        double np2 = nn * nn - sc[SC_NN2];
-        g.h(k, k - 1) = (np2 > 0.0) ? sqrt(np2) : 0.0;
-      }
-      sc[SC_HLL] = g.h(k, k - 1);
+      for (int i = threadIdx.x; i < (lmax + 1) * lmax; i += blockDim.x) g.H[i] = 0.0;
+      if (threadIdx.x == 0) sc[SC_ROT] = 1.0;
       break;
     }
   }
@@ -755,50 +723,116 @@ __global__ void k_gmres_scalar_dev(int op, double *S, const int *l, int lmax) {
   gmres_scalar_op(op, S, *l, lmax);
 }
 
-// Reorthogonalisation decision for basis vector i against V_k
-// (iterativ.c:68-77): dot result in SC_NP; sets SC_GATE (apply?) and SC_COEF.
-__global__ void k_reorth_decide(double *S, int i, int l, int lmax) {
+// End of GMRES iteration l in one launch (modified Gram-Schmidt's projections
+// and their dot products are done): the new norm and the re-orthogonalisation
+// test (iterativ.c:60-84), the Givens update of column l and the residual
+// estimate (iterativ.c:205-250) and, GRAPH, the control step that arms the next
+// iteration (spgmr.c:340-360).  One block: re-orthogonalisation is for a new
+// vector that lost all but 1e-13 of its norm, which a solve meets at an exact
+// breakdown if at all; everything else is a few scalars, staged in shared
+// memory.  It stands for 3 l + 7 launches of 1.5 to 3 us each, most of them
+// gated off.
+template <bool GRAPH>
+__global__ void __launch_bounds__(1024) k_gmres_finish(VecList V, double *vk, long long n,
+                                                       double *S, int l, int lmax, NkState *St,
+                                                       NkConds C) {
   pdl_enter();
-  GS g = gs_view(S, lmax);
+  const GS g = gs_view(S, lmax);
   double *sc = g.sc;
-  int k = l + 1;
-  sc[SC_GATE] = 0.0;
-  if (sc[SC_FLAG] == 0.0) return;
-  double new_product = sc[SC_NP];
-  double temp = 1000.0 * g.h(i, k - 1);
-  if ((temp + new_product) == temp) return;
-  g.h(i, k - 1) += new_product;
-  sc[SC_COEF] = -new_product;
-  sc[SC_NN2] += new_product * new_product;
-  sc[SC_GATE] = 1.0;
+  const int k = l + 1, t = threadIdx.x;
+  __shared__ double h[NK_MAX_KRYLOV + 1], giv[2 * NK_MAX_KRYLOV], red[32], coef;
+  __shared__ bool reorth, apply;
+  if (t < k) h[t] = g.H[t * lmax + k - 1];
+  if (t < 2 * l) giv[t] = g.giv[t];
+  double nn2 = 0.0;
+  if (t == 0) {
+    const double vk_norm = sqrt(sc[SC_VKNORM2]), new_norm = sqrt(sc[SC_NEWNORM2]);
+    const double temp = 1000.0 * vk_norm;
+    reorth = !((temp + new_norm) != temp);
+    h[k] = new_norm;
+  }
+  __syncthreads();
+  if (reorth) {
+    for (int i = 0; i < k; i++) {
+      const double *vi = V.v[i];
+      double acc = 0.0;
+      for (long long q = t; q < n; q += blockDim.x) acc = acc + vi[q] * vk[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc = acc + __shfl_down_sync(0xffffffffu, acc, o);
+      if ((t & 31) == 0) red[t >> 5] = acc;
+      __syncthreads();
+      if (t == 0) {
+        double np = red[0];
+        for (int w = 1; w < (int)blockDim.x / 32; w++) np = np + red[w];
+        const double temp = 1000.0 * h[i];
+        apply = !((temp + np) == temp);
+        if (apply) {
+          h[i] += np;
+          coef = -np;
+          nn2 += np * np;
+        }
+      }
+      __syncthreads();
+      if (apply)
+        for (long long q = t; q < n; q += blockDim.x) vk[q] = vk[q] + coef * vi[q];
+      __syncthreads();
+    }
+  }
+  if (t != 0) return;
+  if (nn2 != 0.0) {
+    const double np2 = h[k] * h[k] - nn2;
+    h[k] = (np2 > 0.0) ? sqrt(np2) : 0.0;
+  }
+  // Givens rotations of the earlier columns, then the column's own
+  for (int i = 0; i < l; i++) {
+    const double t1 = h[i], t2 = h[i + 1], c = giv[2 * i], s = giv[2 * i + 1];
+    h[i] = c * t1 - s * t2;
+    h[i + 1] = s * t1 + c * t2;
+  }
+  double c, s;
+  const double t1 = h[l], t2 = h[k];
+  givens(t1, t2, c, s);
+  h[l] = c * t1 - s * t2;
+  g.giv[2 * l] = c;
+  g.giv[2 * l + 1] = s;
+  for (int i = 0; i <= k; i++) g.H[i * lmax + k - 1] = h[i];
+  const double rot = sc[SC_ROT] * s, rho = fabs(rot * sc[SC_RNORM]);
+  sc[SC_ROT] = rot;
+  sc[SC_RHO] = rho;
+  sc[SC_HLL] = t2;
+  if (GRAPH) {
+    St->execs[NKB_GM0 + l]++;
+    St->lin_iters++;
+    St->pc_solves++;
+    if (St->k.use_dq) St->fevals++;
+    St->krydim = l + 1;
+    St->rho = rho;
+    if (rho <= St->delta)
+      St->converged = 1;
+    else if (l + 1 < St->k.lmax)
+      cudaGraphSetConditional(C.iter[l + 1], 1u);
+  }
 }
 
-// y = y + (*coef) * x when *gate != 0
-__global__ void k_axpy_gated(double *__restrict__ y, const double *__restrict__ x,
-                             const double *__restrict__ coef, const double *__restrict__ gate,
-                             long long n) {
-  pdl_enter();
-  if (*gate == 0.0) return;
-  double a = *coef;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    y[i] = y[i] + a * x[i];
+void launch_gmres_finish(double *const *V, int l, int lmax, long long n, double *S,
+                         cudaStream_t st, NkState *St, const NkConds *C) {
+  VecList L{};
+  for (int k = 0; k <= l; k++) L.v[k] = V[k];
+  if (St)
+    launch_pdl(k_gmres_finish<true>, dim3(1), dim3(1024), st, L, V[l + 1], n, S, l, lmax, St, *C);
+  else
+    launch_pdl(k_gmres_finish<false>, dim3(1), dim3(1024), st, L, V[l + 1], n, S, l, lmax, St,
+               NkConds{});
 }
 
 void launch_gmres_scalar(int op, double *S, int l, int lmax, cudaStream_t st) {
-  launch_pdl(k_gmres_scalar, dim3(1), dim3(1), st, op, S, l, lmax);
+  // (the two that clear the Hessenberg matrix: a thread per entry)
+  const int threads = op == GM_START || op == GM_RESTART_INIT ? 256 : 1;
+  launch_pdl(k_gmres_scalar, dim3(1), dim3(threads), st, op, S, l, lmax);
 }
 void launch_gmres_scalar_dev(int op, double *S, const int *l, int lmax, cudaStream_t st) {
   launch_pdl(k_gmres_scalar_dev, dim3(1), dim3(1), st, op, S, l, lmax);
 }
-void launch_reorth_decide(double *S, int i, int l, int lmax, cudaStream_t st) {
-  launch_pdl(k_reorth_decide, dim3(1), dim3(1), st, S, i, l, lmax);
-}
-void launch_axpy_gated(double *y, const double *x, const double *coef, const double *gate,
-                       long long n, cudaStream_t st) {
-  launch_pdl(k_axpy_gated, dim3(grid_for(n)), dim3(256), st, y, x, coef, gate, n);
-}
-
 // ---- ParFlow layout <-> dense ------------------------------------------------
 __global__ void k_unpad(const double *__restrict__ pad, double *__restrict__ dense, int nx,
                         int ny, int nz) {

@@ -114,22 +114,6 @@ __global__ void k_nk_cycle_begin(NkState *S, NkConds c) {
   for (int l = 1; l < S->k.lmax; l++) setc(c.iter[l], false);
 }
 
-// end of GMRES iteration l: the residual estimate against delta
-__global__ void k_nk_gm_iter(NkState *S, const double *sc, int l, NkConds c) {
-  pdl_enter();
-  S->execs[NKB_GM0 + l]++;
-  S->lin_iters++;
-  S->pc_solves++;
-  if (S->k.use_dq) S->fevals++;
-  S->krydim = l + 1;
-  const double rho = sc[SCI_RHO];
-  S->rho = rho;
-  if (rho <= S->delta)
-    S->converged = 1;
-  else if (l + 1 < S->k.lmax)
-    setc(c.iter[l + 1], true);
-}
-
 // end of a GMRES cycle: QR failure, convergence, the restart limit, or a restart
 __global__ void k_nk_cycle_end(NkState *S, const double *sc, NkConds c) {
   pdl_enter();
@@ -399,9 +383,6 @@ void launch_nk_iter(NkState *S, NkConds c, cudaStream_t st) {
 }
 void launch_nk_cycle_begin(NkState *S, NkConds c, cudaStream_t st) {
   launch_pdl(k_nk_cycle_begin, dim3(1), dim3(1), st, S, c);
-}
-void launch_nk_gm_iter(NkState *S, const double *sc, int l, NkConds c, cudaStream_t st) {
-  launch_pdl(k_nk_gm_iter, dim3(1), dim3(1), st, S, sc, l, c);
 }
 void launch_nk_cycle_end(NkState *S, const double *sc, NkConds c, cudaStream_t st) {
   launch_pdl(k_nk_cycle_end, dim3(1), dim3(1), st, S, sc, c);

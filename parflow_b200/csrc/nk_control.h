@@ -84,7 +84,6 @@ struct NkConds {
 void launch_nk_init(NkState *S, const double *dsc, NkConds c, cudaStream_t st);
 void launch_nk_iter(NkState *S, NkConds c, cudaStream_t st);
 void launch_nk_cycle_begin(NkState *S, NkConds c, cudaStream_t st);
-void launch_nk_gm_iter(NkState *S, const double *sc, int l, NkConds c, cudaStream_t st);
 void launch_nk_cycle_end(NkState *S, const double *sc, NkConds c, cudaStream_t st);
 void launch_nk_count(NkState *S, int body, int pc_solves, cudaStream_t st);
 void launch_nk_after_gmres(NkState *S, NkConds c, cudaStream_t st);
@@ -101,6 +100,10 @@ void launch_nk_final(NkState *S, cudaStream_t st);
 
 // vector steps of the graph solve whose scalars live on the device
 // (krylov_kernels.cu)
+// the end of GMRES iteration l: norm of V[l + 1] and re-orthogonalisation, QR
+// update, residual estimate; St given: also the graph's control step
+void launch_gmres_finish(double *const *V, int l, int lmax, long long n, double *S,
+                         cudaStream_t st, NkState *St = nullptr, const NkConds *C = nullptr);
 void launch_v0_init(double *v0, const double *src, const NkState *S, const double *sc,
                     long long n, cudaStream_t st);
 void launch_gmres_scalar_dev(int op, double *S, const int *l, int lmax, cudaStream_t st);
@@ -111,8 +114,6 @@ void launch_restart_v0_dev(double *const *V, int nv, const double *yg, const int
 void launch_scale_inv_dev_unless(double *x, const double *s, const int *skip, long long n,
                                  cudaStream_t st);
 void launch_fill_if(double *x, double v, const int *flag, long long n, cudaStream_t st);
-void launch_xpay_lam(double *z, const double *x, const double *lam, const double *y, long long n,
-                     cudaStream_t st);
 void launch_scale_by(double *x, const double *a, long long n, cudaStream_t st);
 void launch_copy_if(double *dst, const double *src, const int *flag, long long n, cudaStream_t st);
 

@@ -384,9 +384,21 @@ static void ph_collect(pfgpu_handle *h) {
   h->pmark.clear();
 }
 
-static void feval(pfgpu_handle *h, const double *u, double dt, double *f) {
+// step: u is formed first, u = u0 + lam pp (lam from lam_p when given)
+struct Step {
+  const double *u0, *pp, *lam_p;
+  double lam;
+};
+static void feval(pfgpu_handle *h, double *u, double dt, double *f, const Step *step = nullptr) {
   const int m = ph_begin(h);
-  vg_state(h, u, false);
+  if (step) {
+    launch_vg_step(h->P, step->u0, step->pp, step->lam_p, step->lam, u, h->kr, h->dkr, h->sat,
+                   h->dsat, h->st);
+    h->launches++;
+    h->vg_for = u;
+  } else {
+    vg_state(h, u, false);
+  }
   launch_residual(h->P, u, h->p_old, h->s_old, h->kr, h->sat, dt, f, h->st);
   h->launches++;
   ph_end(h, m, PH_FEVAL);
@@ -649,7 +661,12 @@ static int build_vgraph(pfgpu_handle *h) {
 }
 
 // z = M^{-1} r (dense FP64 device vectors; r and z may alias)
-static int pc_apply_dense_impl(pfgpu_handle *h, const double *r, double *z) {
+// vs (where pc_scales(h)): r = vs.v, scaled and stored on the way
+static bool pc_scales(const pfgpu_handle *h) {
+  return h->mg_max_iter > 0 && (h->mixed ? h->mgf.L[0].split : h->mgd.L[0].split);
+}
+static int pc_apply_dense_impl(pfgpu_handle *h, const double *r, double *z,
+                               const VScale &vs = VScale{}) {
   int k = 0;
   if (h->mg_max_iter == 0) {
     // MGSemi.MaxIter 0: x = b (mg_semi.c:198-203)
@@ -659,10 +676,10 @@ static int pc_apply_dense_impl(pfgpu_handle *h, const double *r, double *z) {
   }
   if (h->mixed)
     k += launch_level_in<float>(h->mgf.L[0], r, h->h16 ? h->mgf.L[0].sinv : nullptr, h->st,
-                                level0_red_done(h->mgf, h->d.mg_smoother));
+                                level0_red_done(h->mgf, h->d.mg_smoother), vs);
   else
     k += launch_level_in<double>(h->mgd.L[0], r, nullptr, h->st,
-                                 level0_red_done(h->mgd, h->d.mg_smoother));
+                                 level0_red_done(h->mgd, h->d.mg_smoother), vs);
   CK(cudaGetLastError());
   if (h->nk.capturing) {
     k += (int)vcycle_launch(h);  // inline in the solve's graph
@@ -680,9 +697,10 @@ static int pc_apply_dense_impl(pfgpu_handle *h, const double *r, double *z) {
   h->launches += k;
   return 0;
 }
-static int pc_apply_dense(pfgpu_handle *h, const double *r, double *z) {
+static int pc_apply_dense(pfgpu_handle *h, const double *r, double *z,
+                          const VScale &vs = VScale{}) {
   const int m = ph_begin(h);
-  const int rc = pc_apply_dense_impl(h, r, z);
+  const int rc = pc_apply_dense_impl(h, r, z, vs);
   ph_end(h, m, PH_PCAPPLY);
   return rc;
 }
@@ -770,15 +788,22 @@ static int spgmr(pfgpu_handle *h, double *x, const double *src, double bsign,
     return 0;
   }
 
+  // each basis vector is scaled as it enters the preconditioner
+  const bool scales = pc_scales(h);
   for (int ntries = 0; ntries <= h->d.max_restarts; ntries++) {
-    if (ntries == 0) {
-      // V0 = b / r_norm = src * (bsign / r_norm)
-      launch_axpby(h->V[0], src, bsign * (1.0 / r_norm), 0.0, N, h->st);
-    } else {
-      // the restart direction (built below) scaled by 1 / r_norm
-      launch_scale_inv_dev(h->V[0], sc + SCI_RNORM, N, h->st);
+    // V0 = b / r_norm = src * (bsign / r_norm), or the restart direction
+    // (built below) scaled by 1 / r_norm
+    const VScale v0 = ntries == 0 ? VScale{VScale::SRC, h->V[0], src, nullptr,
+                                           bsign * (1.0 / r_norm), nullptr}
+                                  : VScale{VScale::INV, h->V[0], nullptr, sc + SCI_RNORM, 0.0,
+                                           nullptr};
+    if (!scales) {
+      if (ntries == 0)
+        launch_axpby(h->V[0], src, v0.a, 0.0, N, h->st);
+      else
+        launch_scale_inv_dev(h->V[0], sc + SCI_RNORM, N, h->st);
+      h->launches++;
     }
-    h->launches++;
     int l;
     for (l = 0; l < lmax; l++) {
       stats->lin_iters++;
@@ -786,7 +811,9 @@ static int spgmr(pfgpu_handle *h, double *x, const double *src, double bsign,
       // z = M^{-1} V[l] (the preconditioner reads V[l], writes z: vtemp, or
       // the kept preconditioned basis vector Z[l])
       double *z = h->zbasis ? h->Z[l] : h->vtemp;
-      if (pc_apply_dense(h, h->V[l], z)) return PFGPU_ERR_CUDA;
+      const VScale vl = l == 0 ? v0 : VScale{VScale::INV, h->V[l], nullptr, Hp(l, l - 1), 0.0,
+                                             nullptr};
+      if (pc_apply_dense(h, h->V[l], z, scales ? vl : VScale{})) return PFGPU_ERR_CUDA;
       stats->pc_solves++;
       atimes(h, u, dt, z, h->V[l + 1], stats);
       // ModifiedGS (iterativ.c:30-86): <vk,vk> and h(0) in one pass, then each
@@ -801,17 +828,8 @@ static int spgmr(pfgpu_handle *h, double *x, const double *src, double bsign,
                         more ? Hp(i + 1, k - 1) : sc + SCI_NEWNORM2, h->rb, h->st);
         h->launches++;
       }
-      launch_gmres_scalar(GM_AFTER_GS, S, l, lmax, h->st);
+      launch_gmres_finish(h->V.data(), l, lmax, N, S, h->st);
       h->launches++;
-      for (int i = 0; i < k; i++) {
-        launch_dot_gated(h->V[i], h->V[k], N, sc + SCI_NP, sc + SCI_FLAG, h->rb, h->st);
-        launch_reorth_decide(S, i, l, lmax, h->st);
-        launch_axpy_gated(h->V[k], h->V[i], sc + SCI_COEF, sc + SCI_GATE, N, h->st);
-        h->launches += 3;
-      }
-      launch_gmres_scalar(GM_REORTH_DONE, S, l, lmax, h->st);
-      launch_gmres_scalar(GM_QR, S, l, lmax, h->st);
-      h->launches += 2;
       CK(cudaMemcpyAsync(h->hsc + D_COUNT, sc + SCI_RHO, sizeof(double), cudaMemcpyDeviceToHost,
                          h->st));
       CK(cudaStreamSynchronize(h->st));
@@ -820,8 +838,11 @@ static int spgmr(pfgpu_handle *h, double *x, const double *src, double bsign,
         converged = 1;
         break;
       }
-      launch_scale_inv_dev(h->V[l + 1], Hp(l + 1, l), N, h->st);
-      h->launches++;
+      // (the last one meets no preconditioner, but a restart uses it)
+      if (!scales || l + 1 == lmax) {
+        launch_scale_inv_dev(h->V[l + 1], Hp(l + 1, l), N, h->st);
+        h->launches++;
+      }
     }
     // QRsol and xcor (+)= V y; with the kept basis x (+)= Z y directly
     launch_gmres_scalar(GM_QRSOL, S, krydim, lmax, h->st);
@@ -975,17 +996,12 @@ static int newton_impl(pfgpu_handle *h, double dt, pfgpu_stats *stats) {
     double rl = 1.0, rlprev = 0.0, alpha_cond, beta_cond;
     const int nfesav = stats->fevals;
     auto try_step = [&](double lam) -> int {
-      if (lam == 0.0) {  // N_VScale(ONE, uu, unew)
-        if (cudaMemcpyAsync(unew, u, N * sizeof(double), cudaMemcpyDeviceToDevice, h->st) !=
-            cudaSuccess)
-          return PFGPU_ERR_CUDA;
-      } else {
-        launch_xpay(unew, u, lam, h->pp, N, h->st);
-      }
-      feval(h, unew, dt, h->fval);
+      // (lam 0: N_VScale(ONE, uu, unew))
+      const Step step{u, h->pp, nullptr, lam};
+      feval(h, unew, dt, h->fval, &step);
       stats->fevals++;
       launch_step_norms(h->fval, N, dsc + D_F2, dsc + D_FMAX, h->rb, h->st);
-      h->launches += 2;
+      h->launches++;
       if (read_scalars(h, 0, 2)) return PFGPU_ERR_CUDA;
       fnormp = sqrt(hsc[D_F2]);
       f1normp = 0.5 * fnormp * fnormp;
@@ -1210,10 +1226,10 @@ static int nk_body(pfgpu_handle *h, cudaGraphConditionalHandle hd,
 static void nk_try_step(pfgpu_handle *h, double dt) {
   const long long N = h->N;
   double *dsc = h->dsc;
-  launch_xpay_lam(h->unew, h->u, &h->nk.S->lam, h->pp, N, h->st);
-  feval(h, h->unew, dt, h->fval);
+  const Step step{h->u, h->pp, &h->nk.S->lam, 0.0};
+  feval(h, h->unew, dt, h->fval, &step);
   launch_step_norms(h->fval, N, dsc + D_F2, dsc + D_FMAX, h->rb, h->st);
-  h->launches += 2;
+  h->launches++;
 }
 
 // one GMRES iteration l of a cycle (as the body of spgmr's inner loop)
@@ -1225,7 +1241,10 @@ static int nk_gmres_iter(pfgpu_handle *h, int l, double dt, NkConds &C) {
   auto Hp = [&](int i, int j) { return S + (long long)i * lmax + j; };
   pfgpu_stats dummy{};
   double *z = h->zbasis ? h->Z[l] : h->vtemp;
-  if (pc_apply_dense_impl(h, h->V[l], z)) return PFGPU_ERR_CUDA;
+  const bool scales = pc_scales(h);
+  const VScale vl = l == 0 ? VScale{VScale::V0, h->V[0], h->fval, sc + SCI_RNORM, 0.0, h->nk.S}
+                           : VScale{VScale::INV, h->V[l], nullptr, Hp(l, l - 1), 0.0, nullptr};
+  if (pc_apply_dense_impl(h, h->V[l], z, scales ? vl : VScale{})) return PFGPU_ERR_CUDA;
   atimes(h, h->u, dt, z, h->V[l + 1], &dummy);
   const int k = l + 1;
   launch_mgs_first(h->V[k], h->V[0], N, sc + SCI_VKNORM2, Hp(0, k - 1), h->rb, h->st);
@@ -1236,19 +1255,14 @@ static int nk_gmres_iter(pfgpu_handle *h, int l, double dt, NkConds &C) {
                     more ? Hp(i + 1, k - 1) : sc + SCI_NEWNORM2, h->rb, h->st);
     h->launches++;
   }
-  launch_gmres_scalar(GM_AFTER_GS, S, l, lmax, h->st);
+  launch_gmres_finish(h->V.data(), l, lmax, N, S, h->st, h->nk.S, &C);
   h->launches++;
-  for (int i = 0; i < k; i++) {
-    launch_dot_gated(h->V[i], h->V[k], N, sc + SCI_NP, sc + SCI_FLAG, h->rb, h->st);
-    launch_reorth_decide(S, i, l, lmax, h->st);
-    launch_axpy_gated(h->V[k], h->V[i], sc + SCI_COEF, sc + SCI_GATE, N, h->st);
-    h->launches += 3;
+  // the next iteration scales V[l + 1] as it enters the preconditioner; the
+  // last one meets none, but a restart uses it
+  if (!scales || l + 1 == lmax) {
+    launch_scale_inv_dev_unless(h->V[l + 1], Hp(l + 1, l), &h->nk.S->converged, N, h->st);
+    h->launches++;
   }
-  launch_gmres_scalar(GM_REORTH_DONE, S, l, lmax, h->st);
-  launch_gmres_scalar(GM_QR, S, l, lmax, h->st);
-  launch_nk_gm_iter(h->nk.S, sc, l, C, h->st);
-  launch_scale_inv_dev_unless(h->V[l + 1], Hp(l + 1, l), &h->nk.S->converged, N, h->st);
-  h->launches += 4;
   return 0;
 }
 
@@ -1263,8 +1277,11 @@ static int nk_gmres_cycle(pfgpu_handle *h, double dt, NkConds &C) {
     if (nk_handle(h->st, &C.iter[l])) return PFGPU_ERR_CUDA;
   if (nk_handle(h->st, &C.do_restart)) return PFGPU_ERR_CUDA;
   launch_nk_cycle_begin(St, C, h->st);
-  launch_v0_init(h->V[0], h->fval, St, sc, N, h->st);
-  h->launches += 2;
+  h->launches++;
+  if (!pc_scales(h)) {
+    launch_v0_init(h->V[0], h->fval, St, sc, N, h->st);
+    h->launches++;
+  }
   // iteration l + 1 nests inside iteration l's body: once GMRES stops, no
   // further conditional node is evaluated
   std::function<int(int)> iteration = [&](int l) -> int {

@@ -307,12 +307,23 @@ int launch_setup_tail(const MGLevel<T> *levels_host, const MGLevel<T> *levels_de
 // natural FP64 vector z, in the level's type and layout (times the FP16
 // scaling when scale is given); return the number of kernels launched
 // (init: with the zero-guess red sweep of the plain operator, where
-// level_in_inits says so)
+// level_in_inits says so; vs, split levels only: r is scaled on the way)
+// The Krylov vector v is formed (and stored) while it goes into the V-cycle:
+// INV v *= 1 / *s; SRC v = a src; V0 the first vector of a GMRES cycle of the
+// graph solve, src * (bsign / r_norm) or, after a restart, v / *s
+struct NkState;
+struct VScale {
+  enum { NONE = 0, INV, SRC, V0 } mode;
+  double *v;
+  const double *src, *s;
+  double a;
+  const NkState *S;
+};
 template <typename T>
 bool level_in_inits(const MGLevel<T> &L, int smoother, bool h16);
 template <typename T>
 int launch_level_in(const MGLevel<T> &L, const double *r, const float *scale, cudaStream_t st,
-                    int init);
+                    int init, const VScale &vs = VScale{});
 template <typename T>
 int launch_level_out(const MGLevel<T> &L, const T *x, double *z, const float *scale, int flip,
                      cudaStream_t st);
@@ -340,9 +351,6 @@ int reduce_partials();  // doubles the partial buffer must hold (multi-value red
 // dst = sum(a .* b); deterministic (fixed grid, fixed order)
 void launch_dot(const double *a, const double *b, long long n, double *dst, ReduceBuf rb,
                 cudaStream_t st);
-// as launch_dot, skipped entirely when *gate == 0
-void launch_dot_gated(const double *a, const double *b, long long n, double *dst,
-                      const double *gate, ReduceBuf rb, cudaStream_t st);
 // dst = max |a|
 void launch_maxabs(const double *a, long long n, double *dst, ReduceBuf rb, cudaStream_t st);
 // dst = max |s| / (1 + |u|)
@@ -394,18 +402,13 @@ void launch_restart_v0(double *const *V, const double *yg, int kdim, long long n
 void launch_fill(double *x, double v, long long n, cudaStream_t st);
 
 // GMRES scalar kernels (single thread); S layout and ops in krylov_kernels.cu
-enum { GM_START = 0, GM_AFTER_GS = 1, GM_QR = 3, GM_QRSOL = 4, GM_REORTH_DONE = 5,
-       GM_RESTART = 6, GM_RESTART_INIT = 7 };
-enum { SCI_RNORM = 0, SCI_ROT, SCI_RHO, SCI_VKNORM2, SCI_NEWNORM2, SCI_FLAG, SCI_NN2, SCI_NP,
-       SCI_GATE, SCI_COEF, SCI_HLL, SCI_BETA, SCI_QRFAIL, SCI_COUNT };
+enum { GM_START = 0, GM_QRSOL = 4, GM_RESTART = 6, GM_RESTART_INIT = 7 };
+enum { SCI_RNORM = 0, SCI_ROT, SCI_RHO, SCI_VKNORM2, SCI_NEWNORM2, SCI_HLL, SCI_BETA, SCI_QRFAIL,
+       SCI_COUNT };
 inline long long gs_size(int lmax) { return (long long)(lmax + 1) * lmax + 2 * lmax + lmax + 1 + SCI_COUNT; }
 inline long long gs_sc_offset(int lmax) { return (long long)(lmax + 1) * lmax + 2 * lmax + lmax + 1; }
 inline long long gs_yg_offset(int lmax) { return (long long)(lmax + 1) * lmax + 2 * lmax; }
 void launch_gmres_scalar(int op, double *S, int l, int lmax, cudaStream_t st);
-void launch_reorth_decide(double *S, int i, int l, int lmax, cudaStream_t st);
-void launch_axpy_gated(double *y, const double *x, const double *coef, const double *gate,
-                       long long n, cudaStream_t st);
-
 // ParFlow layout (ghost frame 1) <-> dense interior
 void launch_unpad(const double *pad, double *dense, int nx, int ny, int nz, cudaStream_t st);
 void launch_pad(const double *dense, double *pad, int nx, int ny, int nz, cudaStream_t st);
