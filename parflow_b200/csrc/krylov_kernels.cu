@@ -723,16 +723,67 @@ __global__ void k_gmres_scalar_dev(int op, double *S, const int *l, int lmax) {
   gmres_scalar_op(op, S, *l, lmax);
 }
 
-// End of GMRES iteration l in one launch (modified Gram-Schmidt's projections
-// and their dot products are done): the new norm and the re-orthogonalisation
-// test (iterativ.c:60-84), the Givens update of column l and the residual
-// estimate (iterativ.c:205-250) and, GRAPH, the control step that arms the next
-// iteration (spgmr.c:340-360).  One block: re-orthogonalisation is for a new
-// vector that lost all but 1e-13 of its norm, which a solve meets at an exact
-// breakdown if at all; everything else is a few scalars, staged in shared
-// memory.  It stands for 3 l + 7 launches of 1.5 to 3 us each, most of them
-// gated off.
-template <bool GRAPH>
+// Scalar end of GMRES iteration l (one thread): column l of the Hessenberg
+// matrix in h[0 .. l + 1], h[l + 1] the norm of the new vector; the rotations
+// of the earlier columns in giv.  The Givens update and the residual estimate
+// (iterativ.c:205-250) and, St given, the control step that arms the next
+// iteration (spgmr.c:340-360).
+__device__ __forceinline__ void gmres_column(const GS &g, double *h, const double *giv, int l,
+                                             NkState *St, const NkConds &C) {
+  double *sc = g.sc;
+  const int k = l + 1;
+  for (int i = 0; i < l; i++) {
+    const double t1 = h[i], t2 = h[i + 1], c = giv[2 * i], s = giv[2 * i + 1];
+    h[i] = c * t1 - s * t2;
+    h[i + 1] = s * t1 + c * t2;
+  }
+  double c, s;
+  const double t1 = h[l], t2 = h[k];
+  givens(t1, t2, c, s);
+  h[l] = c * t1 - s * t2;
+  g.giv[2 * l] = c;
+  g.giv[2 * l + 1] = s;
+  for (int i = 0; i <= k; i++) g.H[i * g.lmax + k - 1] = h[i];
+  const double rot = sc[SC_ROT] * s, rho = fabs(rot * sc[SC_RNORM]);
+  sc[SC_ROT] = rot;
+  sc[SC_RHO] = rho;
+  sc[SC_HLL] = t2;
+  if (St) {
+    St->execs[NKB_GM0 + l]++;
+    St->lin_iters++;
+    St->pc_solves++;
+    if (St->k.use_dq) St->fevals++;
+    St->krydim = l + 1;
+    St->rho = rho;
+    if (rho <= St->delta)
+      St->converged = 1;
+    else if (l + 1 < St->k.lmax)
+      cudaGraphSetConditional(C.iter[l + 1], 1u);
+  }
+}
+// ModifiedGS's test whether the projections cancelled the vector (iterativ.c:60-66)
+__device__ __forceinline__ bool cancelled(double vk_norm, double new_norm) {
+  const double temp = 1000.0 * vk_norm;
+  return !((temp + new_norm) != temp);
+}
+// its second pass (iterativ.c:68-84): one product against basis vector i
+__device__ __forceinline__ bool reorth_step(double np, double &hi, double &nn2) {
+  const double temp = 1000.0 * hi;
+  if ((temp + np) == temp) return false;
+  hi += np;
+  nn2 += np * np;
+  return true;
+}
+__device__ __forceinline__ double reorth_norm(double hk, double nn2) {
+  const double np2 = hk * hk - nn2;
+  return (np2 > 0.0) ? sqrt(np2) : 0.0;
+}
+
+// End of GMRES iteration l in one launch, the projections and their dot
+// products done.  One block: re-orthogonalisation is for a new vector that lost
+// all but 1e-13 of its norm, which a solve meets at an exact breakdown if at
+// all; everything else is a few scalars, staged in shared memory.  It stands
+// for 3 l + 7 launches of 1.5 to 3 us each, most of them gated off.
 __global__ void __launch_bounds__(1024) k_gmres_finish(VecList V, double *vk, long long n,
                                                        double *S, int l, int lmax, NkState *St,
                                                        NkConds C) {
@@ -746,10 +797,8 @@ __global__ void __launch_bounds__(1024) k_gmres_finish(VecList V, double *vk, lo
   if (t < 2 * l) giv[t] = g.giv[t];
   double nn2 = 0.0;
   if (t == 0) {
-    const double vk_norm = sqrt(sc[SC_VKNORM2]), new_norm = sqrt(sc[SC_NEWNORM2]);
-    const double temp = 1000.0 * vk_norm;
-    reorth = !((temp + new_norm) != temp);
-    h[k] = new_norm;
+    h[k] = sqrt(sc[SC_NEWNORM2]);
+    reorth = cancelled(sqrt(sc[SC_VKNORM2]), h[k]);
   }
   __syncthreads();
   if (reorth) {
@@ -764,13 +813,8 @@ __global__ void __launch_bounds__(1024) k_gmres_finish(VecList V, double *vk, lo
       if (t == 0) {
         double np = red[0];
         for (int w = 1; w < (int)blockDim.x / 32; w++) np = np + red[w];
-        const double temp = 1000.0 * h[i];
-        apply = !((temp + np) == temp);
-        if (apply) {
-          h[i] += np;
-          coef = -np;
-          nn2 += np * np;
-        }
+        apply = reorth_step(np, h[i], nn2);
+        coef = -np;
       }
       __syncthreads();
       if (apply)
@@ -779,50 +823,174 @@ __global__ void __launch_bounds__(1024) k_gmres_finish(VecList V, double *vk, lo
     }
   }
   if (t != 0) return;
-  if (nn2 != 0.0) {
-    const double np2 = h[k] * h[k] - nn2;
-    h[k] = (np2 > 0.0) ? sqrt(np2) : 0.0;
+  if (nn2 != 0.0) h[k] = reorth_norm(h[k], nn2);
+  gmres_column(g, h, giv, l, St, C);
+}
+
+// The whole end of GMRES iteration l on one thread-block cluster, for vectors
+// that fit its registers' reach: modified Gram-Schmidt (iterativ.c:30-86) of
+// V[l + 1] against V[0 .. l], re-orthogonalisation, and the column's scalars.
+// The new vector stays in shared memory; a dot product is a block reduction and
+// one exchange of the blocks' partial sums through distributed shared memory
+// (added in block order, so every block holds the same bits).  It stands for
+// l + 3 launches with a grid-wide reduction each.
+// A timestep of 12x10x8 in FP64: 1.25 ms against 1.36.  Up to 65536 cells: at
+// 131072 (16384 per block) it is no faster than the launches, whose passes the
+// whole GPU streams.
+constexpr int MGS_THREADS = 1024, MGS_CLUSTER = 8, MGS_CELLS = 8 * 1024;  // cells per block
+struct MgsCluster {
+  double *sh;               // block reduction
+  double (*part)[2][MGS_CLUSTER];  // [step parity][value][block]
+  int step, rank, blocks;
+  // sums over the cluster of a (and b)
+  __device__ __forceinline__ void sum(double &a, double &b, bool both) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a = a + __shfl_down_sync(0xffffffffu, a, o);
+      if (both) b = b + __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+      sh[w] = a;
+      if (both) sh[32 + w] = b;
+    }
+    __syncthreads();
+    double (*dst)[MGS_CLUSTER] = part[step & 1];
+    if (w < (both ? 2 : 1)) {
+      double v = sh[32 * w + lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, o);
+      v = __shfl_sync(0xffffffffu, v, 0);
+      if (lane < blocks) {  // to every block
+        const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&dst[w][rank]);
+        uint32_t at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(lane));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+      }
+    }
+    if (blocks > 1) {
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else {
+      __syncthreads();
+    }
+    a = dst[0][0];
+    for (int q = 1; q < blocks; q++) a = a + dst[0][q];
+    if (both) {
+      b = dst[1][0];
+      for (int q = 1; q < blocks; q++) b = b + dst[1][q];
+    }
+    step++;
   }
-  // Givens rotations of the earlier columns, then the column's own
-  for (int i = 0; i < l; i++) {
-    const double t1 = h[i], t2 = h[i + 1], c = giv[2 * i], s = giv[2 * i + 1];
-    h[i] = c * t1 - s * t2;
-    h[i + 1] = s * t1 + c * t2;
+};
+__global__ void __launch_bounds__(MGS_THREADS, 1) k_gmres_mgs(VecList V, double *vk, int n,
+                                                              double *S, int l, int lmax,
+                                                              NkState *St, NkConds C) {
+  extern __shared__ double own[];  // this block's cells of vk
+  __shared__ double sh[64], h[NK_MAX_KRYLOV + 1], giv[2 * NK_MAX_KRYLOV], part[2][2][MGS_CLUSTER];
+  const int t = threadIdx.x, k = l + 1;
+  unsigned rank, blocks;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(blocks));
+  MgsCluster R{sh, part, 0, (int)rank, (int)blocks};
+  const GS g = gs_view(S, lmax);
+  if (t < 2 * l) giv[t] = g.giv[t];  // (older than the kernel before this one)
+  const int per = (n + (int)blocks - 1) / (int)blocks, c0 = (int)rank * per;
+  const int m = min(per, n - c0);  // cells of this block (none: n < c0)
+  // a block's shared memory is written by the others from their first sum on
+  if (blocks > 1) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   }
-  double c, s;
-  const double t1 = h[l], t2 = h[k];
-  givens(t1, t2, c, s);
-  h[l] = c * t1 - s * t2;
-  g.giv[2 * l] = c;
-  g.giv[2 * l + 1] = s;
-  for (int i = 0; i <= k; i++) g.H[i * lmax + k - 1] = h[i];
-  const double rot = sc[SC_ROT] * s, rho = fabs(rot * sc[SC_RNORM]);
-  sc[SC_ROT] = rot;
-  sc[SC_RHO] = rho;
-  sc[SC_HLL] = t2;
-  if (GRAPH) {
-    St->execs[NKB_GM0 + l]++;
-    St->lin_iters++;
-    St->pc_solves++;
-    if (St->k.use_dq) St->fevals++;
-    St->krydim = l + 1;
-    St->rho = rho;
-    if (rho <= St->delta)
-      St->converged = 1;
-    else if (l + 1 < St->k.lmax)
-      cudaGraphSetConditional(C.iter[l + 1], 1u);
+  pdl_enter();
+  const double *src = vk + c0, *v0 = V.v[0] + c0;
+  double a = 0.0, b = 0.0;
+#pragma unroll 4
+  for (int q = t; q < m; q += MGS_THREADS) {
+    const double y = src[q];
+    own[q] = y;
+    a = a + y * y;
+    b = b + v0[q] * y;
   }
+  R.sum(a, b, true);
+  const double vk_norm = sqrt(a);
+  double hi = b;
+  for (int i = 0; i < k; i++) {
+    if (t == 0) h[i] = hi;
+    const double *x = V.v[i] + c0, *z = i + 1 < k ? V.v[i + 1] + c0 : nullptr;
+    const double w = -1.0 * hi;
+    a = 0.0;
+#pragma unroll 4
+    for (int q = t; q < m; q += MGS_THREADS) {
+      const double y = own[q] + w * x[q];
+      own[q] = y;
+      a = a + (z ? z[q] : y) * y;
+    }
+    R.sum(a, b, false);
+    hi = a;
+  }
+  double hk = sqrt(hi), nn2 = 0.0;
+  if (cancelled(vk_norm, hk)) {
+    for (int i = 0; i < k; i++) {
+      const double *x = V.v[i] + c0;
+      a = 0.0;
+      for (int q = t; q < m; q += MGS_THREADS) a = a + x[q] * own[q];
+      R.sum(a, b, false);
+      // (every thread of the cluster decides alike, on the same h)
+      double hq = h[i];
+      const bool apply = reorth_step(a, hq, nn2);
+      __syncthreads();
+      if (t == 0) h[i] = hq;
+      if (apply)
+        for (int q = t; q < m; q += MGS_THREADS) own[q] = own[q] - a * x[q];
+      __syncthreads();
+    }
+    if (nn2 != 0.0) hk = reorth_norm(hk, nn2);
+  }
+  double *dst = vk + c0;
+  for (int q = t; q < m; q += MGS_THREADS) dst[q] = own[q];
+  if (t == 0 && rank == 0) {
+    h[k] = hk;
+    gmres_column(g, h, giv, l, St, C);
+  }
+  // no block leaves while another may still write its partial sums
+  if (blocks > 1) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+cudaError_t krylov_prepare_kernels() {
+  return cudaFuncSetAttribute(k_gmres_mgs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              MGS_CELLS * (int)sizeof(double));
+}
+
+// Whether launch_gmres_mgs takes vectors of n elements
+bool gmres_mgs_fits(long long n) {
+  static const long long most = [] {
+    const char *v = getenv("PFGPU_MGS_CELLS");
+    const long long all = (long long)MGS_CLUSTER * MGS_CELLS;
+    const long long m = v && *v ? atoll(v) : all;
+    return m < all ? m : all;
+  }();
+  return n <= most;
+}
+void launch_gmres_mgs(double *const *V, int l, int lmax, long long n, double *S, cudaStream_t st,
+                      NkState *St, const NkConds *C) {
+  VecList L{};
+  for (int k = 0; k <= l; k++) L.v[k] = V[k];
+  int blocks = 1;
+  while (blocks < MGS_CLUSTER && (long long)blocks * 2 * MGS_THREADS < n) blocks *= 2;
+  const size_t smem = (size_t)((n + blocks - 1) / blocks) * sizeof(double);
+  launch_pdl_cluster(k_gmres_mgs, blocks, dim3(MGS_THREADS), smem, st, L, V[l + 1], (int)n, S, l,
+                     lmax, St, C ? *C : NkConds{});
 }
 
 void launch_gmres_finish(double *const *V, int l, int lmax, long long n, double *S,
                          cudaStream_t st, NkState *St, const NkConds *C) {
   VecList L{};
   for (int k = 0; k <= l; k++) L.v[k] = V[k];
-  if (St)
-    launch_pdl(k_gmres_finish<true>, dim3(1), dim3(1024), st, L, V[l + 1], n, S, l, lmax, St, *C);
-  else
-    launch_pdl(k_gmres_finish<false>, dim3(1), dim3(1024), st, L, V[l + 1], n, S, l, lmax, St,
-               NkConds{});
+  launch_pdl(k_gmres_finish, dim3(1), dim3(1024), st, L, V[l + 1], n, S, l, lmax, St,
+             C ? *C : NkConds{});
 }
 
 void launch_gmres_scalar(int op, double *S, int l, int lmax, cudaStream_t st) {

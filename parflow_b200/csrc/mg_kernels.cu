@@ -799,9 +799,9 @@ __global__ void __launch_bounds__(256) k_mg_residual(MGLevel<T> L, const T *__re
 
 // The residual right after a red/black sweep of colour zc: the cells of that
 // colour were just solved against their current neighbours, so their
-// residual is zero up to rounding and is written as zero; one thread per
-// pair of cells (i, i+1) of a row, one of each colour, computes the other
-// cell's residual as k_mg_residual does.
+// residual is zero up to rounding and neither computed nor stored; one thread
+// per pair of cells (i, i+1) of a row computes the other one's, stored in the
+// layout of x (whole lines of one colour).
 template <typename T, bool H>
 __global__ void __launch_bounds__(256) k_mg_residual_pair(MGLevel<T> L, const T *__restrict__ x,
                                                           const T *__restrict__ b,
@@ -815,11 +815,8 @@ __global__ void __launch_bounds__(256) k_mg_residual_pair(MGLevel<T> L, const T 
   if (i0 >= nx || j >= L.ny) return;
   // colour 0 (red) is parity 1 of i + j + k
   const int zpar = zc == 0 ? 1 : 0;
-  const int iz = ((i0 + j + k) & 1) == zpar ? i0 : i0 + 1;  // the zero-residual cell
-  const int ic = iz == i0 ? i0 + 1 : i0;                     // the computed cell
-  const int row = nx * (j + L.ny * k);
-  if (iz < nx) r[iz + row] = T(0);
-  if (ic < nx) r[ic + row] = point_residual<T, H>(L, x, b, ic, j, k);
+  const int ic = ((i0 + j + k) & 1) == zpar ? i0 + 1 : i0;  // the computed cell
+  if (ic < nx) r[xb_index(L, ic, j, k)] = point_residual<T, H>(L, x, b, ic, j, k);
 }
 
 // Residual and restriction in one launch, right after a red/black sweep, on
@@ -912,10 +909,13 @@ __device__ __forceinline__ void restrict_cell(const MGLevel<T> &F, const MGLevel
 
 // grid form of restrict_cell with the direction D fixed at compile time and
 // 32-bit indices (same operations, same order)
-template <typename T, bool H, int D>
+// PAIR: of the residual only the colour that was not swept last (parity
+// zpar ^ 1) is there, in the layout of x; the other is zero.  It halves the
+// bytes of the residual, stored and read.
+template <typename T, bool H, int D, bool PAIR>
 __global__ void __launch_bounds__(256) k_restrict(MGLevel<T> F, MGLevel<T> C,
                                                   const T *__restrict__ rf, T *__restrict__ rc,
-                                                  int flip, int init) {
+                                                  int flip, int zpar, int init) {
   pdl_enter();
   const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
   const int ic = blockIdx.x * blockDim.x + threadIdx.x;
@@ -932,10 +932,22 @@ __global__ void __launch_bounds__(256) k_restrict(MGLevel<T> F, MGLevel<T> C,
   const T *w1 = H ? F.q1 : F.p1;
   const T *w2 = H ? F.q2 : F.p2;
   const bool lo = cd > 0, hi = cd + 1 < nd;
-  const T wc = H ? ldro(w1 + f) : T(0), wl = lo ? ldro(w2 + f - so) : T(0),
-          wh = hi ? ldro(w1 + f + so) : T(0);
-  const T v = restrict_value<T, H>(wc, ldro(rf + f), wl, lo ? ldro(rf + f - so) : T(0), wh,
-                                   hi ? ldro(rf + f + so) : T(0));
+  T v;
+  if constexpr (PAIR) {
+    const bool comp = ((i + j + k) & 1) != zpar;  // f holds the other colour
+    const bool l2 = lo && !comp, h2 = hi && !comp;
+    const int xf = xb_index(F, i, j, k);
+    // f - so and f + so in the layout of x
+    const int xm = l2 ? xb_index(F, i - ox, j - oy, k - oz) : xf;
+    const int xp = h2 ? xb_index(F, i + ox, j + oy, k + oz) : xf;
+    v = restrict_value<T, H>(H && comp ? ldro(w1 + f) : T(0), comp ? ldro(rf + xf) : T(0),
+                             l2 ? ldro(w2 + f - so) : T(0), l2 ? ldro(rf + xm) : T(0),
+                             h2 ? ldro(w1 + f + so) : T(0), h2 ? ldro(rf + xp) : T(0));
+  } else {
+    v = restrict_value<T, H>(H ? ldro(w1 + f) : T(0), ldro(rf + f), lo ? ldro(w2 + f - so) : T(0),
+                             lo ? ldro(rf + f - so) : T(0), hi ? ldro(w1 + f + so) : T(0),
+                             hi ? ldro(rf + f + so) : T(0));
+  }
   const int xi = xb_index(C, ic, jc, kc);
   rc[xi] = v;
   // the zero-guess red sweep of the coarse level
@@ -1007,6 +1019,82 @@ __global__ void __launch_bounds__(256) k_prolong_add(MGLevel<T> F, MGLevel<T> C,
   pdl_enter();
   const T el = ldro(ec + clo), eh = has_hi ? ldro(ec + chi) : T(0);
   xf[xc] = add_rn(xv, prolong_value<T, H>(odd, w1, w2, el, eh));
+}
+
+// Prolongation and the first red sweep of the post-smoother in one launch, on
+// levels where a launch costs more than its work.  The red sweep reads the
+// corrected black cells, and the black sweep after it overwrites them unread:
+// so a red cell's thread corrects its six black neighbours for itself
+// (six times the weights and coarse values from the caches) and nothing black
+// is written.
+template <typename T, bool H, int D>
+__global__ void __launch_bounds__(256) k_prolong_red(MGLevel<T> F, MGLevel<T> C,
+                                                     const T *__restrict__ ec,
+                                                     T *__restrict__ x, const T *__restrict__ b,
+                                                     int flip) {
+  const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
+  const int j = by * blockDim.y + threadIdx.y;
+  const int k = flip ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
+  const int nx = F.nx, ny = F.ny, nz = F.nz, sy = nx, sz = nx * ny;
+  const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((1 ^ j ^ k) & 1);  // i+j+k odd
+  if (i >= nx || j >= ny) return;
+  const int c = i + sy * j + sz * k;
+  const bool has[6] = {i > 0, i + 1 < nx, j > 0, j + 1 < ny, k > 0, k + 1 < nz};
+  const int dc[6] = {-1, 1, -sy, sy, -sz, sz};
+  auto op = [&](int s, int q) -> T {  // E / N / U entry s of cell q
+    if constexpr (H)
+      return (T)ldro_h(F.h[s] + q);
+    else
+      return ldro(F.a[s + 1] + q);
+  };
+  const T *w1p = H ? F.q1 : F.p1, *w2p = H ? F.q2 : F.p2;
+  // everything but the coarse iterate ahead of the wait
+  T co[6], w1[6], w2[6], xv[6];
+  int lo[6], hi[6];
+  bool odd[6], two[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    co[q] = q & 1 ? op(q >> 1, c) : has[q] ? op(q >> 1, c + dc[q]) : T(0);
+    w1[q] = w2[q] = xv[q] = T(0);
+    lo[q] = hi[q] = 0;
+    odd[q] = two[q] = false;
+    if (has[q]) {
+      const int in = i + (q == 0 ? -1 : q == 1 ? 1 : 0), jn = j + (q == 2 ? -1 : q == 3 ? 1 : 0),
+                kn = k + (q == 4 ? -1 : q == 5 ? 1 : 0);
+      const int cd = D == 0 ? in : D == 1 ? jn : kn, nd = D == 0 ? nx : D == 1 ? ny : nz;
+      const int cl = cd >> 1;
+      odd[q] = cd & 1;
+      two[q] = odd[q] && cd + 1 < nd;
+      lo[q] = D == 0 ? xb_index(C, cl, jn, kn) : D == 1 ? xb_index(C, in, cl, kn)
+                                                       : xb_index(C, in, jn, cl);
+      hi[q] = D == 0 ? xb_index(C, cl + 1, jn, kn) : D == 1 ? xb_index(C, in, cl + 1, kn)
+                                                           : xb_index(C, in, jn, cl + 1);
+      if (H || odd[q]) w1[q] = ldro(w1p + c + dc[q]);
+      if (odd[q]) w2[q] = ldro(w2p + c + dc[q]);
+      xv[q] = ldro(x + xb_index(F, in, jn, kn));
+    }
+  }
+  const int xo = xb_index(F, i, j, k);
+  T d = T(1);
+  bool unit = false;
+  if constexpr (H) {
+    unit = ldro(F.hflag) == 0;
+    if (!unit) d = (T)ldro_h(F.h[3] + c);
+  } else {
+    d = ldro(F.a[0] + c);
+  }
+  const T bc = ldro(b + xo);
+  pdl_enter();
+  T acc = T(0);
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    T v = T(0);
+    if (has[q])
+      v = add_rn(xv[q], prolong_value<T, H>(odd[q], w1[q], w2[q], ldro(ec + lo[q]),
+                                            two[q] ? ldro(ec + hi[q]) : T(0)));
+    acc = q == 0 ? mul_rn(co[0], v) : fma(co[q], v, acc);
+  }
+  x[xo] = unit ? bc - acc : (bc - acc) / d;
 }
 
 // ---------------------------------------------------------------------------
@@ -1610,8 +1698,8 @@ int launch_mg_smooth(const MGLevel<T> &L, T *x, const T *b, int zero, int smooth
     rb_sweep(L, x, b, 0, 0, st, 0, h16, 1);
     return 1;
   }
-  // zero: 1 zero initial guess, 2 the same with its red sweep already done by
-  // the kernel that wrote b.  With a zero guess the kernel before the first
+  // zero: 1 zero initial guess, 2 the first red sweep is already done by the
+  // kernel that wrote b (pre-smoother), 3 by the one that prolonged.  With a zero guess the kernel before the first
   // sweep is the one that writes b.
   if (zero == 1 && zero_sweep_from_b(L, smoother, h16)) {
     // the black sweep reads the zero-guess red values from b; the last red
@@ -1622,7 +1710,7 @@ int launch_mg_smooth(const MGLevel<T> &L, T *x, const T *b, int zero, int smooth
     return 2;
   }
   int k = 0;
-  if (zero != 2) {
+  if (zero < 2) {
     rb_sweep(L, x, b, 0, zero, st, f, h16, zero == 0);
     k++;
   }
@@ -1726,16 +1814,16 @@ void launch_mg_residual(const MGLevel<T> &L, const T *x, const T *b, T *r, cudaS
   }
   launch_pdl(k_mg_residual<T, false>, dim3(g.grid), dim3(g.block), st, L, x, b, r, flip);
 }
-template <typename T, bool H>
+template <typename T, bool H, bool PAIR>
 static void restrict_d(const MGLevel<T> &F, const MGLevel<T> &C, const T *rf, T *rc,
-                       cudaStream_t st, int flip, int init) {
+                       cudaStream_t st, int flip, int zpar, int init) {
   Shape3 g = shape3(C.nx, C.ny, C.nz);
   if (F.dir == 0)
-    launch_pdl(k_restrict<T, H, 0>, g.grid, g.block, st, F, C, rf, rc, flip, init);
+    launch_pdl(k_restrict<T, H, 0, PAIR>, g.grid, g.block, st, F, C, rf, rc, flip, zpar, init);
   else if (F.dir == 1)
-    launch_pdl(k_restrict<T, H, 1>, g.grid, g.block, st, F, C, rf, rc, flip, init);
+    launch_pdl(k_restrict<T, H, 1, PAIR>, g.grid, g.block, st, F, C, rf, rc, flip, zpar, init);
   else
-    launch_pdl(k_restrict<T, H, 2>, g.grid, g.block, st, F, C, rf, rc, flip, init);
+    launch_pdl(k_restrict<T, H, 2, PAIR>, g.grid, g.block, st, F, C, rf, rc, flip, zpar, init);
 }
 template <typename T, bool H, bool BLACK>
 static void prolong_d(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, T *xf,
@@ -1750,14 +1838,45 @@ static void prolong_d(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, T *
 }
 template <typename T>
 void launch_mg_restrict(const MGLevel<T> &F, const MGLevel<T> &C, const T *rf, T *rc,
-                        cudaStream_t st, int flip, bool h16, int init) {
+                        cudaStream_t st, int flip, bool h16, int zero_colour, int init) {
+  const int zpar = zero_colour == 0 ? 1 : 0;  // colour 0 (red) is parity 1 of i + j + k
   if constexpr (kHasH16<T>) {
     if (h16) {
-      restrict_d<T, true>(F, C, rf, rc, st, flip, init);
+      if (zero_colour >= 0)
+        restrict_d<T, true, true>(F, C, rf, rc, st, flip, zpar, init);
+      else
+        restrict_d<T, true, false>(F, C, rf, rc, st, flip, 0, init);
       return;
     }
   }
-  restrict_d<T, false>(F, C, rf, rc, st, flip, init);
+  if (zero_colour >= 0)
+    restrict_d<T, false, true>(F, C, rf, rc, st, flip, zpar, init);
+  else
+    restrict_d<T, false, false>(F, C, rf, rc, st, flip, 0, init);
+}
+template <typename T, bool H>
+static void prolong_red_d(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, cudaStream_t st,
+                          int flip) {
+  const Shape3 g = shape3((F.nx + 1) / 2, F.ny, F.nz);
+  T *x = F.x;
+  const T *b = F.b;
+  if (F.dir == 0)
+    launch_pdl(k_prolong_red<T, H, 0>, g.grid, g.block, st, F, C, ec, x, b, flip);
+  else if (F.dir == 1)
+    launch_pdl(k_prolong_red<T, H, 1>, g.grid, g.block, st, F, C, ec, x, b, flip);
+  else
+    launch_pdl(k_prolong_red<T, H, 2>, g.grid, g.block, st, F, C, ec, x, b, flip);
+}
+template <typename T>
+void launch_mg_prolong_red(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, cudaStream_t st,
+                           int flip, bool h16) {
+  if constexpr (kHasH16<T>) {
+    if (h16) {
+      prolong_red_d<T, true>(F, C, ec, st, flip);
+      return;
+    }
+  }
+  prolong_red_d<T, false>(F, C, ec, st, flip);
 }
 template <typename T, bool H>
 static void resid_restrict_d(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st, int flip,
@@ -2251,8 +2370,10 @@ void launch_convert(const TI *in, TO *out, long long n, cudaStream_t st, int fli
   template void launch_mg_resid_restrict<T>(const MGLevel<T> &, const MGLevel<T> &,            \
                                             cudaStream_t, int, bool, int);                    \
   template bool mg_wants_red_init<T>(const MGLevel<T> &, int, bool);                           \
+  template void launch_mg_prolong_red<T>(const MGLevel<T> &, const MGLevel<T> &, const T *,   \
+                                         cudaStream_t, int, bool);                            \
   template void launch_mg_restrict<T>(const MGLevel<T> &, const MGLevel<T> &, const T *, T *, \
-                                      cudaStream_t, int, bool, int);                               \
+                                      cudaStream_t, int, bool, int, int);                               \
   template void launch_mg_prolong_add<T>(const MGLevel<T> &, const MGLevel<T> &, const T *,   \
                                          T *, cudaStream_t, int, bool, int);                  \
   template void launch_vcycle_mid<T>(const MGLevel<T> *, int, int, int, int, double, T *,       \

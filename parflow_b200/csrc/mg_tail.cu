@@ -445,13 +445,13 @@ void launch_tail_pack(const MGLevel<T> *L, int first, int nl, int smoother, void
 
 template <typename T>
 void launch_tail_pairs(const MGLevel<T> *L, int first, int nl, int smoother, void *image,
-                       cudaStream_t st, bool h16) {
+                       cudaStream_t st, bool h16, const T *b, T *x) {
   TailPlan P;
   const size_t smem = (size_t)tail_layout(L, first, nl, h16, &P, nullptr);
   P.nonsym = smoother == 2;
   P.image = image;
-  P.b = L[first].b;
-  P.x = L[first].x;
+  P.b = b ? b : L[first].b;
+  P.x = x ? x : L[first].x;
   P.hflag = L[first].hflag;
   if constexpr (std::is_same<T, float>::value) {
     if (h16) {
@@ -468,7 +468,7 @@ void launch_tail_pairs(const MGLevel<T> *L, int first, int nl, int smoother, voi
   template void launch_tail_pack<T>(const MGLevel<T> *, int, int, int, void *, cudaStream_t, \
                                     bool);                                                   \
   template void launch_tail_pairs<T>(const MGLevel<T> *, int, int, int, void *, cudaStream_t, \
-                                     bool);
+                                     bool, const T *, T *);
 INST(double)
 INST(float)
 

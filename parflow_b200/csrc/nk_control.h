@@ -104,6 +104,11 @@ void launch_nk_final(NkState *S, cudaStream_t st);
 // update, residual estimate; St given: also the graph's control step
 void launch_gmres_finish(double *const *V, int l, int lmax, long long n, double *S,
                          cudaStream_t st, NkState *St = nullptr, const NkConds *C = nullptr);
+// the same with Gram-Schmidt itself, in one launch (gmres_mgs_fits(n))
+bool gmres_mgs_fits(long long n);
+void launch_gmres_mgs(double *const *V, int l, int lmax, long long n, double *S, cudaStream_t st,
+                      NkState *St = nullptr, const NkConds *C = nullptr);
+cudaError_t krylov_prepare_kernels();
 void launch_v0_init(double *v0, const double *src, const NkState *S, const double *sc,
                     long long n, cudaStream_t st);
 void launch_gmres_scalar_dev(int op, double *S, const int *l, int lmax, cudaStream_t st);

@@ -517,6 +517,11 @@ static long long mg_setup_T(MG<T> &mg, int smoother, cudaStream_t st) {
   return k;
 }
 
+// grid levels up to this size take prolongation and first red sweep in one
+// launch (timestep of 197x123x37: 6.5 ms, 6.8 with a limit of 400000; ensemble
+// of eight: 9.8 ms against 10.4)
+constexpr long long PROLONG_RED_CELLS = 30000;
+
 // the input conversion of level 0 also does its zero-guess red sweep
 template <typename T>
 static bool level0_red_done(const MG<T> &mg, int smoother) {
@@ -588,7 +593,7 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
       continue;
     }
     launch_mg_residual<T>(Ll, Ll.x, Ll.b, Ll.t, st, next(), mg.h16, Ll.zc);
-    launch_mg_restrict<T>(Ll, C, Ll.t, C.b, st, next(), mg.h16, red_done ? 1 : 0);
+    launch_mg_restrict<T>(Ll, C, Ll.t, C.b, st, next(), mg.h16, Ll.zc, red_done ? 1 : 0);
     k += 2;
   }
   // levels first .. nl-1, coarse solve (RedBlackGSPoint, mg_semi.c:1276) included
@@ -617,7 +622,12 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
     // the plain red/black post-smoothers begin with a red sweep
     const int skip_red = (smoother == PFGPU_SMOOTH_RBGS || smoother == PFGPU_SMOOTH_RBGS_NONSYM) &&
                          !mg.fused[l] && !mg.waved[l];
-    launch_mg_prolong_add<T>(Ll, C, mg.res(l + 1), Ll.x, st, next(), mg.h16, skip_red);
+    const bool with_red =
+        skip_red && !Ll.lo[0] && Ll.n <= std::min(mg.fuse_cells, PROLONG_RED_CELLS);
+    if (with_red)
+      launch_mg_prolong_red<T>(Ll, C, mg.res(l + 1), st, next(), mg.h16);
+    else
+      launch_mg_prolong_add<T>(Ll, C, mg.res(l + 1), Ll.x, st, next(), mg.h16, skip_red);
     if (Ll.lo[0]) {
       k += 1 + launch_mg_full_smooth<T>(Ll, Ll.x, Ll.b, 0,
                                         smoother != PFGPU_SMOOTH_RBGS_NONSYM, st);
@@ -629,7 +639,8 @@ static long long vcycle_T(MG<T> &mg, int smoother, double w, cudaStream_t st,
       f = mg.flip ? 1 : 0;
       k += 2;
     } else {
-      k += 1 + launch_mg_smooth<T>(Ll, Ll.x, Ll.b, 0, smoother, w, mg.wtmp, st, fp, mg.h16);
+      k += 1 + launch_mg_smooth<T>(Ll, Ll.x, Ll.b, with_red ? 3 : 0, smoother, w, mg.wtmp, st, fp,
+                                   mg.h16);
     }
   }
   }
@@ -672,6 +683,15 @@ static int pc_apply_dense_impl(pfgpu_handle *h, const double *r, double *z,
     // MGSemi.MaxIter 0: x = b (mg_semi.c:198-203)
     if (z != r)
       CK(cudaMemcpyAsync(z, r, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+    return 0;
+  }
+  if (!h->mixed && h->nk.capturing && h->mg_max_iter == 1 && h->mgd.mid == 0 &&
+      h->mgd.tail_image) {
+    // the whole hierarchy is the tail: straight from r to z
+    launch_tail_pairs<double>(h->mgd.L.data(), 0, (int)h->mgd.L.size(), h->d.mg_smoother,
+                              h->mgd.tail_image, h->st, false, r, z);
+    h->launches++;
+    CK(cudaGetLastError());
     return 0;
   }
   if (h->mixed)
@@ -754,6 +774,31 @@ static void atimes(pfgpu_handle *h, const double *u, double dt, const double *v,
   h->launches++;
 }
 
+// ModifiedGS (iterativ.c:30-86) of V[l + 1] and the scalar end of GMRES
+// iteration l: one cluster launch where the vector fits it; else <vk,vk> and
+// h(0) in one pass, each projection vk -= h(i) v_i fused with the next dot
+// (h(i+1), or the new <vk,vk> after the last), and the scalars.  St, C: the
+// graph solve's control step too.
+static void orthogonalise(pfgpu_handle *h, int l, NkState *St, const NkConds *C) {
+  const long long N = h->N;
+  const int lmax = h->d.krylov_dim, k = l + 1;
+  double *S = h->gs, *sc = S + gs_sc_offset(lmax);
+  auto Hp = [&](int i, int j) { return S + (long long)i * lmax + j; };
+  if (gmres_mgs_fits(N)) {
+    launch_gmres_mgs(h->V.data(), l, lmax, N, S, h->st, St, C);
+    h->launches++;
+    return;
+  }
+  launch_mgs_first(h->V[k], h->V[0], N, sc + SCI_VKNORM2, Hp(0, k - 1), h->rb, h->st);
+  for (int i = 0; i < k; i++) {
+    const bool more = i + 1 < k;
+    launch_axpy_dot(h->V[k], h->V[i], Hp(i, k - 1), -1.0, more ? h->V[i + 1] : nullptr, N,
+                    more ? Hp(i + 1, k - 1) : sc + SCI_NEWNORM2, h->rb, h->st);
+  }
+  launch_gmres_finish(h->V.data(), l, lmax, N, S, h->st, St, C);
+  h->launches += k + 2;
+}
+
 static int spgmr(pfgpu_handle *h, double *x, const double *src, double bsign,
                  const double *bn2_dev, double bnorm, double delta, const double *u, double dt,
                  pfgpu_stats *stats, int *status) {
@@ -816,20 +861,7 @@ static int spgmr(pfgpu_handle *h, double *x, const double *src, double bsign,
       if (pc_apply_dense(h, h->V[l], z, scales ? vl : VScale{})) return PFGPU_ERR_CUDA;
       stats->pc_solves++;
       atimes(h, u, dt, z, h->V[l + 1], stats);
-      // ModifiedGS (iterativ.c:30-86): <vk,vk> and h(0) in one pass, then each
-      // projection vk -= h(i) v_i fused with the next dot (h(i+1), or the
-      // new <vk,vk> after the last); same per-element arithmetic
-      const int k = l + 1;
-      launch_mgs_first(h->V[k], h->V[0], N, sc + SCI_VKNORM2, Hp(0, k - 1), h->rb, h->st);
-      h->launches++;
-      for (int i = 0; i < k; i++) {
-        const bool more = i + 1 < k;
-        launch_axpy_dot(h->V[k], h->V[i], Hp(i, k - 1), -1.0, more ? h->V[i + 1] : nullptr, N,
-                        more ? Hp(i + 1, k - 1) : sc + SCI_NEWNORM2, h->rb, h->st);
-        h->launches++;
-      }
-      launch_gmres_finish(h->V.data(), l, lmax, N, S, h->st);
-      h->launches++;
+      orthogonalise(h, l, nullptr, nullptr);
       CK(cudaMemcpyAsync(h->hsc + D_COUNT, sc + SCI_RHO, sizeof(double), cudaMemcpyDeviceToHost,
                          h->st));
       CK(cudaStreamSynchronize(h->st));
@@ -1246,17 +1278,7 @@ static int nk_gmres_iter(pfgpu_handle *h, int l, double dt, NkConds &C) {
                            : VScale{VScale::INV, h->V[l], nullptr, Hp(l, l - 1), 0.0, nullptr};
   if (pc_apply_dense_impl(h, h->V[l], z, scales ? vl : VScale{})) return PFGPU_ERR_CUDA;
   atimes(h, h->u, dt, z, h->V[l + 1], &dummy);
-  const int k = l + 1;
-  launch_mgs_first(h->V[k], h->V[0], N, sc + SCI_VKNORM2, Hp(0, k - 1), h->rb, h->st);
-  h->launches++;
-  for (int i = 0; i < k; i++) {
-    const bool more = i + 1 < k;
-    launch_axpy_dot(h->V[k], h->V[i], Hp(i, k - 1), -1.0, more ? h->V[i + 1] : nullptr, N,
-                    more ? Hp(i + 1, k - 1) : sc + SCI_NEWNORM2, h->rb, h->st);
-    h->launches++;
-  }
-  launch_gmres_finish(h->V.data(), l, lmax, N, S, h->st, h->nk.S, &C);
-  h->launches++;
+  orthogonalise(h, l, h->nk.S, &C);
   // the next iteration scales V[l + 1] as it enters the preconditioner; the
   // last one meets none, but a restart uses it
   if (!scales || l + 1 == lmax) {
@@ -1773,10 +1795,10 @@ static int alloc_mg(pfgpu_handle *h, MG<T> &mg) {
     L.hx = (nx + 1) / 2;
     for (int s = 0; s < 4; s++)
       if (dalloc(&L.a[s], L.n)) return PFGPU_ERR_NOMEM;
-    // x and b sized for the colour-split layout too (one slot more per row of
+    // x, b and t sized for the colour-split layout too (one slot more per row of
     // the shorter colour when nx is odd)
     const long long nxb = std::max(L.n, 2LL * L.hx * ny * nz);
-    if (dalloc(&L.x, nxb) || dalloc(&L.b, nxb) || dalloc(&L.t, L.n)) return PFGPU_ERR_NOMEM;
+    if (dalloc(&L.x, nxb) || dalloc(&L.b, nxb) || dalloc(&L.t, nxb)) return PFGPU_ERR_NOMEM;
     if (dalloc(&L.wg, (long long)ny * nz)) return PFGPU_ERR_NOMEM;
     CK(cudaMemset(L.wg, 0, (long long)ny * nz * sizeof(T)));
     if (l < nl - 1) {
@@ -2005,6 +2027,7 @@ static int create_impl(pfgpu_handle *h) {
   const long long N = h->N;
   CK(cudaSetDevice(h->device));
   CK(mg_prepare_kernels());
+  CK(krylov_prepare_kernels());
   CK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
   double **vecs[] = {&h->kx, &h->u, &h->unew, &h->fval, &h->pp, &h->bb, &h->p_old,
                      &h->s_old, &h->kr, &h->dkr, &h->sat, &h->dsat, &h->xcor, &h->vtemp};

@@ -217,14 +217,20 @@ int launch_mg_smooth(const MGLevel<T> &L, T *x, const T *b, int zero, int smooth
 cudaError_t mg_prepare_kernels();
 // h16: the level's scaled FP16 operator and weights (float levels only)
 // r = b - A x; zero_colour >= 0: right after a sweep of that colour, whose
-// cells' residual is written as zero
+// cells' residual is zero: only the other colour's is computed, stored in the
+// layout of x (L.t holds either)
 template <typename T>
 void launch_mg_residual(const MGLevel<T> &L, const T *x, const T *b, T *r, cudaStream_t st,
                         int flip = 0, bool h16 = false, int zero_colour = -1);
-// init: also the zero-guess red sweep of C
+// of such a residual (zero_colour); init: also the zero-guess red sweep of C
 template <typename T>
 void launch_mg_restrict(const MGLevel<T> &F, const MGLevel<T> &C, const T *rf, T *rc,
-                        cudaStream_t st, int flip = 0, bool h16 = false, int init = 0);
+                        cudaStream_t st, int flip = 0, bool h16 = false, int zero_colour = -1,
+                        int init = 0);
+// prolongation and the first red sweep of a red/black post-smoother
+template <typename T>
+void launch_mg_prolong_red(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, cudaStream_t st,
+                           int flip, bool h16);
 // both in one launch from F.x, F.b to C.b, after a red/black smoother (F.zc >= 0)
 template <typename T>
 void launch_mg_resid_restrict(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st, int flip,
@@ -293,9 +299,10 @@ cudaError_t tail_pairs_prepare();
 template <typename T>
 void launch_tail_pack(const MGLevel<T> *levels_host, int first, int nl, int smoother, void *image,
                       cudaStream_t st, bool h16);
+// (b, x: in place of the first level's own)
 template <typename T>
 void launch_tail_pairs(const MGLevel<T> *levels_host, int first, int nl, int smoother, void *image,
-                       cudaStream_t st, bool h16);
+                       cudaStream_t st, bool h16, const T *b = nullptr, T *x = nullptr);
 // setup of the tail levels (weights, coarse operators and, h16, their scaled
 // operators); returns the kernels launched
 constexpr size_t SETUP_TAIL_SMEM_MAX = 160 * 1024;
