@@ -57,8 +57,10 @@ struct OpStepDiff {  // |a - b| / (1 + |a|)  (KINStop, kinsol.c:1541-1544)
 
 template <typename Op>
 __global__ void __launch_bounds__(RED_THREADS) k_reduce(Op op, long long n, double *partial,
-                                                        double *dst, unsigned int *ticket) {
+                                                        double *dst, unsigned int *ticket,
+                                                        const int *gate) {
   pdl_enter();
+  if (gate && !*gate) return;  // not needed this time
   __shared__ double sh[RED_THREADS / 32];
   __shared__ bool last;
   double acc = Op::init();
@@ -79,10 +81,15 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce(Op op, long long n, doub
   if (threadIdx.x == 0) {
     double b = sh[0];
     for (int w = 1; w < RED_THREADS / 32; w++) b = Op::comb(b, sh[w]);
-    partial[blockIdx.x] = b;
-    __threadfence();
-    unsigned int t = atomicAdd(ticket, 1u);
-    last = (t == gridDim.x - 1);
+    if (gridDim.x == 1) {
+      *dst = b;
+      last = false;
+    } else {
+      partial[blockIdx.x] = b;
+      __threadfence();
+      unsigned int t = atomicAdd(ticket, 1u);
+      last = (t == gridDim.x - 1);
+    }
   }
   __syncthreads();
   if (!last) return;
@@ -107,8 +114,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce(Op op, long long n, doub
 }
 
 template <typename Op>
-static void reduce(Op op, long long n, double *dst, ReduceBuf rb, cudaStream_t st) {
-  launch_pdl(k_reduce<Op>, dim3(red_grid(n, rb.blocks)), dim3(RED_THREADS), st, op, n, rb.partial, dst, rb.ticket);
+static void reduce(Op op, long long n, double *dst, ReduceBuf rb, cudaStream_t st,
+                   const int *gate = nullptr) {
+  launch_pdl(k_reduce<Op>, dim3(red_grid(n, rb.blocks)), dim3(RED_THREADS), st, op, n, rb.partial, dst, rb.ticket, gate);
 }
 
 void launch_dot(const double *a, const double *b, long long n, double *dst, ReduceBuf rb,
@@ -121,9 +129,9 @@ void launch_maxabs(const double *a, long long n, double *dst, ReduceBuf rb, cuda
   reduce(op, n, dst, rb, st);
 }
 void launch_steplen(const double *s, const double *u, long long n, double *dst, ReduceBuf rb,
-                    cudaStream_t st) {
+                    cudaStream_t st, const int *gate) {
   OpStep op{s, u};
-  reduce(op, n, dst, rb, st);
+  reduce(op, n, dst, rb, st, gate);
 }
 void launch_steplen_diff(const double *a, const double *b, long long n, double *dst,
                          ReduceBuf rb, cudaStream_t st) {
@@ -174,11 +182,17 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_multi(Op op, long long n
     for (int q = 0; q < K; q++) {
       double b = sh[q][0];
       for (int w = 1; w < RED_THREADS / 32; w++) b = Op::comb(q, b, sh[q][w]);
-      partial[q * gridDim.x + blockIdx.x] = b;
+      if (gridDim.x == 1)
+        *o.dst[q] = b;
+      else
+        partial[q * gridDim.x + blockIdx.x] = b;
     }
-    __threadfence();
-    unsigned int t = atomicAdd(ticket, 1u);
-    last = (t == gridDim.x - 1);
+    last = false;
+    if (gridDim.x > 1) {
+      __threadfence();
+      unsigned int t = atomicAdd(ticket, 1u);
+      last = (t == gridDim.x - 1);
+    }
   }
   __syncthreads();
   if (!last) return;
@@ -575,8 +589,10 @@ __global__ void k_fill_if(double *__restrict__ x, double v, const int *flag, lon
        i += (long long)gridDim.x * blockDim.x)
     x[i] = v;
 }
-__global__ void k_scale_by(double *__restrict__ x, const double *a_p, long long n) {
+__global__ void k_scale_if(double *__restrict__ x, const double *a_p, const int *flag,
+                           long long n) {
   pdl_enter();
+  if (!*flag) return;
   const double a = *a_p;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -614,8 +630,8 @@ void launch_scale_inv_dev_unless(double *x, const double *s, const int *skip, lo
 void launch_fill_if(double *x, double v, const int *flag, long long n, cudaStream_t st) {
   launch_pdl(k_fill_if, dim3(grid_for(n)), dim3(256), st, x, v, flag, n);
 }
-void launch_scale_by(double *x, const double *a, long long n, cudaStream_t st) {
-  launch_pdl(k_scale_by, dim3(grid_for(n)), dim3(256), st, x, a, n);
+void launch_scale_if(double *x, const double *a, const int *flag, long long n, cudaStream_t st) {
+  launch_pdl(k_scale_if, dim3(grid_for(n)), dim3(256), st, x, a, flag, n);
 }
 void launch_copy_if(double *dst, const double *src, const int *flag, long long n,
                     cudaStream_t st) {

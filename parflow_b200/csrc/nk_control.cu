@@ -103,7 +103,6 @@ __global__ void k_nk_iter(NkState *S, NkConds c) {
     S->gm_status = 2;
     setc(c.restart, true);
   }
-  setc(c.post, false);
 }
 
 // start of a GMRES cycle: only iteration 0 is armed
@@ -134,24 +133,23 @@ __global__ void k_nk_cycle_end(NkState *S, const double *sc, NkConds c) {
     S->ntries++;
     restart = true;
   }
-  setc(c.do_restart, restart);
+  if (S->k.max_restarts > 0) setc(c.do_restart, restart);
   setc(c.restart, restart);
 }
 
-// executions of a body without a control kernel of its own (and the
-// preconditioner solves it made)
-__global__ void k_nk_count(NkState *S, int body, int pc_solves) {
+// executions of a body without a control kernel of its own
+__global__ void k_nk_count(NkState *S, int body) {
   pdl_enter();
   S->execs[body]++;
-  S->pc_solves += pc_solves;
 }
 
-// after SPGMR: its solution is M^{-1} V y unless x = 0; a failed linear
-// solve ends KINSol with 8
-__global__ void k_nk_after_gmres(NkState *S, NkConds c) {
+// after SPGMR: its solution is M^{-1} V y (post = 1; the V-cycle runs in any
+// case and counts when it is used) unless x = 0; a failed linear solve ends
+// KINSol with 8
+__global__ void k_nk_after_gmres(NkState *S, int post, NkConds c) {
   pdl_enter();
   const int st = S->gm_status;
-  setc(c.post, !S->zero_x && (st == 0 || st == 1));
+  if (!S->zero_x && (st == 0 || st == 1)) S->pc_solves += post;
   if (st != 0 && st != 1) {
     S->lin_conv_fails++;
     S->ret = 8;
@@ -166,7 +164,7 @@ __global__ void k_nk_after_gmres(NkState *S, NkConds c) {
 }
 
 // sJpnorm, sfdotJp (kinspgmr.c:384-398) and the line search's first steps
-__global__ void k_nk_ls_init(NkState *S, const double *dsc, NkConds c) {
+__global__ void k_nk_ls_init(NkState *S, const double *dsc) {
   pdl_enter();
   S->execs[NKB_OK]++;
   if (S->k.use_dq) S->fevals++;
@@ -183,10 +181,9 @@ __global__ void k_nk_ls_init(NkState *S, const double *dsc, NkConds c) {
   } else {
     S->scaled = 0;
   }
-  setc(c.scale, S->scaled != 0);
 }
 
-__global__ void k_nk_ls_setup(NkState *S, const double *dsc, NkConds c) {
+__global__ void k_nk_ls_setup(NkState *S, const double *dsc) {
   pdl_enter();
   if (S->scaled) S->pnorm = S->mxnewtstep;
   S->slpi = S->sfdotJp * S->ratio;
@@ -198,34 +195,24 @@ __global__ void k_nk_ls_setup(NkState *S, const double *dsc, NkConds c) {
   S->lam = S->rl;
   S->ls_it = 0;
   S->ls_phase = 0;
-  setc(c.ls1, true);
 }
 
-// after each trial of the backtracking loop
-__global__ void k_nk_ls1(NkState *S, const double *dsc, NkConds c) {
-  pdl_enter();
-  S->execs[NKB_LS1]++;
+// one trial of the backtracking loop; whether another follows
+__device__ __forceinline__ bool ls1_continues(NkState *S, const double *dsc) {
   take_trial(S, dsc);
-  if (S->k.inexact) {  // KINInexactNewton takes the full step (kinsol.c:1152-1208)
-    setc(c.ls1, false);
-    return;
-  }
+  // KINInexactNewton takes the full step (kinsol.c:1152-1208)
+  if (S->k.inexact) return false;
   if (S->ls_phase == 1) {  // the step was too small: u itself was re-evaluated
     S->backtracks = S->fevals - S->nfesav - 1;
     S->globalret = 1;
-    setc(c.ls1, false);
-    return;
+    return false;
   }
   S->alpha_cond = S->f1norm + LS_ALPHA * S->slpi * S->rl;
-  if (S->f1normp <= S->alpha_cond) {
-    setc(c.ls1, false);
-    return;
-  }
+  if (S->f1normp <= S->alpha_cond) return false;
   if (S->rl < S->rlmin) {
     S->ls_phase = 1;
     S->lam = 0.0;
-    setc(c.ls1, true);
-    return;
+    return true;
   }
   double rltmp = -S->slpi / (2.0 * (S->f1normp - S->f1norm - S->slpi));
   if (rltmp > 0.5 * S->rl) rltmp = 0.5 * S->rl;
@@ -235,10 +222,20 @@ __global__ void k_nk_ls1(NkState *S, const double *dsc, NkConds c) {
   S->lam = S->rl;
   if (++S->ls_it > LS_MAX_ITERS) {
     S->err = 1;
-    setc(c.ls1, false);
-    return;
+    return false;
   }
-  setc(c.ls1, true);
+  return true;
+}
+
+// after each trial of the backtracking loop.  The first one is made outside
+// the loop's conditional node; when it is accepted (at rl = 1, which the
+// refinement leaves alone) the rest of the line search is skipped as a whole.
+__global__ void k_nk_ls1(NkState *S, const double *dsc, int first, NkConds c) {
+  pdl_enter();
+  if (!first) S->execs[NKB_LS1]++;
+  const bool go_on = ls1_continues(S, dsc);
+  setc(c.ls1, go_on);
+  if (first) setc(c.more, go_on);
 }
 
 // the beta condition and the start of the refinement loop
@@ -387,20 +384,20 @@ void launch_nk_cycle_begin(NkState *S, NkConds c, cudaStream_t st) {
 void launch_nk_cycle_end(NkState *S, const double *sc, NkConds c, cudaStream_t st) {
   launch_pdl(k_nk_cycle_end, dim3(1), dim3(1), st, S, sc, c);
 }
-void launch_nk_count(NkState *S, int body, int pc_solves, cudaStream_t st) {
-  launch_pdl(k_nk_count, dim3(1), dim3(1), st, S, body, pc_solves);
+void launch_nk_count(NkState *S, int body, cudaStream_t st) {
+  launch_pdl(k_nk_count, dim3(1), dim3(1), st, S, body);
 }
-void launch_nk_after_gmres(NkState *S, NkConds c, cudaStream_t st) {
-  launch_pdl(k_nk_after_gmres, dim3(1), dim3(1), st, S, c);
+void launch_nk_after_gmres(NkState *S, int post, NkConds c, cudaStream_t st) {
+  launch_pdl(k_nk_after_gmres, dim3(1), dim3(1), st, S, post, c);
 }
-void launch_nk_ls_init(NkState *S, const double *dsc, NkConds c, cudaStream_t st) {
-  launch_pdl(k_nk_ls_init, dim3(1), dim3(1), st, S, dsc, c);
+void launch_nk_ls_init(NkState *S, const double *dsc, cudaStream_t st) {
+  launch_pdl(k_nk_ls_init, dim3(1), dim3(1), st, S, dsc);
 }
-void launch_nk_ls_setup(NkState *S, const double *dsc, NkConds c, cudaStream_t st) {
-  launch_pdl(k_nk_ls_setup, dim3(1), dim3(1), st, S, dsc, c);
+void launch_nk_ls_setup(NkState *S, const double *dsc, cudaStream_t st) {
+  launch_pdl(k_nk_ls_setup, dim3(1), dim3(1), st, S, dsc);
 }
-void launch_nk_ls1(NkState *S, const double *dsc, NkConds c, cudaStream_t st) {
-  launch_pdl(k_nk_ls1, dim3(1), dim3(1), st, S, dsc, c);
+void launch_nk_ls1(NkState *S, const double *dsc, int first, NkConds c, cudaStream_t st) {
+  launch_pdl(k_nk_ls1, dim3(1), dim3(1), st, S, dsc, first, c);
 }
 void launch_nk_ls2_init(NkState *S, NkConds c, cudaStream_t st) {
   launch_pdl(k_nk_ls2_init, dim3(1), dim3(1), st, S, c);

@@ -39,9 +39,8 @@ enum {
   NKB_NEWTON,
   NKB_CYCLE,
   NKB_RESTART,
-  NKB_POST,
   NKB_OK,
-  NKB_SCALE,
+  NKB_MORE,  // the line search beyond its first trial
   NKB_LS1,
   NKB_LS2,
   NKB_LS3,
@@ -76,7 +75,7 @@ struct NkState {
 };
 
 struct NkConds {
-  cudaGraphConditionalHandle newton, ok, scale, ls1, ls2, ls3, restart, do_restart, post;
+  cudaGraphConditionalHandle newton, ok, more, ls1, ls2, ls3, restart, do_restart;
   cudaGraphConditionalHandle iter[NK_MAX_L];  // iter[l], l >= 1: GMRES iteration l runs
 };
 
@@ -85,11 +84,13 @@ void launch_nk_init(NkState *S, const double *dsc, NkConds c, cudaStream_t st);
 void launch_nk_iter(NkState *S, NkConds c, cudaStream_t st);
 void launch_nk_cycle_begin(NkState *S, NkConds c, cudaStream_t st);
 void launch_nk_cycle_end(NkState *S, const double *sc, NkConds c, cudaStream_t st);
-void launch_nk_count(NkState *S, int body, int pc_solves, cudaStream_t st);
-void launch_nk_after_gmres(NkState *S, NkConds c, cudaStream_t st);
-void launch_nk_ls_init(NkState *S, const double *dsc, NkConds c, cudaStream_t st);
-void launch_nk_ls_setup(NkState *S, const double *dsc, NkConds c, cudaStream_t st);
-void launch_nk_ls1(NkState *S, const double *dsc, NkConds c, cudaStream_t st);
+void launch_nk_count(NkState *S, int body, cudaStream_t st);
+// post: preconditioner solves that turn SPGMR's solution into x
+void launch_nk_after_gmres(NkState *S, int post, NkConds c, cudaStream_t st);
+void launch_nk_ls_init(NkState *S, const double *dsc, cudaStream_t st);
+void launch_nk_ls_setup(NkState *S, const double *dsc, cudaStream_t st);
+// first: the trial every line search makes
+void launch_nk_ls1(NkState *S, const double *dsc, int first, NkConds c, cudaStream_t st);
 void launch_nk_ls2_init(NkState *S, NkConds c, cudaStream_t st);
 void launch_nk_ls2(NkState *S, const double *dsc, NkConds c, cudaStream_t st);
 void launch_nk_ls3_decide(NkState *S, NkConds c, cudaStream_t st);
@@ -119,7 +120,7 @@ void launch_restart_v0_dev(double *const *V, int nv, const double *yg, const int
 void launch_scale_inv_dev_unless(double *x, const double *s, const int *skip, long long n,
                                  cudaStream_t st);
 void launch_fill_if(double *x, double v, const int *flag, long long n, cudaStream_t st);
-void launch_scale_by(double *x, const double *a, long long n, cudaStream_t st);
+void launch_scale_if(double *x, const double *a, const int *flag, long long n, cudaStream_t st);
 void launch_copy_if(double *dst, const double *src, const int *flag, long long n, cudaStream_t st);
 
 }  // namespace pfgpu

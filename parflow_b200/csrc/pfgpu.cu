@@ -1172,12 +1172,14 @@ static int newton_impl(pfgpu_handle *h, double dt, pfgpu_stats *stats) {
 //       iteration 0, IF iteration 1, ..., IF iteration lmax-1
 //       QR solve; x (+)= V y; cycle_end
 //       IF restart: restart direction
-//     after_gmres; IF post: x = M^{-1} V y; x = 0 when SPGMR gave none
+//     after_gmres; x = M^{-1} V y; x = 0 when SPGMR gave none
 //     IF ok:
-//       J p, line-search inputs; ls_init; IF scale: scale p
-//       WHILE backtrack: trial; ls1
-//       WHILE refine: trial; ls2
-//       IF rllo: trial; ls3
+//       J p, line-search inputs; ls_init; scale p when it is too long
+//       trial; ls1
+//       IF more:
+//         WHILE backtrack: trial; ls1
+//         WHILE refine: trial; ls2
+//         IF rllo: trial; ls3
 //       newton_end; u <- unew
 //     tail
 //   final
@@ -1297,7 +1299,8 @@ static int nk_gmres_cycle(pfgpu_handle *h, double dt, NkConds &C) {
   NkState *St = h->nk.S;
   for (int l = 1; l < lmax; l++)
     if (nk_handle(h->st, &C.iter[l])) return PFGPU_ERR_CUDA;
-  if (nk_handle(h->st, &C.do_restart)) return PFGPU_ERR_CUDA;
+  const bool restarts = h->d.max_restarts > 0;
+  if (restarts && nk_handle(h->st, &C.do_restart)) return PFGPU_ERR_CUDA;
   launch_nk_cycle_begin(St, C, h->st);
   h->launches++;
   if (!pc_scales(h)) {
@@ -1325,11 +1328,12 @@ static int nk_gmres_cycle(pfgpu_handle *h, double dt, NkConds &C) {
                        &St->accumulate, N, h->st);
   launch_nk_cycle_end(St, sc, C, h->st);
   h->launches += 3;
+  if (!restarts) return 0;
   return nk_body(h, C.do_restart, cudaGraphCondTypeIf, 3, NKB_RESTART, [&]() {
     launch_gmres_scalar_dev(GM_RESTART, S, &St->krydim, lmax, h->st);
     launch_restart_v0_dev(h->V.data(), lmax + 1, S + gs_yg_offset(lmax), &St->krydim, N, h->st);
     launch_gmres_scalar(GM_RESTART_INIT, S, 0, lmax, h->st);
-    launch_nk_count(St, NKB_RESTART, 0, h->st);
+    launch_nk_count(St, NKB_RESTART, h->st);
     h->launches += 4;
     return 0;
   });
@@ -1341,47 +1345,48 @@ static int nk_line_search(pfgpu_handle *h, double dt, NkConds &C) {
   double *dsc = h->dsc;
   NkState *St = h->nk.S;
   pfgpu_stats dummy{};
-  if (nk_handle(h->st, &C.scale) || nk_handle(h->st, &C.ls1) || nk_handle(h->st, &C.ls2) ||
+  if (nk_handle(h->st, &C.more) || nk_handle(h->st, &C.ls1) || nk_handle(h->st, &C.ls2) ||
       nk_handle(h->st, &C.ls3))
     return PFGPU_ERR_CUDA;
   atimes(h, h->u, dt, h->pp, h->bb, &dummy);
   launch_linesearch_inputs(h->bb, h->fval, h->pp, h->u, N, dsc + D_JP2, dsc + D_FJP, dsc + D_P2,
                            dsc + D_PLEN, h->rb, h->st);
-  launch_nk_ls_init(St, dsc, C, h->st);
-  h->launches += 2;
-  int rc = nk_body(h, C.scale, cudaGraphCondTypeIf, 3, NKB_SCALE, [&]() {
-    launch_scale_by(h->pp, &St->ratio, N, h->st);
-    launch_steplen(h->pp, h->u, N, dsc + D_PLEN, h->rb, h->st);
-    launch_nk_count(St, NKB_SCALE, 0, h->st);
-    h->launches += 3;
-    return 0;
-  });
-  if (rc) return rc;
-  launch_nk_ls_setup(St, dsc, C, h->st);
-  h->launches++;
-  rc = nk_body(h, C.ls1, cudaGraphCondTypeWhile, 3, NKB_LS1, [&]() {
-    nk_try_step(h, dt);
-    launch_nk_ls1(St, dsc, C, h->st);
+  launch_nk_ls_init(St, dsc, h->st);
+  // a step longer than the maximum (two launches that return at once
+  // otherwise: a conditional node costs more)
+  launch_scale_if(h->pp, &St->ratio, &St->scaled, N, h->st);
+  launch_steplen(h->pp, h->u, N, dsc + D_PLEN, h->rb, h->st, &St->scaled);
+  launch_nk_ls_setup(St, dsc, h->st);
+  nk_try_step(h, dt);
+  launch_nk_ls1(St, dsc, 1, C, h->st);
+  h->launches += 6;
+  int rc = nk_body(h, C.more, cudaGraphCondTypeIf, 3, NKB_MORE, [&]() {
+    launch_nk_count(St, NKB_MORE, h->st);
     h->launches++;
-    return 0;
-  });
-  if (rc) return rc;
-  launch_nk_ls2_init(St, C, h->st);
-  h->launches++;
-  rc = nk_body(h, C.ls2, cudaGraphCondTypeWhile, 3, NKB_LS2, [&]() {
-    nk_try_step(h, dt);
-    launch_nk_ls2(St, dsc, C, h->st);
+    int r = nk_body(h, C.ls1, cudaGraphCondTypeWhile, 4, NKB_LS1, [&]() {
+      nk_try_step(h, dt);
+      launch_nk_ls1(St, dsc, 0, C, h->st);
+      h->launches++;
+      return 0;
+    });
+    if (r) return r;
+    launch_nk_ls2_init(St, C, h->st);
     h->launches++;
-    return 0;
-  });
-  if (rc) return rc;
-  launch_nk_ls3_decide(St, C, h->st);
-  h->launches++;
-  rc = nk_body(h, C.ls3, cudaGraphCondTypeIf, 3, NKB_LS3, [&]() {
-    nk_try_step(h, dt);
-    launch_nk_ls3(St, dsc, h->st);
+    r = nk_body(h, C.ls2, cudaGraphCondTypeWhile, 4, NKB_LS2, [&]() {
+      nk_try_step(h, dt);
+      launch_nk_ls2(St, dsc, C, h->st);
+      h->launches++;
+      return 0;
+    });
+    if (r) return r;
+    launch_nk_ls3_decide(St, C, h->st);
     h->launches++;
-    return 0;
+    return nk_body(h, C.ls3, cudaGraphCondTypeIf, 4, NKB_LS3, [&]() {
+      nk_try_step(h, dt);
+      launch_nk_ls3(St, dsc, h->st);
+      h->launches++;
+      return 0;
+    });
   });
   if (rc) return rc;
   launch_nk_newton_end(St, h->st);
@@ -1397,8 +1402,7 @@ static int nk_newton_iter(pfgpu_handle *h, double dt, NkConds &C) {
   double *S = h->gs;
   double *sc = S + gs_sc_offset(lmax);
   NkState *St = h->nk.S;
-  if (nk_handle(h->st, &C.ok) || nk_handle(h->st, &C.restart) || nk_handle(h->st, &C.post))
-    return PFGPU_ERR_CUDA;
+  if (nk_handle(h->st, &C.ok) || nk_handle(h->st, &C.restart)) return PFGPU_ERR_CUDA;
   launch_nk_iter(St, C, h->st);
   h->launches++;
   h->jac_valid = 0;
@@ -1410,19 +1414,10 @@ static int nk_newton_iter(pfgpu_handle *h, double dt, NkConds &C) {
   int rc = nk_body(h, C.restart, cudaGraphCondTypeWhile, 2, NKB_CYCLE,
                    [&]() { return nk_gmres_cycle(h, dt, C); });
   if (rc) return rc;
-  launch_nk_after_gmres(St, C, h->st);
+  launch_nk_after_gmres(St, h->zbasis ? 0 : 1, C, h->st);
   h->launches++;
-  rc = nk_body(h, C.post, cudaGraphCondTypeIf, 2, NKB_POST, [&]() {
-    if (h->zbasis) {  // x = Z y is already formed
-      launch_nk_count(St, NKB_POST, 0, h->st);
-    } else {
-      if (pc_apply_dense_impl(h, h->xcor, h->pp)) return (int)PFGPU_ERR_CUDA;
-      launch_nk_count(St, NKB_POST, 1, h->st);
-    }
-    h->launches++;
-    return 0;
-  });
-  if (rc) return rc;
+  // x = M^{-1} V y (with the kept basis x = Z y is already formed)
+  if (!h->zbasis && pc_apply_dense_impl(h, h->xcor, h->pp)) return PFGPU_ERR_CUDA;
   launch_fill_if(h->pp, 0.0, &St->zero_x, N, h->st);
   h->launches++;
   rc = nk_body(h, C.ok, cudaGraphCondTypeIf, 2, NKB_OK,

@@ -360,9 +360,9 @@ void launch_dot(const double *a, const double *b, long long n, double *dst, Redu
                 cudaStream_t st);
 // dst = max |a|
 void launch_maxabs(const double *a, long long n, double *dst, ReduceBuf rb, cudaStream_t st);
-// dst = max |s| / (1 + |u|)
+// dst = max |s| / (1 + |u|) (gate given: only when *gate is nonzero)
 void launch_steplen(const double *s, const double *u, long long n, double *dst, ReduceBuf rb,
-                    cudaStream_t st);
+                    cudaStream_t st, const int *gate = nullptr);
 // dst = max |a - b| / (1 + |a|)
 void launch_steplen_diff(const double *a, const double *b, long long n, double *dst,
                          ReduceBuf rb, cudaStream_t st);
