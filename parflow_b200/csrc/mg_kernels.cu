@@ -1732,7 +1732,7 @@ static cudaError_t mid_prepare(K kern) {
 }
 
 template <typename T, bool H>
-__global__ void k_setup_tail_smem(const MGLevel<T> *__restrict__ Ls, int first, int nl);
+__global__ void k_setup_tail_smem(const MGLevel<T> *__restrict__ Ls, int first, int nl, int cells);
 
 // opt the fused smoother, the shared-memory tails and the cluster kernel into
 // their dynamic shared memory (> 48 KB) and cluster sizes above 8; called once
@@ -2118,13 +2118,15 @@ __global__ void __launch_bounds__(512) k_h16_scale_tail(const MGLevel<float> *__
 // memory as they come.  Bound by the chain of levels: 11 phases instead of
 // the 22 global-memory phases of k_setup_tail and the 11 of k_h16_scale_tail.
 template <typename T, int D, bool H>
-__device__ __forceinline__ void setup_tail_level(const MGLevel<T> &F, const MGLevel<T> &C, T *fs,
-                                                 T *cs) {
+__device__ __forceinline__ void setup_tail_level(const MGLevel<T> &F, const MGLevel<T> &Cg, T *fs,
+                                                 T *cs, T *fw, T *cw) {
+  MGLevel<T> C = Cg;  // with the ghost column in shared memory
+  C.wg = cw;
   const int nf = (int)F.n, nc = (int)C.n;
   LV<T> L;
   L.nx = F.nx; L.ny = F.ny; L.nz = F.nz; L.n = nf;
   L.a0 = fs; L.ae = fs + nf; L.an = fs + 2 * nf; L.au = fs + 3 * nf;
-  L.wg = F.wg;
+  L.wg = fw;
   const FastDiv fx = fast_div(C.nx), fy = fast_div(C.ny);
   for (int t = threadIdx.x; t < nc; t += blockDim.x) {
     int i, j, k;
@@ -2138,11 +2140,12 @@ __device__ __forceinline__ void setup_tail_level(const MGLevel<T> &F, const MGLe
     C.a[1][t] = r.e;
     C.a[2][t] = r.n;
     C.a[3][t] = r.u;
+    if (i == 0) Cg.wg[j + C.ny * k] = cw[j + C.ny * k];
   }
 }
 template <typename T, bool H>
 __global__ void __launch_bounds__(TAIL_THREADS, 1)
-    k_setup_tail_smem(const MGLevel<T> *__restrict__ Ls, int first, int nl) {
+    k_setup_tail_smem(const MGLevel<T> *__restrict__ Ls, int first, int nl, int cells) {
   extern __shared__ __align__(16) unsigned char setup_raw[];
   __shared__ __align__(16) unsigned char tab[TAIL_MAX_LEVELS * sizeof(MGLevel<T>)];
   static_assert(sizeof(MGLevel<T>) % 4 == 0, "copied in words");
@@ -2153,10 +2156,12 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
   __syncthreads();
   pdl_enter();
   const MGLevel<T> *S = reinterpret_cast<const MGLevel<T> *>(tab);
-  T *fs = reinterpret_cast<T *>(setup_raw);
+  T *fs = reinterpret_cast<T *>(setup_raw), *fw = fs + 4 * cells;
   {
     const int n = (int)S[0].n;
-    const T *a0 = S[0].a[0], *a1 = S[0].a[1], *a2 = S[0].a[2], *a3 = S[0].a[3];
+    const T *a0 = S[0].a[0], *a1 = S[0].a[1], *a2 = S[0].a[2], *a3 = S[0].a[3], *w = S[0].wg;
+    const int nw = S[0].ny * S[0].nz;
+    for (int t = threadIdx.x; t < nw; t += blockDim.x) fw[t] = w[t];
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
       const T v0 = a0[t], v1 = a1[t], v2 = a2[t], v3 = a3[t];
       fs[t] = v0;
@@ -2168,15 +2173,16 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
   __syncthreads();
   for (int l = 0; l + 1 < nt; l++) {
     const MGLevel<T> &F = S[l], &C = S[l + 1];
-    T *cs = fs + 4 * (int)F.n;
+    T *cs = fs + 4 * (int)F.n, *cw = fw + F.ny * F.nz;
     if (F.dir == 0)
-      setup_tail_level<T, 0, H>(F, C, fs, cs);
+      setup_tail_level<T, 0, H>(F, C, fs, cs, fw, cw);
     else if (F.dir == 1)
-      setup_tail_level<T, 1, H>(F, C, fs, cs);
+      setup_tail_level<T, 1, H>(F, C, fs, cs, fw, cw);
     else
-      setup_tail_level<T, 2, H>(F, C, fs, cs);
+      setup_tail_level<T, 2, H>(F, C, fs, cs, fw, cw);
     fs = cs;
-    __syncthreads();  // (the coarse ghost column too, written to global memory)
+    fw = cw;
+    __syncthreads();
   }
   if constexpr (H) {
     // the coarsest level's scaling
@@ -2193,28 +2199,33 @@ void launch_h16_scale(const MGLevel<float> &F, const MGLevel<float> *C, cudaStre
   Shape3 g = shape3(F.nx, F.ny, F.nz);
   launch_pdl(k_h16_scale, dim3(g.grid), dim3(g.block), st, F, C ? *C : F, C ? 1 : 0);
 }
-// the operators of all tail levels in shared memory
+// the operators of all tail levels and their ghost columns in shared memory
 template <typename T>
-static size_t setup_tail_bytes(const MGLevel<T> *L, int first, int nl) {
-  long long n = 0;
-  for (int q = first; q < nl; q++) n += L[q].n;
-  return (size_t)(4 * n * (long long)sizeof(T));
+static size_t setup_tail_bytes(const MGLevel<T> *L, int first, int nl, long long *cells) {
+  long long n = 0, w = 0;
+  for (int q = first; q < nl; q++) {
+    n += L[q].n;
+    w += (long long)L[q].ny * L[q].nz;
+  }
+  *cells = n;
+  return (size_t)((4 * n + w) * (long long)sizeof(T));
 }
 template <typename T>
 int launch_setup_tail(const MGLevel<T> *L, const MGLevel<T> *levels_dev, int first, int nl,
                       cudaStream_t st, bool h16) {
-  const size_t smem = setup_tail_bytes(L, first, nl);
+  long long cells = 0;
+  const size_t smem = setup_tail_bytes(L, first, nl, &cells);
   if (nl - first <= TAIL_MAX_LEVELS && smem <= SETUP_TAIL_SMEM_MAX) {
     if constexpr (kHasH16<T>) {
       if (h16) {
         launch_pdl_smem(k_setup_tail_smem<T, true>, dim3(1), dim3(TAIL_THREADS), smem, st,
-                        levels_dev, first, nl);
+                        levels_dev, first, nl, (int)cells);
         return 1;
       }
     }
     if (first + 1 < nl)
       launch_pdl_smem(k_setup_tail_smem<T, false>, dim3(1), dim3(TAIL_THREADS), smem, st,
-                      levels_dev, first, nl);
+                      levels_dev, first, nl, (int)cells);
     return first + 1 < nl ? 1 : 0;
   }
   // tails that do not fit (a hierarchy cut short by MaxLevels)
