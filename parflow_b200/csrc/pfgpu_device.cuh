@@ -97,27 +97,66 @@ __device__ __forceinline__ void tfg_face_y(const DevProblem &P, int i, int j, do
   gc = 0.5 * (__ldg(P.tfg_yc + a) + (in ? __ldg(P.tfg_yc + a + P.nx) : g * 1.0));
 }
 
-// 1/x: the hardware's approximation (rcp.approx.ftz.f64, some 20 bits) and two
-// Newton-Raphson steps y += y (1 - x y), each squaring the relative error;
-// within 2 ulp of the division at a third of its instructions.  Operands near
-// the ends of the exponent range take the division.
-__device__ __forceinline__ double fast_rcp(double x) {
-  // exponent field outside 24 .. 2022: zero, tiny, huge, infinite, NaN
-  if (((unsigned)__double2hiint(x) >> 20 & 0x7ffu) - 24u > 1998u) return 1.0 / x;
+// 1/x: the hardware's approximation (rcp.approx.ftz.f64, some 20 bits) and
+// Newton-Raphson steps y += y (1 - x y), each squaring the relative error; with
+// two within 2 ulp of the division at a third of its instructions.  a/b: one
+// step and one correction of the quotient, q += y (a - b q), whose error is the
+// product of q's and y's (some 2^-80) before it is rounded.  Operands outside
+// 2^-1000 .. 2^500 (rcp_far: zero, tiny, huge, infinite, NaN; also where a
+// product of two of them may overflow) take the division.
+__device__ __forceinline__ bool rcp_far(double x) {
+  return ((unsigned)__double2hiint(x) >> 20 & 0x7ffu) - 24u > 1499u;
+}
+__device__ __forceinline__ double rcp_step(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(fma(-x, y, 1.0), y, y);
   return fma(fma(-x, y, 1.0), y, y);
 }
+__device__ __forceinline__ double fast_rcp(double x) {
+  if (rcp_far(x)) return 1.0 / x;
+  const double y = rcp_step(x);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+// FP32 (the face terms of an FP32 Jacobian): 2^-111 .. 2^62
+__device__ __forceinline__ bool rcp_far(float x) {
+  return ((unsigned)__float_as_int(x) >> 23 & 0xffu) - 16u > 173u;
+}
+__device__ __forceinline__ float rcp_step(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fmaf(fmaf(-x, y, 1.0f), y, y);
+}
+template <typename T>
+__device__ __forceinline__ T quotient_near(T a, T b) {
+  const T y = rcp_step(b), q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
 
-// ParFlow's mean macros (pfsimulator/parflow_lib/solver.h:42-47)
+// ParFlow's mean macros (pfsimulator/parflow_lib/solver.h:42-47);
+// (not inlined: the division's registers cost every cell 1 % of the residual)
+static __device__ __noinline__ double quotient_far(double a, double b) { return b ? a / b : 0.0; }
+// a face's mean permeability in two parts, numerator and denominator, so that
+// several faces can share one test for operands that need the division (a
+// subnormal denominator has no finite reciprocal)
+struct Mean {
+  double num, den;
+  __device__ __forceinline__ double near() const { return quotient_near(num, den); }
+  __device__ __forceinline__ bool far() const { return rcp_far(den); }
+  __device__ __forceinline__ double value() const {
+    return far() ? quotient_far(num, den) : near();
+  }
+};
+__device__ __forceinline__ Mean mean_xy(double a, double b) {  // harmonic
+  return Mean{__dmul_rn(__dmul_rn(2.0, a), b), a + b};
+}
+__device__ __forceinline__ Mean mean_z(double a, double b, double c, double d) {  // harmonic_dz
+  return Mean{__dmul_rn(__dmul_rn(c + d, a), b), fma(b, c, __dmul_rn(a, d))};
+}
 __device__ __forceinline__ double harmonic(double a, double b) {
-  const double den = a + b;
-  return den ? __dmul_rn(__dmul_rn(__dmul_rn(2.0, a), b), fast_rcp(den)) : 0.0;
+  return mean_xy(a, b).value();
 }
 __device__ __forceinline__ double harmonic_dz(double a, double b, double c, double d) {
-  const double den = fma(b, c, __dmul_rn(a, d));
-  return den ? __dmul_rn(__dmul_rn(__dmul_rn(c + d, a), b), fast_rcp(den)) : 0.0;
+  return mean_z(a, b, c, d).value();
 }
 __device__ __forceinline__ double upstream(double a, double b, double c, double d) {
   return ((a - b) >= 0) ? c : d;
@@ -203,9 +242,12 @@ __device__ __forceinline__ double vg_dkr(const DevProblem &P, double p, double a
 // All four van Genuchten quantities of one cell from log(alpha h) and
 // log(1 + (alpha h)^n): every power of the reference formulas
 // (problem_saturation.c:221-415, problem_phase_rel_perm.c:788, :981) comes
-// from two exponentials of these logarithms ((1+A)^(-m/2), squared for
-// (1+A)^-m), a reciprocal of alpha h (for the (alpha h)^(n-1), (alpha h)^(n-2)
-// factors) and one of 1 + (alpha h)^n.  inv_rg = 1 / (density gravity), m = 1 - 1/n.
+// from two exponentials of these logarithms, a square root ((1+A)^(-m/2)), a
+// reciprocal of alpha h (for the (alpha h)^(n-1), (alpha h)^(n-2) factors) and
+// one of 1 + (alpha h)^n.  inv_rg = 1 / (density gravity), m = 1 - 1/n.  Against
+// a residual in extended steps the error is that of log1p and of divisions
+// (2.1e-15 of its norm); a plain log(1 + A), |p| inv_rg and the square of one
+// exponential made it 2.5e-15.
 struct VGAll {
   double kr, dkr, s, ds;
 };
@@ -222,14 +264,17 @@ __device__ __forceinline__ VGAll vg_all(const DevProblem &P, double p, const VG 
     return r;
   }
   const double n = v.n, alpha = v.alpha;
-  const double ah = alpha * (fabs(p) * inv_rg);
+  // |p| / rg, the quotient corrected once (quotient_near)
+  const double rg = P.density * P.gravity, h = fabs(p) * inv_rg;
+  const double ah = alpha * (h < 1e300 ? fma(fma(-rg, h, fabs(p)), inv_rg, h) : h);
   const double ahn = exp(n * log(ah));          // (alpha h)^n
   const double inv_ah = fast_rcp(ah);
   const double ahnm1 = ahn * inv_ah;            // (alpha h)^(n-1)
-  const double op = 1.0 + ahn;
-  const double inv_opm2 = exp(-0.5 * m * log(op));  // op^(-m/2)
-  const double inv_opm = inv_opm2 * inv_opm2;   // op^-m
-  const double inv_op = fast_rcp(op);
+  const double op = 1.0 + ahn, inv_op = fast_rcp(op);
+  // log(1 + ahn): the logarithm of the rounded sum and the rounding's share
+  const double lop = log(op) + (op < 1e300 ? (ahn - (op - 1.0)) * inv_op : 0.0);
+  const double inv_opm = exp(-m * lop);         // op^-m
+  const double inv_opm2 = sqrt(inv_opm);        // op^(-m/2)
   const double t = 1.0 - ahnm1 * inv_opm;
   const double na1 = n * alpha * ahnm1, mq = m * (inv_opm * inv_op) * na1;
   r.kr = (t * t) * inv_opm2;
@@ -267,26 +312,35 @@ __device__ __forceinline__ FluxConst flux_const(const DevProblem &P) {
   const double q = P.density * P.inv_visc;
   return FluxConst{P.dy * P.dz * q, P.dx * P.dz * q, P.dx * P.dy * q};
 }
-// x or y face with its spacing's reciprocal (inv_d) and constant (c)
+// x or y face from its mean permeability, with its spacing's reciprocal
+// (inv_d) and constant (c)
+__device__ __forceinline__ double flux_xy_km(double inv_d, double c, double km, double pa,
+                                             double pb, double kra, double krb, double zm,
+                                             double dir_g, double dir_g_c) {
+  const double drive = fma(__dmul_rn(pa - pb, inv_d), dir_g_c, -dir_g);
+  return __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(c, zm), km), drive),
+                   (drive >= 0.0) ? kra : krb);
+}
 __device__ __forceinline__ double flux_xy(double inv_d, double c, double pa, double pb, double ka,
                                           double kb, double kra, double krb, double zm,
                                           double dir_g, double dir_g_c) {
-  const double drive = fma(__dmul_rn(pa - pb, inv_d), dir_g_c, -dir_g);
-  return __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(c, zm), harmonic(ka, kb)), drive),
-                   (drive >= 0.0) ? kra : krb);
+  return flux_xy_km(inv_d, c, harmonic(ka, kb), pa, pb, kra, krb, zm, dir_g, dir_g_c);
 }
 
 // z face between layer k (a, below) and k+1 (b, above)
-__device__ __forceinline__ double flux_z(const DevProblem &P, double c, double pa, double pb,
-                                         double ka, double kb, double kra, double krb, double za,
-                                         double zb, int k) {
+__device__ __forceinline__ double flux_z_km(const DevProblem &P, double c, double km, double pa,
+                                            double pb, double kra, double krb, int k) {
   const double rg = P.density * P.gravity;
   const double inv_sep = __ldg(P.zface + 3 * k);
   const double lower = fma(pa, inv_sep, -__dmul_rn(__ldg(P.zface + 3 * k + 1), rg));
   const double upper = fma(pb, inv_sep, __dmul_rn(__ldg(P.zface + 3 * k + 2), rg));
   const double drive = lower - upper;
-  return __dmul_rn(__dmul_rn(__dmul_rn(c, harmonic_dz(ka, kb, za, zb)), drive),
-                   (drive >= 0.0) ? kra : krb);
+  return __dmul_rn(__dmul_rn(__dmul_rn(c, km), drive), (drive >= 0.0) ? kra : krb);
+}
+__device__ __forceinline__ double flux_z(const DevProblem &P, double c, double pa, double pb,
+                                         double ka, double kb, double kra, double krb, double za,
+                                         double zb, int k) {
+  return flux_z_km(P, c, harmonic_dz(ka, kb, za, zb), pa, pb, kra, krb, k);
 }
 
 // ---------------------------------------------------------------------------

@@ -26,31 +26,17 @@ __device__ __forceinline__ bool launch_ijk(int nx, int ny, int nz, int &i, int &
 // dS/dp (problem_phase_rel_perm.c:1312-1361, problem_saturation.c:342-412).
 // The residual uses kr and S; the Jacobian at the same iterate reuses all four.
 // STEP: the iterate is formed here, pn = u + lam pp (lam from lam_p when
-// given), and written too, which is free: the pass is bound by instruction
-// issue (exp and log), not by memory.
+// given), and written too.  Bound by the latency of its loads (28 % of the
+// issue slots used) over the chain of exponentials and logarithms that follows.
 // 512x512x50: 136 us (memory floor 79 us) against 192 with the logarithms and
 // powers of the reference one by one, a division per reciprocal and per n.
 // q: 1/(rho g), and m = 1 - 1/n of a uniform n
 struct VGUniform {
   double inv_rg, m;
 };
-template <bool STEP>
-__global__ void __launch_bounds__(256, 5) k_vg_all(DevProblem P, VGUniform q,
-                         const double *__restrict__ p, double *__restrict__ kr,
-                         double *__restrict__ dkr, double *__restrict__ sat,
-                         double *__restrict__ dsat, const double *__restrict__ pp,
-                         const double *lam_p, double lam, double *__restrict__ pn) {
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= P.n) return;
-  const VG vg = vg_at(P, c);  // (fields: older than the kernel before this one)
+__device__ __forceinline__ VGAll vg_cell(const DevProblem &P, const VGUniform &q, const VG &vg,
+                                         double pc) {
   const double m = P.vgn ? 1.0 - fast_rcp(vg.n) : q.m;
-  pdl_enter();
-  double pc = p[c];
-  if (STEP) {
-    const double a = lam_p ? *lam_p : lam;
-    if (a != 0.0) pc = pc + a * pp[c];
-    pn[c] = pc;
-  }
   VGAll v = vg_all(P, pc, vg, q.inv_rg, m);
   if (P.krt) {  // relative permeability from the lookup table
     if (pc >= 0.0) {
@@ -62,6 +48,50 @@ __global__ void __launch_bounds__(256, 5) k_vg_all(DevProblem P, VGUniform q,
       v.dkr = krt_lookup(P, head, 1);
     }
   }
+  return v;
+}
+// VEC: two cells per thread in 16-byte accesses (every pointer 16-byte
+// aligned), for fields of VG_VEC_CELLS and more: the pass waits on memory, and
+// two cells per thread keep more bytes in flight once the grid is many waves
+// deep.  256x256x50: 31.6 us against 33.7; 197x123x37, where half as many
+// threads leave a worse last wave: 10.1 us against 9.3.
+constexpr long long VG_VEC_CELLS = 2000000;
+template <bool STEP, bool VEC>
+__global__ void __launch_bounds__(256, VEC ? 4 : 5) k_vg_all(DevProblem P, VGUniform q,
+                         const double *__restrict__ p, double *__restrict__ kr,
+                         double *__restrict__ dkr, double *__restrict__ sat,
+                         double *__restrict__ dsat, const double *__restrict__ pp,
+                         const double *lam_p, double lam, double *__restrict__ pn) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long c = VEC ? 2 * t : t;
+  if (c >= P.n) return;
+  const VG vg = vg_at(P, c);  // (fields: older than the kernel before this one)
+  pdl_enter();
+  const double a = STEP ? (lam_p ? *lam_p : lam) : 0.0;
+  if (VEC && c + 1 < P.n) {
+    double2 pc = reinterpret_cast<const double2 *>(p)[t];
+    if (STEP) {
+      if (a != 0.0) {
+        const double2 d = reinterpret_cast<const double2 *>(pp)[t];
+        pc.x = fma(a, d.x, pc.x);
+        pc.y = fma(a, d.y, pc.y);
+      }
+      reinterpret_cast<double2 *>(pn)[t] = pc;
+    }
+    const VGAll v = vg_cell(P, q, vg, pc.x),
+                w = vg_cell(P, q, vg_at(P, c + 1), pc.y);
+    reinterpret_cast<double2 *>(kr)[t] = make_double2(v.kr, w.kr);
+    reinterpret_cast<double2 *>(dkr)[t] = make_double2(v.dkr, w.dkr);
+    reinterpret_cast<double2 *>(sat)[t] = make_double2(v.s, w.s);
+    reinterpret_cast<double2 *>(dsat)[t] = make_double2(v.ds, w.ds);
+    return;
+  }
+  double pc = p[c];  // (VEC: the last cell of an odd count)
+  if (STEP) {
+    if (a != 0.0) pc = fma(a, pp[c], pc);
+    pn[c] = pc;
+  }
+  const VGAll v = vg_cell(P, q, vg, pc);
   kr[c] = v.kr;
   dkr[c] = v.dkr;
   sat[c] = v.s;
@@ -136,6 +166,10 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
   }
 
   // boundary patches (nl_function_eval.c:979-1435)
+  if (i > 0 && i < P.nx - 1 && j > 0 && j < P.ny - 1 && k > 0 && k < P.nz - 1) {
+    f[c] = fc;
+    return;
+  }
   const double ffx = P.dy * P.dz, ffy = P.dx * P.dz, ffz = P.dx * P.dy;
   const bool onf[6] = {i == 0, i == P.nx - 1, j == 0, j == P.ny - 1, k == 0, k == P.nz - 1};
 #pragma unroll
@@ -342,8 +376,11 @@ __global__ void __launch_bounds__(256, 5) k_residual(DevProblem P, const double 
 // in a register as the lower one of the next plane: four faces per cell instead
 // of six and half the loads, with no barrier and no shared memory.  Every flux
 // is the same function of the same operands as in the gather form.
-// The gather form is bound by instruction issue and the latency its occupancy
-// leaves; 512x512x50: 232 us against 311 (memory floor 112 us, 56 B per cell).
+// Bound by instruction issue (two thirds of the slots) and the latency its
+// occupancy leaves: the four faces are evaluated without a branch between them
+// and an inner cell meets one test for the boundary patches.  512x512x50: 211
+// us, 230 with a branch per face and per patch, gather form 311 (memory floor
+// 112 us, 56 B per cell).
 // Four blocks of 64 registers per SM; three (five) give 267 (250) us; with the
 // slopes of a terrain-following grid, which need more registers, three give 45
 // us at 256x256x20, four 51, gather 54.  Two rows per warp (3.6 faces per cell,
@@ -377,6 +414,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, SURF ? 3 : 4) k_residual_mar
   const int ii = in ? i : (i < 0 ? 0 : nx - 1), sz = nx * ny;
   const FluxConst A = flux_const(P);
   const VelOut V{};
+  const bool barriers = P.fbx || P.fby || P.fbz;
   // gravity terms of the column's faces (constant through the planes)
   double gse = 0.0, gce = P.gravity, gss = 0.0, gcs = P.gravity, gsn = 0.0, gcn = P.gravity;
   if (SURF) {
@@ -401,24 +439,34 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, SURF ? 3 : 4) k_residual_mar
     const MCell s = mcell(P, p, kr, south ? c - nx : c);
     const MCell t = mcell(P, p, kr, north ? c + nx : c);
     const double sat = satv[c], so = s_old[c], po = p_old[c];
-    double ux = 0.0, us = 0.0, un = 0.0, uz = 0.0;
-    if (east) {
-      ux = flux_xy(P.inv_dx, A.cx, q.p, e.p, q.k, e.k, q.kr, e.kr, zm, gse, gce);
+    // the four faces side by side, without a branch: one that does not exist
+    // is evaluated against the cell itself and dropped
+    const Mean mx = mean_xy(q.k, e.k), ms = mean_xy(s.k, q.k), mn = mean_xy(q.k, t.k),
+               mz = mean_z(q.k, n.k, zm, zu);
+    double kx = mx.near(), ks = ms.near(), kn = mn.near(), kz = mz.near();
+    if (mx.far() | ms.far() | mn.far() | mz.far()) {
+      kx = mx.value();
+      ks = ms.value();
+      kn = mn.value();
+      kz = mz.value();
+    }
+    double ux = flux_xy_km(P.inv_dx, A.cx, kx, q.p, e.p, q.kr, e.kr, zm, gse, gce);
+    double us = flux_xy_km(P.inv_dy, A.cy, ks, s.p, q.p, s.kr, q.kr, zm, gss, gcs);
+    double un = flux_xy_km(P.inv_dy, A.cy, kn, q.p, t.p, q.kr, t.kr, zm, gsn, gcn);
+    double uz = flux_z_km(P, A.cz, kz, q.p, n.p, q.kr, n.kr, k);
+    if (barriers) {
       if (P.fbx) ux = ux * fb_x(P, c);
-    }
-    const double wx = __shfl_up_sync(0xffffffffu, ux, 1);
-    if (south) {
-      us = flux_xy(P.inv_dy, A.cy, s.p, q.p, s.k, q.k, s.kr, q.kr, zm, gss, gcs);
-      if (P.fby) us = us * fb_y(P, c - nx);
-    }
-    if (north) {
-      un = flux_xy(P.inv_dy, A.cy, q.p, t.p, q.k, t.k, q.kr, t.kr, zm, gsn, gcn);
-      if (P.fby) un = un * fb_y(P, c);
-    }
-    if (up) {
-      uz = flux_z(P, A.cz, q.p, n.p, q.k, n.k, q.kr, n.kr, zm, zu, k);
+      if (P.fby) {
+        if (south) us = us * fb_y(P, c - nx);
+        un = un * fb_y(P, c);
+      }
       if (P.fbz) uz = uz * fb_z(P, c);
     }
+    ux = east ? ux : 0.0;
+    us = south ? us : 0.0;
+    un = north ? un : 0.0;
+    uz = up ? uz : 0.0;
+    const double wx = __shfl_up_sync(0xffffffffu, ux, 1);
     if (out)
       residual_cell<SURF, false>(P, i, j, k, c, p, p_old, dt, f, V, q.p, q.kr, sat, so, po, zm, lz,
                                  us, i > 0 ? wx : 0.0, ux, un, uz);
@@ -439,16 +487,33 @@ struct FaceDer {
   TA lo, hi, sym;  // d/dp of the face flux w.r.t. lower cell (negated), upper cell; sym part
 };
 
-__device__ __forceinline__ float quotient(float a, float b) { return a / b; }
-__device__ __forceinline__ double quotient(double a, double b) { return a * fast_rcp(b); }
+__device__ __forceinline__ float mul_rn_t(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn_t(double a, double b) { return __dmul_rn(a, b); }
+// Mean in the face arithmetic
+template <typename TA>
+struct MeanT {
+  TA num, den;
+  __device__ __forceinline__ TA near() const { return quotient_near(num, den); }
+  __device__ __forceinline__ bool far() const { return rcp_far(den); }
+  __device__ __forceinline__ TA value() const {
+    return far() ? (den ? num / den : TA(0)) : near();
+  }
+};
+template <typename TA>
+__device__ __forceinline__ MeanT<TA> mean_xy_t(TA a, TA b) {
+  return MeanT<TA>{mul_rn_t(mul_rn_t(TA(2), a), b), a + b};
+}
+template <typename TA>
+__device__ __forceinline__ MeanT<TA> mean_z_t(TA a, TA b, TA c, TA d) {
+  return MeanT<TA>{mul_rn_t(mul_rn_t(c + d, a), b), fma(b, c, mul_rn_t(a, d))};
+}
 template <typename TA>
 __device__ __forceinline__ TA harmonic_t(TA a, TA b) {
-  return (a + b) ? quotient(TA(2) * a * b, a + b) : TA(0);
+  return mean_xy_t(a, b).value();
 }
 template <typename TA>
 __device__ __forceinline__ TA harmonic_dz_t(TA a, TA b, TA c, TA d) {
-  const TA den = (b * c) + (a * d);
-  return den ? quotient((c + d) * a * b, den) : TA(0);
+  return mean_z_t(a, b, c, d).value();
 }
 
 // What a face term needs of a cell: the pressure in FP64 (its differences take
@@ -477,42 +542,42 @@ struct JFace {
 // x_coeff / y_coeff (richards_jacobian_eval.c:662, 692): FB * dt * ...; the
 // upwinded terms of the reference's macros with their common factors formed once
 template <typename TA>
-__device__ __forceinline__ FaceDer<TA> face_der_xy(const JFace<TA> &F, double fb,
+__device__ __forceinline__ FaceDer<TA> face_der_xy(const JFace<TA> &F, double fb, TA km,
                                                    const JCell<TA> &a, const JCell<TA> &b,
                                                    TA zm, double dir_g, double dir_g_c) {
   const double diff64 = a.p - b.p;
   const bool lower = ((diff64 * F.inv_d) * dir_g_c - dir_g) >= 0.0;  // flow from a to b
   const TA diff = (TA)diff64, dgc = (TA)dir_g_c, dg = (TA)dir_g;
-  const TA coeff = (TA)fb * F.c * zm * harmonic_t<TA>(a.k, b.k);
+  const TA coeff = mul_rn_t(mul_rn_t(mul_rn_t((TA)fb, F.c), zm), km);
   // derivative of the upwind cell's mobility times the driving difference
-  const TA drive = coeff * (diff * dgc - F.d * dg);
-  const TA sym = (-coeff * (lower ? a.prod : b.prod)) * dgc;
+  const TA drive = mul_rn_t(coeff, fma(diff, dgc, -mul_rn_t(F.d, dg)));
+  const TA sym = mul_rn_t(mul_rn_t(-coeff, lower ? a.prod : b.prod), dgc);
   FaceDer<TA> r;
   r.sym = sym;
-  r.lo = lower ? sym - drive * a.prod_der : sym;
-  r.hi = lower ? sym : sym + drive * b.prod_der;
+  r.lo = lower ? fma(-drive, a.prod_der, sym) : sym;
+  r.hi = lower ? sym : fma(drive, b.prod_der, sym);
   return r;
 }
 
 // z face between a (lower) and b (upper) (richards_jacobian_eval.c:697-745);
 // the terms with the density's derivative are zero (constant density)
 template <typename TA>
-__device__ __forceinline__ FaceDer<TA> face_der_z(const DevProblem &P, TA cz, double fb,
+__device__ __forceinline__ FaceDer<TA> face_der_z(const DevProblem &P, TA cz, double fb, TA km,
                                                   const JCell<TA> &a, const JCell<TA> &b,
-                                                  double za, double zb, int k) {
+                                                  int k) {
   const double rg = P.density * P.gravity;
   const double inv_sep = __ldg(P.zface + 3 * k);
-  const double lower_cond = a.p * inv_sep - __ldg(P.zface + 3 * k + 1) * rg;
-  const double upper_cond = b.p * inv_sep + __ldg(P.zface + 3 * k + 2) * rg;
+  const double lower_cond = fma(a.p, inv_sep, -__dmul_rn(__ldg(P.zface + 3 * k + 1), rg));
+  const double upper_cond = fma(b.p, inv_sep, __dmul_rn(__ldg(P.zface + 3 * k + 2), rg));
   const double diff64 = lower_cond - upper_cond;
   const bool lower = diff64 >= 0.0;
-  const TA coeff = (TA)fb * cz * harmonic_dz_t<TA>(a.k, b.k, (TA)za, (TA)zb);
-  const TA drive = coeff * (TA)diff64;
-  const TA sym = -coeff * (TA)inv_sep * (lower ? a.prod : b.prod);
+  const TA coeff = mul_rn_t(mul_rn_t((TA)fb, cz), km);
+  const TA drive = mul_rn_t(coeff, (TA)diff64);
+  const TA sym = mul_rn_t(mul_rn_t(-coeff, (TA)inv_sep), lower ? a.prod : b.prod);
   FaceDer<TA> r;
   r.sym = sym;
-  r.lo = lower ? sym - drive * a.prod_der : sym;
-  r.hi = lower ? sym : sym + drive * b.prod_der;
+  r.lo = lower ? fma(-drive, a.prod_der, sym) : sym;
+  r.hi = lower ? sym : fma(drive, b.prod_der, sym);
   return r;
 }
 
@@ -587,6 +652,7 @@ __device__ __forceinline__ void jacobian_cell(const DevProblem &P, int i, int j,
   // Dirichlet patches (richards_jacobian_eval.c:1049-1200); flux patches
   // leave the row as is (their boundary entries are zero)
   const bool onf[6] = {i == 0, i == P.nx - 1, j == 0, j == P.ny - 1, k == 0, k == P.nz - 1};
+  if (onf[0] || onf[1] || onf[2] || onf[3] || onf[4] || onf[5])
 #pragma unroll
   for (int face = 0; face < 6; face++) {
     if (!onf[face] || P.bc_type[face] != 1) continue;
@@ -828,39 +894,44 @@ __global__ void __launch_bounds__(128, 8) k_jacobian(DevProblem P, const double 
   FaceLH<TA> dl_z{}, dl_y{}, dl_x{};
   FaceDer<TA> de{}, dn{}, du{};
   if (k > 0) {
+    const JCell<TA> o = jcell<TA>(p, P.kz, kr, dkr, rho, c - sz);
+    const double zl = __ldg(P.zmult + k - 1);
     const FaceDer<TA> d = face_der_z<TA>(P, A.cz, fb_z(P, c - sz),
-                                         jcell<TA>(p, P.kz, kr, dkr, rho, c - sz), qz,
-                                         __ldg(P.zmult + k - 1), zm, k - 1);
+                                         harmonic_dz_t<TA>(o.k, qz.k, (TA)zl, (TA)zm), o, qz,
+                                         k - 1);
     dl_z = {d.lo, d.hi};
   }
   double gs = 0.0, gc = g;
   if (j > 0) {
     if (SURF) tfg_face_y(P, i, j - 1, gs, gc);
-    const FaceDer<TA> d = face_der_xy<TA>(A.y, fb_y(P, c - sy),
-                                          jcell<TA>(p, P.ky, kr, dkr, rho, c - sy), qy, (TA)zm, gs,
-                                          gc);
+    const JCell<TA> o = jcell<TA>(p, P.ky, kr, dkr, rho, c - sy);
+    const FaceDer<TA> d = face_der_xy<TA>(A.y, fb_y(P, c - sy), harmonic_t<TA>(o.k, qy.k), o, qy,
+                                          (TA)zm, gs, gc);
     dl_y = {d.lo, d.hi};
   }
   if (i > 0) {
     if (SURF) tfg_face_x(P, i - 1, j, gs, gc);
-    const FaceDer<TA> d = face_der_xy<TA>(A.x, fb_x(P, c - 1),
-                                          jcell<TA>(p, P.kx, kr, dkr, rho, c - 1), q, (TA)zm, gs,
-                                          gc);
+    const JCell<TA> o = jcell<TA>(p, P.kx, kr, dkr, rho, c - 1);
+    const FaceDer<TA> d = face_der_xy<TA>(A.x, fb_x(P, c - 1), harmonic_t<TA>(o.k, q.k), o, q,
+                                          (TA)zm, gs, gc);
     dl_x = {d.lo, d.hi};
   }
   if (i + 1 < P.nx) {
     if (SURF) tfg_face_x(P, i, j, gs, gc);
-    de = face_der_xy<TA>(A.x, fb_x(P, c), q, jcell<TA>(p, P.kx, kr, dkr, rho, c + 1), (TA)zm, gs,
-                         gc);
+    const JCell<TA> o = jcell<TA>(p, P.kx, kr, dkr, rho, c + 1);
+    de = face_der_xy<TA>(A.x, fb_x(P, c), harmonic_t<TA>(q.k, o.k), q, o, (TA)zm, gs, gc);
   }
   if (j + 1 < P.ny) {
     if (SURF) tfg_face_y(P, i, j, gs, gc);
-    dn = face_der_xy<TA>(A.y, fb_y(P, c), qy, jcell<TA>(p, P.ky, kr, dkr, rho, c + sy), (TA)zm,
-                         gs, gc);
+    const JCell<TA> o = jcell<TA>(p, P.ky, kr, dkr, rho, c + sy);
+    dn = face_der_xy<TA>(A.y, fb_y(P, c), harmonic_t<TA>(qy.k, o.k), qy, o, (TA)zm, gs, gc);
   }
-  if (k + 1 < P.nz)
-    du = face_der_z<TA>(P, A.cz, fb_z(P, c), qz, jcell<TA>(p, P.kz, kr, dkr, rho, c + sz), zm,
-                        __ldg(P.zmult + k + 1), k);
+  if (k + 1 < P.nz) {
+    const JCell<TA> o = jcell<TA>(p, P.kz, kr, dkr, rho, c + sz);
+    const double zu = __ldg(P.zmult + k + 1);
+    du = face_der_z<TA>(P, A.cz, fb_z(P, c), harmonic_dz_t<TA>(qz.k, o.k, (TA)zm, (TA)zu), qz, o,
+                        k);
+  }
   jacobian_cell<TJ, TP, SURF>(P, i, j, k, c, p, kr, dkr, dt, J, M, q.p, satv[c], dsatv[c], zm,
                               dl_z, dl_y, dl_x, de, dn, du);
 }
@@ -869,10 +940,12 @@ __global__ void __launch_bounds__(128, 8) k_jacobian(DevProblem P, const double 
 // the next column by shuffles and to the next plane in registers.
 // The gather form converts every operand of every face to the face arithmetic
 // (103 conversions and reciprocals per cell on a pipe of 16 lanes), this one a
-// cell's values once per thread that needs them.  512x512x50, FP32: 347 us
-// against 449; FP64: 503 against 516.
+// cell's values once per thread that needs them, and evaluates the four faces
+// without a branch between them.  512x512x50, FP32: 293 us against 449 (343
+// with the branches).  Blocks per SM, FP64 512x512x50 with the van Genuchten pass:
+// three (80 registers) 559 us, two (128) 588; 197x123x37 48.0 and 47.1.
 template <typename TJ, typename TP, bool SURF>
-__global__ void __launch_bounds__(32 * MARCH_WARPS, sizeof(TJ) == 8 ? 2 : SURF ? 3 : 4)
+__global__ void __launch_bounds__(32 * MARCH_WARPS, sizeof(TJ) == 8 || SURF ? 3 : 4)
     k_jacobian_march(
     DevProblem P, const double *__restrict__ p, const double *__restrict__ kr,
     const double *__restrict__ dkr, const double *__restrict__ satv,
@@ -897,13 +970,16 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, sizeof(TJ) == 8 ? 2 : SURF ?
     if (north) tfg_face_y(P, ii, j, gsn, gcn);
   }
   int c = ii + nx * (j + ny * k0);
+  const bool barriers = P.fbx || P.fby || P.fbz;
   auto cell = [&](int q) { return jcell<TA>(p, P.kx, kr, dkr, rho, q); };
   JCell<TA> q = cell(c);
   FaceLH<TA> lz = {};
   double zm = __ldg(P.zmult + k0);
   if (k0 > 0) {
-    const FaceDer<TA> d = face_der_z<TA>(P, A.cz, fb_z(P, c - sz), cell(c - sz), q,
-                                         __ldg(P.zmult + k0 - 1), zm, k0 - 1);
+    const JCell<TA> o = cell(c - sz);
+    const double zl = __ldg(P.zmult + k0 - 1);
+    const FaceDer<TA> d = face_der_z<TA>(P, A.cz, fb_z(P, c - sz),
+                                         harmonic_dz_t<TA>(o.k, q.k, (TA)zl, (TA)zm), o, q, k0 - 1);
     lz = {d.lo, d.hi};
   }
   for (int k = k0; k < k1; k++, c += sz) {
@@ -912,17 +988,34 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, sizeof(TJ) == 8 ? 2 : SURF ?
     const JCell<TA> n = cell(up ? c + sz : c), e = cell(east ? c + 1 : c);
     const JCell<TA> s = cell(south ? c - nx : c), t = cell(north ? c + nx : c);
     const double sat = satv[c], dsat = dsatv[c];
-    FaceDer<TA> dx = {}, dn = {}, dz = {};
-    FaceLH<TA> wx, dsl = {};
-    if (east) dx = face_der_xy<TA>(A.x, fb_x(P, c), q, e, (TA)zm, gse, gce);
+    // the four faces side by side (as in k_residual_march)
+    const MeanT<TA> mx = mean_xy_t<TA>(q.k, e.k), ms = mean_xy_t<TA>(s.k, q.k),
+                    mn = mean_xy_t<TA>(q.k, t.k), mz = mean_z_t<TA>(q.k, n.k, (TA)zm, (TA)zu);
+    TA kx = mx.near(), ks = ms.near(), kn = mn.near(), kz = mz.near();
+    if (mx.far() | ms.far() | mn.far() | mz.far()) {
+      kx = mx.value();
+      ks = ms.value();
+      kn = mn.value();
+      kz = mz.value();
+    }
+    double bx = 1.0, bs = 1.0, bn = 1.0, bz = 1.0;
+    if (barriers) {
+      bx = fb_x(P, c);
+      if (south) bs = fb_y(P, c - nx);
+      bn = fb_y(P, c);
+      bz = fb_z(P, c);
+    }
+    FaceDer<TA> dx = face_der_xy<TA>(A.x, bx, kx, q, e, (TA)zm, gse, gce);
+    const FaceDer<TA> ds = face_der_xy<TA>(A.y, bs, ks, s, q, (TA)zm, gss, gcs);
+    FaceDer<TA> dn = face_der_xy<TA>(A.y, bn, kn, q, t, (TA)zm, gsn, gcn);
+    FaceDer<TA> dz = face_der_z<TA>(P, A.cz, bz, kz, q, n, k);
+    if (!east) dx = FaceDer<TA>{};
+    if (!north) dn = FaceDer<TA>{};
+    if (!up) dz = FaceDer<TA>{};
+    const FaceLH<TA> dsl = south ? FaceLH<TA>{ds.lo, ds.hi} : FaceLH<TA>{};
+    FaceLH<TA> wx;
     wx.lo = __shfl_up_sync(0xffffffffu, dx.lo, 1);
     wx.hi = __shfl_up_sync(0xffffffffu, dx.hi, 1);
-    if (south) {
-      const FaceDer<TA> d = face_der_xy<TA>(A.y, fb_y(P, c - nx), s, q, (TA)zm, gss, gcs);
-      dsl = {d.lo, d.hi};
-    }
-    if (north) dn = face_der_xy<TA>(A.y, fb_y(P, c), q, t, (TA)zm, gsn, gcn);
-    if (up) dz = face_der_z<TA>(P, A.cz, fb_z(P, c), q, n, zm, zu, k);
     if (out)
       jacobian_cell<TJ, TP, SURF>(P, i, j, k, c, p, kr, dkr, dt, J, M, q.p, sat, dsat, zm, lz, dsl,
                                   wx, dx, dn, dz);
@@ -981,16 +1074,27 @@ static inline void shape_tuned(int nx, int ny, int nz, int threads, const int ti
 static VGUniform vg_uniform(const DevProblem &P) {
   return VGUniform{1.0 / (P.density * P.gravity), 1.0 - 1.0 / P.vgn0};
 }
+template <bool STEP>
+static void vg_launch(const DevProblem &P, const double *p, double *kr, double *dkr, double *sat,
+                      double *dsat, const double *pp, const double *lam_p, double lam, double *pn,
+                      cudaStream_t st) {
+  const uintptr_t at = (uintptr_t)p | (uintptr_t)kr | (uintptr_t)dkr | (uintptr_t)sat |
+                       (uintptr_t)dsat | (uintptr_t)pp | (uintptr_t)pn;
+  if (P.n >= VG_VEC_CELLS && (at & 15) == 0)
+    launch_pdl(k_vg_all<STEP, true>, dim3(blocks_for((P.n + 1) / 2, 256)), dim3(256), st, P,
+               vg_uniform(P), p, kr, dkr, sat, dsat, pp, lam_p, lam, pn);
+  else
+    launch_pdl(k_vg_all<STEP, false>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P),
+               p, kr, dkr, sat, dsat, pp, lam_p, lam, pn);
+}
 void launch_vg_all(const DevProblem &P, const double *p, double *kr, double *dkr, double *sat,
                    double *dsat, cudaStream_t st) {
-  launch_pdl(k_vg_all<false>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), p, kr,
-             dkr, sat, dsat, nullptr, nullptr, 0.0, nullptr);
+  vg_launch<false>(P, p, kr, dkr, sat, dsat, nullptr, nullptr, 0.0, nullptr, st);
 }
 void launch_vg_step(const DevProblem &P, const double *u, const double *pp, const double *lam_p,
                     double lam, double *unew, double *kr, double *dkr, double *sat, double *dsat,
                     cudaStream_t st) {
-  launch_pdl(k_vg_all<true>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), u, kr,
-             dkr, sat, dsat, pp, lam_p, lam, unew);
+  vg_launch<true>(P, u, kr, dkr, sat, dsat, pp, lam_p, lam, unew, st);
 }
 
 void launch_saturation(const DevProblem &P, const double *p, double *s, cudaStream_t st) {
@@ -1000,9 +1104,10 @@ void launch_saturation(const DevProblem &P, const double *p, double *s, cudaStre
 // March or gather: the march form reads one permeability field and has a
 // warp per 31 columns and chunk of planes, so it needs a grid that fills the
 // GPU several times over.  Residual with its VG pass, march against gather:
-// 350k cells 20 us against 14, 900k 27 against 34, 3.3M 97 against 111, 13.1M
-// 357 against 430.  PFGPU_RESIDUAL_FACE_ONCE=1 / 0 forces march / gather
-// (bitwise the same results).
+// 350k cells 18.6 us against 13.6, 512k 22.5 against 16.9, 900k 27.5 against 32,
+// 3.3M 87 against 101; Jacobian in FP32 at 512k 30 against 22, 900k 32.5
+// against 43.5.  PFGPU_RESIDUAL_FACE_ONCE=1 / 0 forces march / gather (bitwise
+// the same results).
 static int face_once_env() {
   static const int v = [] {
     const char *e = getenv("PFGPU_RESIDUAL_FACE_ONCE");

@@ -1,7 +1,7 @@
 """The march form of the residual and the Jacobian (a warp walks 31 columns of a
 row up through a chunk of planes) equals the gather form bit for bit on grids
 around its strip width and chunk length, flat and with slopes, barriers and
-several permeability fields (which only the gather form takes).  The form is
+permeabilities whose face means need the division (zero, subnormal, tiny).  The form is
 chosen once per process (PFGPU_RESIDUAL_FACE_ONCE), so each runs in a child."""
 
 import json
@@ -24,7 +24,7 @@ from parflow_b200.solver import RichardsGPU
 out = {}
 for nx, ny, nz in ((1, 1, 2), (2, 1, 1), (30, 1, 3), (31, 2, 1), (32, 3, 8), (33, 8, 9),
                    (62, 9, 17), (63, 5, 16), (94, 2, 25)):
-    for kind in ("box", "overland", "barrier"):
+    for kind in ("box", "overland", "barrier", "tight"):
         if kind == "overland" and nx * ny == 1:
             continue  # (no slope field of one column)
         if kind == "overland":
@@ -34,6 +34,8 @@ for nx, ny, nz in ((1, 1, 2), (2, 1, 1), (30, 1, 3), (31, 2, 1), (32, 3, 8), (33
         rng = np.random.default_rng(nx + 100 * ny + 10000 * nz)
         if kind == "barrier":
             prob.fbx, prob.fby, prob.fbz = (rng.uniform(0.05, 1.0, prob.shape) for _ in range(3))
+        if kind == "tight":
+            prob.perm = rng.choice([0.0, 5e-324, 1e-310, 1e-300, 1e-37, 1.0], size=prob.shape)
         p_old = prob.initial_pressure()
         p = p_old + 0.1 * rng.standard_normal(p_old.shape)
         x = rng.standard_normal(p.shape)
@@ -63,4 +65,33 @@ def test_march_equals_gather(tmp_path):
         pytest.fail("CUDA device required for gpu tests")
     march, gather = _run(tmp_path, "1"), _run(tmp_path, "0")
     assert march == gather
-    assert len(march) == (9 * 3 - 1) * 2
+    assert len(march) == (9 * 4 - 1) * 2
+
+
+@pytest.mark.parametrize("bottom", (False, True))
+def test_paired_van_genuchten(bottom):
+    """Grids of 2 million cells and more take the van Genuchten pass two cells
+    per thread: its residual equals, bit for bit, that of a smaller grid with
+    the same planes, at either end of an odd number of cells."""
+    import numpy as np
+
+    from parflow_b200 import configs
+    from parflow_b200.solver import RichardsGPU
+
+    nx, ny, nz, part = 127, 129, 123, 61
+    rng = np.random.default_rng(7)
+    p_old = -0.5 + 0.6 * rng.standard_normal((nz, ny, nx))
+    p = p_old + 0.1 * rng.standard_normal(p_old.shape)
+    perm = rng.uniform(0.01, 1.0, p.shape)
+    f = []
+    for planes in (slice(0, nz), slice(0, part) if bottom else slice(nz - part, nz)):
+        n = planes.stop - planes.start
+        prob = configs.box(nx=nx, ny=ny, nz=n, nsteps=1)
+        prob.perm = perm[planes]
+        g = RichardsGPU(prob, precision="fp64")
+        f.append(g.nl_function_eval(p[planes], p_old[planes], g.saturation(p_old[planes]), prob.dt))
+        g.close()
+    assert nx * ny * nz > 2000000 > nx * ny * part and nx * ny * nz % 2 == 1
+    # (the cut plane has another neighbour or a boundary)
+    same = slice(0, part - 1) if bottom else slice(nz - part + 1, nz)
+    np.testing.assert_array_equal(f[0][same], f[1][:-1] if bottom else f[1][1:])
