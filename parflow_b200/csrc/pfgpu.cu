@@ -1738,22 +1738,19 @@ static bool mg_pairs_smoother(const pfgpu_handle *h) {
          env_ll("PFGPU_PAIR_RESIDUAL", 1) != 0;
 }
 
-// how the levels mg.tail .. run: the pair kernel, or the generic tail in
-// shared or global memory
+// the generic tail of the levels mg.tail ..: in shared or global memory
 template <typename T>
-static int tail_form(const pfgpu_handle *h, MG<T> &mg) {
-  const int nl = (int)mg.L.size();
-  const size_t b = tail_smem_bytes<T>(mg.L.data(), mg.tail, nl, mg.h16);
-  const bool smem = env_ll("PFGPU_TAIL_SMEM", 1) != 0;
-  mg.tail_smem = b <= TAIL_SMEM_MAX && smem ? b : 0;
-  cudaFree(mg.tail_image);
-  mg.tail_image = nullptr;
-  if (smem && mg_pairs_smoother(h)) {
-    const size_t img = tail_image_bytes<T>(mg.L.data(), mg.tail, nl, mg.h16);
-    if (img > 0 && dalloc((unsigned char **)&mg.tail_image, (long long)img))
-      return PFGPU_ERR_NOMEM;
-  }
-  return 0;
+static void tail_form(MG<T> &mg) {
+  const size_t b = tail_smem_bytes<T>(mg.L.data(), mg.tail, (int)mg.L.size(), mg.h16);
+  mg.tail_smem = b <= TAIL_SMEM_MAX && env_ll("PFGPU_TAIL_SMEM", 1) != 0 ? b : 0;
+}
+// ... and the pair kernel's packed operators, where that kernel runs them.
+// Allocated once per handle: a tail that loses its first level needs less.
+template <typename T>
+static int tail_image_alloc(const pfgpu_handle *h, MG<T> &mg) {
+  if (env_ll("PFGPU_TAIL_SMEM", 1) == 0 || !mg_pairs_smoother(h)) return 0;
+  const size_t img = tail_image_bytes<T>(mg.L.data(), mg.tail, (int)mg.L.size(), mg.h16);
+  return img > 0 ? dalloc((unsigned char **)&mg.tail_image, (long long)img) : 0;
 }
 
 template <typename T>
@@ -1834,7 +1831,8 @@ static int alloc_mg(pfgpu_handle *h, MG<T> &mg) {
       mg.tail = l;
       break;
     }
-  if (tail_form<T>(h, mg)) return PFGPU_ERR_NOMEM;
+  tail_form<T>(mg);
+  if (tail_image_alloc<T>(h, mg)) return PFGPU_ERR_NOMEM;
   mg.fuse_cells = env_ll("PFGPU_FUSE_CELLS", 400000);
   mg.flip = env_ll("PFGPU_FLIP", 1) != 0;
   // middle levels: the grid levels at or below PFGPU_MID_CELLS cells just
@@ -1941,11 +1939,13 @@ static int mg_level0_on_grid(pfgpu_handle *h, MG<T> &mg) {
   MGLevel<T> &L0 = mg.L[0];
   if (nl > 1) {
     if (mg.tail < 1) {
-      // captured solves hold the old tail and its image
+      // captured solves hold the old tail
       solve_graphs_forget(h);
       mg.tail = 1;
-      if (tail_form<T>(h, mg)) return PFGPU_ERR_NOMEM;
-      // the operators of an earlier setup, for a V-cycle before the next one
+      tail_form<T>(mg);
+      // the image with one level less, packed from the operators of an earlier
+      // setup for a V-cycle before the next one.  Nothing is freed or allocated
+      // here: whatever fails after this, no graph holds a pointer that is gone.
       if (mg.tail_image)
         launch_tail_pack<T>(mg.L.data(), mg.tail, nl, h->d.mg_smoother, mg.tail_image, h->st,
                             mg.h16);
