@@ -7,6 +7,7 @@
 // face once.  Neither needs atomics.  Per-cell relative permeabilities are produced by a first pass
 // (k_vg_all) so that each cell's van Genuchten state is evaluated once per
 // iterate and shared by the residual and the Jacobian.
+#include "march_rule.h"
 #include "pfgpu_device.cuh"
 #include "pdl.cuh"
 #include "pfgpu_kernels.h"
@@ -385,9 +386,6 @@ __global__ void __launch_bounds__(256, 5) k_residual(DevProblem P, const double 
 // slopes of a terrain-following grid, which need more registers, three give 45
 // us at 256x256x20, four 51, gather 54.  Two rows per warp (3.6 faces per cell,
 // 96 registers) were slower than gather: 20 warps per SM hide too little.
-constexpr int MARCH_WARPS = 8, MARCH_COLS = 31;
-constexpr long long MARCH_MIN_CELLS = 600000;
-
 // a column's value of one plane
 struct MCell {
   double p, k, kr;
@@ -1052,9 +1050,7 @@ static inline unsigned blocks_for(long long n, int bs) { return (unsigned)((n + 
 
 // 3-D launch covering (nx, ny, nz) with `threads` threads per block
 static inline void shape(int nx, int ny, int nz, int threads, dim3 &grid, dim3 &block) {
-  int bx = 32;
-  while (bx < nx && bx < 128) bx *= 2;
-  if (bx > threads) bx = threads;
+  const int bx = gather_columns(nx, threads);
   int by = threads / bx;
   if (by > ny) by = ny;
   block = dim3(bx, by, 1);
@@ -1101,34 +1097,17 @@ void launch_saturation(const DevProblem &P, const double *p, double *s, cudaStre
   launch_pdl(k_saturation, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), p, s);
 }
 
-// March or gather: the march form reads one permeability field and has a
-// warp per 31 columns and chunk of planes, so it needs a grid that fills the
-// GPU several times over.  Residual with its VG pass, march against gather:
-// 350k cells 18.6 us against 13.6, 512k 22.5 against 16.9, 900k 27.5 against 32,
-// 3.3M 87 against 101; Jacobian in FP32 at 512k 30 against 22, 900k 32.5
-// against 43.5.  PFGPU_RESIDUAL_FACE_ONCE=1 / 0 forces march / gather (bitwise
-// the same results).
-static int face_once_env() {
-  static const int v = [] {
+// March (planes per chunk) or gather (0): the march form reads one permeability
+// field; march_pays knows the rest.  PFGPU_RESIDUAL_FACE_ONCE=1 / 0 forces
+// march / gather (bitwise the same results).
+static int march_chunk(const DevProblem &P, MarchKernel kernel, bool slopes) {
+  static const int forced = [] {
     const char *e = getenv("PFGPU_RESIDUAL_FACE_ONCE");
     return e && *e ? (*e == '1' ? 1 : 0) : -1;
   }();
-  return v;
-}
-// planes per chunk of the march form, 0: gather
-static int march_chunk(const DevProblem &P) {
-  const int env = face_once_env();
-  if (env == 0 || P.ky != P.kx || P.kz != P.kx) return 0;
-  const long long strips = (long long)((P.nx + MARCH_COLS - 1) / MARCH_COLS) *
-                           P.ny;
-  // chunks of at least eight planes (one more z face per chunk), four waves
-  // of 32 warps per SM where the planes allow it
-  const long long want = 4LL * 32 * 148;
-  long long chunks = (want + strips - 1) / strips;
-  const long long most = (P.nz + 7) / 8;
-  if (chunks > most) chunks = most;
-  if (env < 0 && P.n < MARCH_MIN_CELLS) return 0;
-  return (int)((P.nz + chunks - 1) / chunks);
+  if (forced == 0 || P.ky != P.kx || P.kz != P.kx) return 0;
+  if (forced < 0 && !march_pays(kernel, slopes, P.nx, P.ny, P.nz)) return 0;
+  return march_planes(P.nx, P.ny, P.nz);
 }
 static dim3 march_grid(const DevProblem &P, int kchunk) {
   return dim3((P.nx + MARCH_COLS - 1) / MARCH_COLS,
@@ -1141,7 +1120,7 @@ static void launch_residual_t(const DevProblem &P, const double *p, const double
                               const double *s_old, const double *kr, const double *sat,
                               double dt, double *f, cudaStream_t st, const VelOut &vel) {
   if constexpr (!VEL) {
-    if (const int kchunk = march_chunk(P)) {
+    if (const int kchunk = march_chunk(P, MARCH_RESIDUAL, SURF)) {
       launch_pdl(k_residual_march<SURF>, march_grid(P, kchunk), dim3(32, MARCH_WARPS), st, P, p,
                  p_old, s_old, kr, sat, dt, f, kchunk);
       return;
@@ -1174,9 +1153,9 @@ void launch_jacobian(const DevProblem &P, const double *p, const double *kr,
                      const double *dkr, const double *sat, const double *dsat, double dt,
                      JacOut<TJ> J, PCOut<TP> M, cudaStream_t st) {
   const bool surf = P.tfg_xs || P.bc_type[5] == 2 || P.bc_type[5] == 3 || P.bc_type[5] == 4;
-  const int kchunk = march_chunk(P);
-  if (kchunk && !(surf && sizeof(TJ) == 8 && face_once_env() < 0)) {
-    // (FP64 with slopes: gather, 71 us against 75 at 256x256x20)
+  const int kchunk =
+      march_chunk(P, sizeof(TJ) == 8 ? MARCH_JACOBIAN_F64 : MARCH_JACOBIAN_F32, surf);
+  if (kchunk) {
     if (surf)
       launch_pdl(k_jacobian_march<TJ, TP, true>, march_grid(P, kchunk), dim3(32, MARCH_WARPS), st,
                  P, p, kr, dkr, sat, dsat, dt, J, M, kchunk);
