@@ -6,6 +6,7 @@
 // The scalar GMRES steps (modified Gram-Schmidt bookkeeping, Givens QR,
 // back substitution) run in one thread on device-resident scalars and follow
 // pfsimulator/kinsol/iterativ.c:30-286 and spgmr.c:168-450.
+#include "gpu_wait.cuh"
 #include "pdl.cuh"
 #include "pfgpu_kernels.h"
 #include "nk_control.h"
@@ -795,51 +796,143 @@ __device__ __forceinline__ double reorth_norm(double hk, double nn2) {
   return (np2 > 0.0) ? sqrt(np2) : 0.0;
 }
 
-// End of GMRES iteration l in one launch, the projections and their dot
-// products done.  One block: re-orthogonalisation is for a new vector that lost
-// all but 1e-13 of its norm, which a solve meets at an exact breakdown if at
-// all; everything else is a few scalars, staged in shared memory.  It stands
-// for 3 l + 7 launches of 1.5 to 3 us each, most of them gated off.
-__global__ void __launch_bounds__(1024) k_gmres_finish(VecList V, double *vk, long long n,
-                                                       double *S, int l, int lmax, NkState *St,
-                                                       NkConds C) {
-  pdl_enter();
-  const GS g = gs_view(S, lmax);
-  double *sc = g.sc;
-  const int k = l + 1, t = threadIdx.x;
-  __shared__ double h[NK_MAX_KRYLOV + 1], giv[2 * NK_MAX_KRYLOV], red[32], coef;
-  __shared__ bool reorth, apply;
-  if (t < k) h[t] = g.H[t * lmax + k - 1];
-  if (t < 2 * l) giv[t] = g.giv[t];
-  double nn2 = 0.0;
-  if (t == 0) {
-    h[k] = sqrt(sc[SC_NEWNORM2]);
-    reorth = cancelled(sqrt(sc[SC_VKNORM2]), h[k]);
-  }
-  __syncthreads();
-  if (reorth) {
-    for (int i = 0; i < k; i++) {
-      const double *vi = V.v[i];
-      double acc = 0.0;
-      for (long long q = t; q < n; q += blockDim.x) acc = acc + vi[q] * vk[q];
+// Re-orthogonalisation of a long vector over the whole grid, as phases: phase p
+// takes product p - 1 off vk and sums its product with V[p], in chunks (items)
+// that any block may claim; the block that finishes a phase's last item adds the
+// partial sums in item order, takes ModifiedGS's decision (reorth_step) and
+// lets the next phase begin.  No block waits for one that is not running: an
+// unfinished item belongs to a block that has claimed it, so the launch needs
+// no co-residency.  Waits are bounded; a block that gives up writes 4 into the
+// error word and leaves.
+struct ReorthCtl {  // behind the scalars of S; zero between launches
+  unsigned next[NK_MAX_KRYLOV + 1], done[NK_MAX_KRYLOV + 1], ready[NK_MAX_KRYLOV + 1], left;
+  double coef[NK_MAX_KRYLOV + 1], nn2;
+};
+static_assert(sizeof(ReorthCtl) <= GS_REORTH_DOUBLES * sizeof(double), "its space in S");
+constexpr int FIN_THREADS = 512;
+constexpr unsigned long long FIN_WAIT_NS = 1000000000ull;  // 1 s
+
+__device__ __forceinline__ double block_sum(double a, double *red) {
+  const int t = threadIdx.x;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc = acc + __shfl_down_sync(0xffffffffu, acc, o);
-      if ((t & 31) == 0) red[t >> 5] = acc;
-      __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) a = a + __shfl_down_sync(0xffffffffu, a, o);
+  if ((t & 31) == 0) red[t >> 5] = a;
+  __syncthreads();
+  a = red[0];
+  for (int w = 1; w < FIN_THREADS / 32; w++) a = a + red[w];
+  __syncthreads();  // (red may be written again)
+  return a;
+}
+
+// true in the one block that leaves last, when everything is done
+__device__ bool reorthogonalise(const VecList &V, double *vk, long long n, unsigned items,
+                                long long chunk, double *partial, const GS &g, int k,
+                                ReorthCtl *ctl, int *kerr) {
+  const int t = threadIdx.x;
+  __shared__ double red[FIN_THREADS / 32], coef;
+  __shared__ unsigned word;
+  __shared__ bool gave_up;
+  for (int p = 0; p <= k; p++) {
+    double a = 0.0;  // coefficient of V[p - 1]
+    if (p > 0) {
       if (t == 0) {
-        double np = red[0];
-        for (int w = 1; w < (int)blockDim.x / 32; w++) np = np + red[w];
-        apply = reorth_step(np, h[i], nn2);
-        coef = -np;
+        gave_up = false;
+        unsigned long long since = 0;
+        for (unsigned it = 1; ld_acquire_gpu(&ctl->ready[p - 1]) == 0; it++) {
+          __nanosleep(64);
+          if (it % 64) continue;
+          const unsigned long long now = global_ns();
+          if (!since) since = now;
+          if (now - since > FIN_WAIT_NS || *(volatile int *)kerr) {
+            *(volatile int *)kerr = 4;
+            gave_up = true;
+            break;
+          }
+        }
+        coef = __ldcg(&ctl->coef[p - 1]);
       }
       __syncthreads();
-      if (apply)
-        for (long long q = t; q < n; q += blockDim.x) vk[q] = vk[q] + coef * vi[q];
+      if (gave_up) break;
+      a = coef;
+    }
+    if (p == k && a == 0.0) break;
+    const double *x = p > 0 ? V.v[p - 1] : nullptr, *z = p < k ? V.v[p] : nullptr;
+    for (;;) {
       __syncthreads();
+      if (t == 0) word = atomicAdd(&ctl->next[p], 1u);
+      __syncthreads();
+      const unsigned item = word;
+      if (item >= items) break;
+      const long long q0 = item * chunk, q1 = min(n, q0 + chunk);
+      double acc = 0.0;
+#pragma unroll 4
+      for (long long q = q0 + t; q < q1; q += FIN_THREADS) {
+        double y = __ldcg(vk + q);  // (another block's store of the phase before)
+        if (a != 0.0) {
+          y = y + a * x[q];
+          __stcg(vk + q, y);
+        }
+        if (z) acc = acc + z[q] * y;
+      }
+      const double sum = block_sum(acc, red);
+      if (t == 0) {
+        __stcg(partial + item, sum);
+        word = atom_add_acq_rel_gpu(&ctl->done[p], 1u);
+      }
+      __syncthreads();
+      if (word + 1 != items || !z) continue;
+      // the phase's last item
+      acc = 0.0;
+      for (unsigned q = t; q < items; q += FIN_THREADS) acc = acc + __ldcg(partial + q);
+      const double np = block_sum(acc, red);
+      if (t == 0) {
+        double *hp = g.H + p * g.lmax + k - 1, h = __ldcg(hp), nn2 = __ldcg(&ctl->nn2);
+        const bool apply = reorth_step(np, h, nn2);
+        __stcg(hp, h);
+        __stcg(&ctl->nn2, nn2);
+        __stcg(&ctl->coef[p], apply ? -np : 0.0);
+        atom_add_acq_rel_gpu(&ctl->ready[p], 1u);
+      }
     }
   }
+  __syncthreads();
+  if (t == 0) word = atom_add_acq_rel_gpu(&ctl->left, 1u);
+  __syncthreads();
+  return word + 1 == gridDim.x;
+}
+
+// End of GMRES iteration l in one launch, the projections and their dot
+// products done: one block stages a few scalars in shared memory and does them,
+// the others leave at once, unless ModifiedGS re-orthogonalises (iterativ.c:60-84),
+// which is for a new vector that lost all but 1e-13 of its norm: an exact
+// breakdown.  It stands for 3 l + 7 launches of 1.5 to 3 us each, most of
+// them gated off.
+__global__ void __launch_bounds__(FIN_THREADS) k_gmres_finish(
+    VecList V, double *vk, long long n, unsigned items, long long chunk, double *partial,
+    double *S, int l, int lmax, NkState *St, NkConds C, int *kerr) {
+  pdl_enter();
+  const GS g = gs_view(S, lmax);
+  const double *sc = g.sc;
+  const int k = l + 1, t = threadIdx.x;
+  __shared__ double h[NK_MAX_KRYLOV + 1], giv[2 * NK_MAX_KRYLOV];
+  double hk = sqrt(sc[SC_NEWNORM2]);
+  if (cancelled(sqrt(sc[SC_VKNORM2]), hk)) {
+    ReorthCtl *ctl = reinterpret_cast<ReorthCtl *>(g.sc + SCI_COUNT);
+    if (!reorthogonalise(V, vk, n, items, chunk, partial, g, k, ctl, kerr)) return;
+    const double nn2 = __ldcg(&ctl->nn2);
+    if (nn2 != 0.0) hk = reorth_norm(hk, nn2);
+    if (*(volatile int *)kerr) hk = nan("");
+    __syncthreads();
+    for (int q = t; q < (int)(sizeof(ReorthCtl) / 4); q += FIN_THREADS)
+      reinterpret_cast<unsigned *>(ctl)[q] = 0u;
+  } else if (blockIdx.x != 0) {
+    return;
+  }
+  if (t < k) h[t] = __ldcg(g.H + t * lmax + k - 1);
+  if (t < 2 * l) giv[t] = g.giv[t];
+  __syncthreads();
   if (t != 0) return;
-  if (nn2 != 0.0) h[k] = reorth_norm(h[k], nn2);
+  h[k] = hk;
   gmres_column(g, h, giv, l, St, C);
 }
 
@@ -1002,11 +1095,17 @@ void launch_gmres_mgs(double *const *V, int l, int lmax, long long n, double *S,
 }
 
 void launch_gmres_finish(double *const *V, int l, int lmax, long long n, double *S,
-                         cudaStream_t st, NkState *St, const NkConds *C) {
+                         double *partial, int *kerr, cudaStream_t st, NkState *St, const NkConds *C) {
   VecList L{};
   for (int k = 0; k <= l; k++) L.v[k] = V[k];
-  launch_pdl(k_gmres_finish, dim3(1), dim3(1024), st, L, V[l + 1], n, S, l, lmax, St,
-             C ? *C : NkConds{});
+  // a block per SM and two chunks for each, of 2048 cells (whole lines) and more
+  long long items = (n + 2047) / 2048;
+  if (items > 2 * 148) items = 2 * 148;
+  if (items < 1) items = 1;
+  const long long chunk = ((n + items - 1) / items + 15) / 16 * 16;
+  items = (n + chunk - 1) / chunk;
+  launch_pdl(k_gmres_finish, dim3((unsigned)((items + 1) / 2)), dim3(FIN_THREADS), st, L, V[l + 1],
+             n, (unsigned)items, chunk, partial, S, l, lmax, St, C ? *C : NkConds{}, kerr);
 }
 
 void launch_gmres_scalar(int op, double *S, int l, int lmax, cudaStream_t st) {

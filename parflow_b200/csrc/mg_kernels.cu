@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "gpu_wait.cuh"
 #include "mg_common.cuh"
 #include "pdl.cuh"
 #include "nk_control.h"
@@ -1144,25 +1145,9 @@ struct ClusterTeam {
 // A fence on both sides of the barrier orders one phase's global writes
 // before the next phase's plain loads on every SM.
 constexpr unsigned long long GRID_WAIT_NS = 1000000000ull;  // 1 s
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 __device__ __forceinline__ GridCtl &grid_ctl() {
   __shared__ GridCtl ctl;
   return ctl;
-}
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned atom_add_acq_rel_gpu(unsigned *p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v)
-               : "memory");
-  return old;
 }
 __device__ __forceinline__ void grid_barrier(const GridCtl &g) {
   __syncthreads();

@@ -102,9 +102,11 @@ void launch_nk_final(NkState *S, cudaStream_t st);
 // vector steps of the graph solve whose scalars live on the device
 // (krylov_kernels.cu)
 // the end of GMRES iteration l: norm of V[l + 1] and re-orthogonalisation, QR
-// update, residual estimate; St given: also the graph's control step
+// update, residual estimate; St given: also the graph's control step.  partial:
+// reduce_partials() doubles; kerr: error word of a wait that ran out (4)
 void launch_gmres_finish(double *const *V, int l, int lmax, long long n, double *S,
-                         cudaStream_t st, NkState *St = nullptr, const NkConds *C = nullptr);
+                         double *partial, int *kerr, cudaStream_t st, NkState *St = nullptr,
+                         const NkConds *C = nullptr);
 // the same with Gram-Schmidt itself, in one launch (gmres_mgs_fits(n))
 bool gmres_mgs_fits(long long n);
 void launch_gmres_mgs(double *const *V, int l, int lmax, long long n, double *S, cudaStream_t st,

@@ -272,7 +272,8 @@ static int check_kernel_error(pfgpu_handle *h) {
     const int code = *h->hkerr;
     *h->hkerr = 0;
     CK(cudaMemsetAsync(h->kerr, 0, sizeof(int), h->st));
-    set_err(code == 3 ? "a cooperative multigrid kernel gave up waiting at a grid barrier"
+    set_err(code == 4 ? "the re-orthogonalisation of a Krylov vector gave up waiting for its sums"
+            : code == 3 ? "a cooperative multigrid kernel gave up waiting at a grid barrier"
             : code == 2 ? "the wavefront smoother gave up waiting for a neighbouring plane"
                         : "a pipelined smoother kernel gave up waiting for its TMA copies");
     return PFGPU_ERR_CUDA;
@@ -795,7 +796,7 @@ static void orthogonalise(pfgpu_handle *h, int l, NkState *St, const NkConds *C)
     launch_axpy_dot(h->V[k], h->V[i], Hp(i, k - 1), -1.0, more ? h->V[i + 1] : nullptr, N,
                     more ? Hp(i + 1, k - 1) : sc + SCI_NEWNORM2, h->rb, h->st);
   }
-  launch_gmres_finish(h->V.data(), l, lmax, N, S, h->st, St, C);
+  launch_gmres_finish(h->V.data(), l, lmax, N, S, h->rb.partial, h->kerr, h->st, St, C);
   h->launches += k + 2;
 }
 

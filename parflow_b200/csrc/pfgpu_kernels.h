@@ -412,7 +412,11 @@ void launch_fill(double *x, double v, long long n, cudaStream_t st);
 enum { GM_START = 0, GM_QRSOL = 4, GM_RESTART = 6, GM_RESTART_INIT = 7 };
 enum { SCI_RNORM = 0, SCI_ROT, SCI_RHO, SCI_VKNORM2, SCI_NEWNORM2, SCI_HLL, SCI_BETA, SCI_QRFAIL,
        SCI_COUNT };
-inline long long gs_size(int lmax) { return (long long)(lmax + 1) * lmax + 2 * lmax + lmax + 1 + SCI_COUNT; }
+// ... and the re-orthogonalisation's words (ReorthCtl)
+constexpr int GS_REORTH_DOUBLES = 192;
+inline long long gs_size(int lmax) {
+  return (long long)(lmax + 1) * lmax + 2 * lmax + lmax + 1 + SCI_COUNT + GS_REORTH_DOUBLES;
+}
 inline long long gs_sc_offset(int lmax) { return (long long)(lmax + 1) * lmax + 2 * lmax + lmax + 1; }
 inline long long gs_yg_offset(int lmax) { return (long long)(lmax + 1) * lmax + 2 * lmax; }
 void launch_gmres_scalar(int op, double *S, int l, int lmax, cudaStream_t st);
