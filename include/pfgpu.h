@@ -458,7 +458,8 @@ int pfgpu_mg_levels(pfgpu_handle *h, int *levels, int *dims, int max_levels);
 
 /* Times one of the library's kernels on its own stream with CUDA events:
  * `reps` back-to-back launches on the handle's current state (after a solve
- * or pfgpu_pc_setup), average duration per launch in *ms, and the kernel's
+ * or pfgpu_pc_setup; at that call's pressure when the handle was given no
+ * other), average duration per launch in *ms, and the kernel's
  * algorithmic HBM bytes per launch (each distinct per-cell array it needs
  * counted once; uniform fields count zero) in *bytes.
  * kernel: 0 residual (with its van Genuchten pass), 1 Jacobian + PC matrix

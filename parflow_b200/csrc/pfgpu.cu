@@ -160,6 +160,7 @@ struct pfgpu_handle {
   double *p_old = nullptr, *s_old = nullptr;
   double *kr = nullptr, *dkr = nullptr, *sat = nullptr, *dsat = nullptr;
   const double *vg_for = nullptr;  // iterate the cached kr/dkr/S/dS belong to
+  bool has_pressure = false;       // u was given (else it is the zero of the creation)
   double *zface = nullptr;
   double *xcor = nullptr, *vtemp = nullptr;
   std::vector<double *> V;
@@ -303,6 +304,7 @@ static int dalloc(T **p, long long n) {
 // ParFlow-layout input (host or device) -> dense device array
 static int in_vec(pfgpu_handle *h, const double *src, double *dense) {
   if (h->vg_for == dense) h->vg_for = nullptr;
+  if (dense == h->u) h->has_pressure = true;
   if (is_device_ptr(src)) {
     launch_unpad(src, dense, h->nx, h->ny, h->nz, h->st);
   } else {
@@ -2086,7 +2088,7 @@ static int create_impl(pfgpu_handle *h) {
       if (dalloc(a, N)) return PFGPU_ERR_NOMEM;
     if (int rc = alloc_mg<double>(h, h->mgd)) return rc;
   }
-  CK(cudaMemsetAsync(h->u, 0, N * sizeof(double), h->st));
+  for (double *v : {h->u, h->p_old, h->s_old}) CK(cudaMemsetAsync(v, 0, N * sizeof(double), h->st));
   // device problem
   DevProblem &P = h->P;
   memset(&P, 0, sizeof(P));
@@ -2670,6 +2672,7 @@ int pfgpu_read_pfb(pfgpu_handle *h, int what, const char *path) {
   fclose(f);
   if (what == PFGPU_PFB_PRESSURE) {
     CK(cudaMemcpyAsync(h->u, h->vtemp, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+    h->has_pressure = true;
     if (h->vg_for == h->u) h->vg_for = nullptr;
     CK(cudaStreamSynchronize(h->st));
     return PFGPU_OK;
@@ -3233,6 +3236,7 @@ static int load_step_inputs(pfgpu_handle *h, const double *p_old, const double *
   if (in_vec(h, p_old, h->p_old) || in_vec(h, s_old, h->s_old)) return PFGPU_ERR_CUDA;
   if (p == p_old) {
     CK(cudaMemcpyAsync(h->u, h->p_old, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+    h->has_pressure = true;
     if (h->vg_for == h->u) h->vg_for = nullptr;
     return 0;
   }
@@ -3641,10 +3645,24 @@ int pfgpu_time_kernel(pfgpu_handle *h, int kernel, int reps, double *ms, double 
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   const double dt = 0.05;
+  // at the handle's pressure; at that of pfgpu_pc_setup, as its own old state,
+  // when none was ever given (at zero pressure the van Genuchten pass has
+  // nothing to evaluate)
+  double *u = h->u, *p_old = h->p_old, *s_old = h->s_old;
+  if (!h->has_pressure) {
+    u = p_old = h->unew;
+    s_old = h->vtemp;
+    launch_saturation(h->P, u, s_old, h->st);
+    h->launches++;
+  }
   auto one = [&]() {
     switch (kernel) {
-      case PFGPU_KERNEL_RESIDUAL: feval(h, h->u, dt, h->fval); break;
-      case PFGPU_KERNEL_JACOBIAN: assemble(h, h->u, dt, true, true); break;
+      case PFGPU_KERNEL_RESIDUAL:
+        vg_state(h, u, false);
+        launch_residual(h->P, u, p_old, s_old, h->kr, h->sat, dt, h->fval, h->st);
+        h->launches++;
+        break;
+      case PFGPU_KERNEL_JACOBIAN: assemble(h, u, dt, true, true); break;
       case PFGPU_KERNEL_MATVEC: matvec(h, h->pp, h->bb); break;
       case PFGPU_KERNEL_RB_SWEEP:  // the finest level's post-smoother as the V-cycle runs it
         if (h->mixed) {
