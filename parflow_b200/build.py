@@ -75,6 +75,28 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+CHECK_SRC = os.path.join(ROOT, "tests", "device", "arith_check.cu")
+CHECK_LIB = os.path.join(ROOT, "tests", "device", "libarith_check.so")
+
+
+def build_checks(force: bool = False) -> str:
+    """The device functions of csrc/pfgpu_device.cuh as a library of their own,
+    for the tests of their arithmetic (tests/test_gpu_arithmetic.py)."""
+    needs = [CHECK_SRC] + [d for d in deps() if not d.endswith(".cu")]
+    if not force and os.path.exists(CHECK_LIB) and \
+            all(os.path.getmtime(d) <= os.path.getmtime(CHECK_LIB) for d in needs):
+        return CHECK_LIB
+    tmp = CHECK_LIB + ".tmp"
+    subprocess.check_call([nvcc()] + ARCH + ["-O3", "-std=c++17", "-shared", "-cudart", "static",
+                                             "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+                                             "-I" + os.path.join(ROOT, "include"),
+                                             "-I" + os.path.join(HERE, "csrc"), CHECK_SRC,
+                                             "-o", tmp])
+    os.replace(tmp, CHECK_LIB)
+    return CHECK_LIB
+
+
 if __name__ == "__main__":
     build(force="--force" in sys.argv, verbose="-v" in sys.argv)
+    build_checks(force="--force" in sys.argv)
     print(LIB)

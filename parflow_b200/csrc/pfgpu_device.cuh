@@ -97,13 +97,17 @@ __device__ __forceinline__ void tfg_face_y(const DevProblem &P, int i, int j, do
   gc = 0.5 * (__ldg(P.tfg_yc + a) + (in ? __ldg(P.tfg_yc + a + P.nx) : g * 1.0));
 }
 
-// 1/x: the hardware's approximation (rcp.approx.ftz.f64, some 20 bits) and
-// Newton-Raphson steps y += y (1 - x y), each squaring the relative error; with
-// two within 2 ulp of the division at a third of its instructions.  a/b: one
-// step and one correction of the quotient, q += y (a - b q), whose error is the
-// product of q's and y's (some 2^-80) before it is rounded.  Operands outside
-// 2^-1000 .. 2^500 (rcp_far: zero, tiny, huge, infinite, NaN; also where a
-// product of two of them may overflow) take the division.
+// 1/x: the hardware's approximation (rcp.approx.ftz.f64, a relative error of some
+// 2^-20) and two Newton-Raphson steps y += y (1 - x y), each squaring the error:
+// within 1 ulp of the division at a third of its instructions.  a/b: one step
+// and Markstein's correction of the quotient, q += y (a - b q) (P. W. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, IBM
+// J. Res. Dev. 34, 1990), whose error before rounding is the product of q's and
+// y's, some 2^-76: within 1 ulp, and where a - b q falls below the normal range
+// (numerators near it) within what half a unit of the smallest subnormal in the
+// numerator makes.  For numerators and quotients that are finite.
+// Operands below 2^-999 and from 2^501 on (rcp_far: zero, tiny, huge, infinite,
+// NaN; also where a product of two of them may overflow) take the division.
 __device__ __forceinline__ bool rcp_far(double x) {
   return ((unsigned)__double2hiint(x) >> 20 & 0x7ffu) - 24u > 1499u;
 }
@@ -117,7 +121,8 @@ __device__ __forceinline__ double fast_rcp(double x) {
   const double y = rcp_step(x);
   return fma(fma(-x, y, 1.0), y, y);
 }
-// FP32 (the face terms of an FP32 Jacobian): 2^-111 .. 2^62
+// FP32 (the face terms of an FP32 Jacobian): the division below 2^-111 and from
+// 2^63 on; the approximation errs by 1 ulp and a step leaves its rounding
 __device__ __forceinline__ bool rcp_far(float x) {
   return ((unsigned)__float_as_int(x) >> 23 & 0xffu) - 16u > 173u;
 }
