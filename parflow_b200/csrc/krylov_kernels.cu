@@ -35,23 +35,9 @@ struct OpDot {
   __device__ static double comb(double x, double y) { return x + y; }
   __device__ static double init() { return 0.0; }
 };
-struct OpMaxAbs {
-  const double *a;
-  __device__ double operator()(long long i) const { return fabs(a[i]); }
-  __device__ static double comb(double x, double y) { return x > y ? x : y; }
-  __device__ static double init() { return 0.0; }
-};
 struct OpStep {  // |s| / (1/1 + |u|)  (KINScSteplength, kinsol.c:1490-1505)
   const double *s, *u;
   __device__ double operator()(long long i) const { return fabs(s[i] / (1.0 / 1.0 + fabs(u[i]))); }
-  __device__ static double comb(double x, double y) { return x > y ? x : y; }
-  __device__ static double init() { return 0.0; }
-};
-struct OpStepDiff {  // |a - b| / (1 + |a|)  (KINStop, kinsol.c:1541-1544)
-  const double *a, *b;
-  __device__ double operator()(long long i) const {
-    return fabs((a[i] - b[i]) / (1.0 / 1.0 + fabs(a[i])));
-  }
   __device__ static double comb(double x, double y) { return x > y ? x : y; }
   __device__ static double init() { return 0.0; }
 };
@@ -125,19 +111,10 @@ void launch_dot(const double *a, const double *b, long long n, double *dst, Redu
   OpDot op{a, b};
   reduce(op, n, dst, rb, st);
 }
-void launch_maxabs(const double *a, long long n, double *dst, ReduceBuf rb, cudaStream_t st) {
-  OpMaxAbs op{a};
-  reduce(op, n, dst, rb, st);
-}
 void launch_steplen(const double *s, const double *u, long long n, double *dst, ReduceBuf rb,
                     cudaStream_t st, const int *gate) {
   OpStep op{s, u};
   reduce(op, n, dst, rb, st, gate);
-}
-void launch_steplen_diff(const double *a, const double *b, long long n, double *dst,
-                         ReduceBuf rb, cudaStream_t st) {
-  OpStepDiff op{a, b};
-  reduce(op, n, dst, rb, st);
 }
 
 // ---- fused multi-value reductions ------------------------------------------
@@ -425,14 +402,6 @@ void launch_dq_finish(double *z, const double *fw, const double *f, const double
 }
 
 // ---- element-wise ---------------------------------------------------------
-__global__ void k_axpy_dev(double *__restrict__ y, const double *__restrict__ x,
-                           const double *__restrict__ s, double sign, long long n) {
-  pdl_enter();
-  double a = sign * (*s);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    y[i] = y[i] + a * x[i];
-}
 __global__ void k_axpby(double *__restrict__ y, const double *__restrict__ x, double a, double b,
                         long long n) {
   pdl_enter();
@@ -503,10 +472,6 @@ static inline int grid_for(long long n) {
   return (int)(b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16);
 }
 
-void launch_axpy_dev(double *y, const double *x, const double *s, double sign, long long n,
-                     cudaStream_t st) {
-  launch_pdl(k_axpy_dev, dim3(grid_for(n)), dim3(256), st, y, x, s, sign, n);
-}
 void launch_axpby(double *y, const double *x, double a, double b, long long n, cudaStream_t st) {
   launch_pdl(k_axpby, dim3(grid_for(n)), dim3(256), st, y, x, a, b, n);
 }

@@ -100,15 +100,6 @@ __device__ __forceinline__ void thread_ijk(int &i, int &j, int &k) {
   j = blockIdx.y * blockDim.y + threadIdx.y;
   k = blockIdx.z;
 }
-// the same with the block order along y and z reversed when flip is set:
-// consecutive sweeps over a level that alternate direction begin on the
-// planes the previous launch touched last, which are still in L2
-__device__ __forceinline__ void thread_ijk_flip(int &i, int &j, int &k, int flip) {
-  const int by = flip ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
-  i = blockIdx.x * blockDim.x + threadIdx.x;
-  j = by * blockDim.y + threadIdx.y;
-  k = flip ? gridDim.z - 1 - blockIdx.z : blockIdx.z;
-}
 // (i, j, k) of linear index t inside a level (32-bit; single-block loops)
 __device__ __forceinline__ void split_ijk(int t, int nx, int ny, int &i, int &j, int &k) {
   i = t % nx;
@@ -145,14 +136,6 @@ __device__ __forceinline__ void prolong_weights_cell(const MGLevel<T> &F, int i,
   weights_at(L, F.dir, i, j, k, w1, w2);
   F.p1[c] = w1;
   F.p2[c] = w2;
-}
-
-template <typename T>
-__global__ void k_prolong_weights(MGLevel<T> F) {
-  pdl_enter();
-  int i, j, k;
-  thread_ijk(i, j, k);
-  prolong_weights_cell(F, i, j, k);
 }
 
 // collapsed-stencil coarse operator (mg_semi.c:577-740), stored symmetric:
@@ -212,31 +195,6 @@ __device__ __forceinline__ void coarse_op_cell(const MGLevel<T> &F, const MGLeve
   const T p2_1 = vget(F.nx, F.ny, F.nz, (const T *)F.p2, i - ox, j - oy, k - oz);
   const T p1_2 = vget(F.nx, F.ny, F.nz, (const T *)F.p1, i + ox, j + oy, k + oz);
   const T p2_2 = vget(F.nx, F.ny, F.nz, (const T *)F.p2, i + ox, j + oy, k + oz);
-  coarse_op_core(F, C, ic, jc, kc, p2_1, p1_2, p2_2);
-}
-
-// weights and coarse operator of one level in one pass: the thread of
-// coarse point c computes the weights of fine points 2c-1 and 2c+1 itself
-// (the same arithmetic as prolong_weights_cell) and stores those of 2c+1,
-// so every fine point's weights are written once and the fine operator is
-// read in a single sweep
-template <typename T>
-__device__ __forceinline__ void setup_level_cell(const MGLevel<T> &F, const MGLevel<T> &C,
-                                                 int ic, int jc, int kc) {
-  if (ic >= C.nx || jc >= C.ny || kc >= C.nz) return;
-  const int d = F.dir;
-  const int ox = d == 0, oy = d == 1, oz = d == 2;
-  const int i = ox ? 2 * ic : ic, j = oy ? 2 * jc : jc, k = oz ? 2 * kc : kc;
-  LV<T> L = lv(F);
-  T p2_1 = T(0), p1_2 = T(0), p2_2 = T(0), w1;
-  if (inside(F.nx, F.ny, F.nz, i - ox, j - oy, k - oz))
-    weights_at(L, d, i - ox, j - oy, k - oz, w1, p2_1);
-  if (inside(F.nx, F.ny, F.nz, i + ox, j + oy, k + oz)) {
-    weights_at(L, d, i + ox, j + oy, k + oz, p1_2, p2_2);
-    const long long f = (i + ox) + (long long)F.nx * ((j + oy) + (long long)F.ny * (k + oz));
-    F.p1[f] = p1_2;
-    F.p2[f] = p2_2;
-  }
   coarse_op_core(F, C, ic, jc, kc, p2_1, p1_2, p2_2);
 }
 
@@ -302,11 +260,14 @@ __device__ __forceinline__ void gather7(const LV<T> &L, int i, int j, int k, T s
   st[6] = in ? L.au[c] : T(0);
 }
 
-// setup_level_cell with the coarsening direction D fixed at compile time and
-// every fine operand gathered up front (fine points 2c-1, 2c, 2c+1 along D;
-// the lower entry of 2c+2 is the upper entry of 2c+1 in symmetric storage).
-// Same operations in the same order as weights_at + coarse_op_core, so the
-// result is bitwise that of setup_level_cell.
+// Weights and coarse operator of one level in one pass: the thread of coarse
+// point c computes the weights of fine points 2c-1 and 2c+1 and stores those of
+// 2c+1, so every weight is written once and the fine operator is read in a
+// single sweep.  The coarsening direction D is fixed at compile time and every
+// fine operand gathered up front (fine points 2c-1, 2c, 2c+1 along D; the lower
+// entry of 2c+2 is the upper entry of 2c+1 in symmetric storage).  Same
+// operations in the same order as weights_at + coarse_op_core, so the result is
+// bitwise that of the generic tail setup (k_setup_tail).
 //
 // H (float only): the same thread also writes the scaled FP16 operator of
 // its fine points 2c and 2c+1 and the scaled weights q1(2c) = s_c,
@@ -421,14 +382,6 @@ __global__ void __launch_bounds__(256) k_setup_level(MGLevel<T> F, MGLevel<T> C)
   C.a[1][cc] = r.e;
   C.a[2][cc] = r.n;
   C.a[3][cc] = r.u;
-}
-
-template <typename T>
-__global__ void k_coarse_op(MGLevel<T> F, MGLevel<T> C) {
-  pdl_enter();
-  int i, j, k;
-  thread_ijk(i, j, k);
-  coarse_op_cell(F, C, i, j, k);
 }
 
 // one colour of red/black Gauss-Seidel; colour 0 = red = (i+j+k) odd
@@ -1564,16 +1517,6 @@ static inline Shape3 shape3(int nx, int ny, int nz) {
   return s;
 }
 
-template <typename T>
-void launch_mg_prolong_weights(const MGLevel<T> &F, cudaStream_t st) {
-  Shape3 g = shape3(F.nx, F.ny, F.nz);
-  launch_pdl(k_prolong_weights<T>, dim3(g.grid), dim3(g.block), st, F);
-}
-template <typename T>
-void launch_mg_coarse_op(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st) {
-  Shape3 g = shape3(C.nx, C.ny, C.nz);
-  launch_pdl(k_coarse_op<T>, dim3(g.grid), dim3(g.block), st, F, C);
-}
 template <typename T, bool H>
 static void setup_level_d(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st) {
   Shape3 g = shape3(C.nx, C.ny, C.nz);
@@ -2075,13 +2018,6 @@ __device__ __forceinline__ void h16_scale_cell(const MGLevel<float> &F, const MG
   }
 }
 
-__global__ void k_h16_scale(MGLevel<float> F, MGLevel<float> C, int has_coarse) {
-  pdl_enter();
-  int i, j, k;
-  thread_ijk(i, j, k);
-  h16_scale_cell(F, C, has_coarse, i, j, k);
-}
-
 __global__ void __launch_bounds__(512) k_h16_scale_tail(const MGLevel<float> *__restrict__ Ls,
                                                         int first, int nl) {
   pdl_enter();
@@ -2180,10 +2116,6 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
   }
 }
 
-void launch_h16_scale(const MGLevel<float> &F, const MGLevel<float> *C, cudaStream_t st) {
-  Shape3 g = shape3(F.nx, F.ny, F.nz);
-  launch_pdl(k_h16_scale, dim3(g.grid), dim3(g.block), st, F, C ? *C : F, C ? 1 : 0);
-}
 // the operators of all tail levels and their ghost columns in shared memory
 template <typename T>
 static size_t setup_tail_bytes(const MGLevel<T> *L, int first, int nl, long long *cells) {
@@ -2213,7 +2145,8 @@ int launch_setup_tail(const MGLevel<T> *L, const MGLevel<T> *levels_dev, int fir
                       levels_dev, first, nl, (int)cells);
     return first + 1 < nl ? 1 : 0;
   }
-  // tails that do not fit (a hierarchy cut short by MaxLevels)
+  // tails that do not fit: a hierarchy cut short by MaxLevels, or one whose ghost
+  // columns are as large as its levels (1x45x45 in FP64)
   int k = 0;
   if (first + 1 < nl) {
     launch_pdl(k_setup_tail<T>, dim3(1), dim3(512), st, levels_dev, first, nl);
@@ -2355,8 +2288,6 @@ void launch_convert(const TI *in, TO *out, long long n, cudaStream_t st, int fli
 }
 
 #define INST(T)                                                                              \
-  template void launch_mg_prolong_weights<T>(const MGLevel<T> &, cudaStream_t);               \
-  template void launch_mg_coarse_op<T>(const MGLevel<T> &, const MGLevel<T> &, cudaStream_t); \
   template void launch_mg_setup_level<T>(const MGLevel<T> &, const MGLevel<T> &, cudaStream_t, \
                                          bool);                                               \
   template int launch_mg_smooth<T>(const MGLevel<T> &, T *, const T *, int, int, double, T *,  \

@@ -181,24 +181,6 @@ __device__ __forceinline__ VG vg_at(const DevProblem &P, long long c) {
   return v;
 }
 
-// Saturation (pfsimulator/parflow_lib/problem_saturation.c:221-415)
-__device__ __forceinline__ double vg_sat(const DevProblem &P, double p, const VG &v) {
-  double m = 1.0 - (1.0 / v.n);
-  double s_dif = v.ssat - v.sres;
-  if (p >= 0.0) return P.vg_from_file ? v.ssat : s_dif + v.sres;
-  double head = fabs(p) / (P.density * P.gravity);
-  return s_dif / pow(1.0 + pow(v.alpha * head, v.n), m) + v.sres;
-}
-
-__device__ __forceinline__ double vg_dsat(const DevProblem &P, double p, const VG &v) {
-  double m = 1.0 - (1.0 / v.n);
-  double s_dif = v.ssat - v.sres;
-  if (p >= 0.0) return 0.0;
-  double head = fabs(p) / (P.density * P.gravity);
-  return (m * v.n * v.alpha * pow(v.alpha * head, (v.n - 1))) * s_dif /
-         (pow(1.0 + pow(v.alpha * head, v.n), m + 1));
-}
-
 // Relative permeability (pfsimulator/parflow_lib/problem_phase_rel_perm.c:788, :981)
 // table lookup at a pressure head >= 0: kr (der = 0) or the table's
 // derivative (der = 1) (VanGLookupSpline :265-355, linear :357-400, 718-758)
@@ -229,19 +211,6 @@ __device__ __forceinline__ double vg_kr(const DevProblem &P, double p, double al
   double ahnm1 = pow(alpha * head, n - 1);
   double t = 1.0 - ahnm1 / pow(opahn, m);
   return (t * t) / pow(opahn, m / 2);
-}
-
-__device__ __forceinline__ double vg_dkr(const DevProblem &P, double p, double alpha, double n) {
-  if (p >= 0.0) return 0.0;
-  double m = 1.0 - (1.0 / n);
-  double head = fabs(p) / (P.density * P.gravity);
-  double opahn = 1.0 + pow(alpha * head, n);
-  double ahnm1 = pow(alpha * head, n - 1);
-  double coeff = 1.0 - ahnm1 * pow(opahn, -m);
-  return 2.0 * (coeff / (pow(opahn, (m / 2)))) *
-             ((n - 1) * pow(alpha * head, n - 2) * alpha * pow(opahn, -m) -
-              ahnm1 * m * pow(opahn, -(m + 1)) * n * alpha * ahnm1) +
-         (coeff * coeff) * (m / 2) * pow(opahn, (-(m + 2) / 2)) * n * alpha * ahnm1;
 }
 
 // All four van Genuchten quantities of one cell from log(alpha h) and

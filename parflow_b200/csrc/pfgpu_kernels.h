@@ -185,10 +185,6 @@ template <typename T>
 void launch_rbr_wave(const MGLevel<T> &L, const WaveLevel &w, T *x, const T *b, int zero,
                      int *err, cudaStream_t st);
 
-template <typename T>
-void launch_mg_prolong_weights(const MGLevel<T> &F, cudaStream_t st);
-template <typename T>
-void launch_mg_coarse_op(const MGLevel<T> &F, const MGLevel<T> &C, cudaStream_t st);
 // prolongation weights of F and the coarse operator C in one launch
 // (h16: also the scaled FP16 operator of F and its scaled transfer weights)
 template <typename T>
@@ -243,10 +239,6 @@ bool mg_wants_red_init(const MGLevel<T> &L, int smoother, bool h16);
 template <typename T>
 void launch_mg_prolong_add(const MGLevel<T> &F, const MGLevel<T> &C, const T *ec, T *xf,
                            cudaStream_t st, int flip = 0, bool h16 = false, int black = 0);
-// scaled FP16 operator of level F from its FP32 operator and the diagonal of
-// the next coarser level C (null on the coarsest); sets *F.hflag when a
-// scaled diagonal is not +1 (the flag is cleared before the first level)
-void launch_h16_scale(const MGLevel<float> &F, const MGLevel<float> *C, cudaStream_t st);
 // levels `first` .. nl-1 of a V-cycle / of the setup in one single-block
 // kernel; levels_dev is a device copy of the level table.  With smem > 0
 // (tail_smem_bytes of those levels, at most TAIL_SMEM_MAX) the V-cycle tail
@@ -358,14 +350,9 @@ int reduce_partials();  // doubles the partial buffer must hold (multi-value red
 // dst = sum(a .* b); deterministic (fixed grid, fixed order)
 void launch_dot(const double *a, const double *b, long long n, double *dst, ReduceBuf rb,
                 cudaStream_t st);
-// dst = max |a|
-void launch_maxabs(const double *a, long long n, double *dst, ReduceBuf rb, cudaStream_t st);
 // dst = max |s| / (1 + |u|) (gate given: only when *gate is nonzero)
 void launch_steplen(const double *s, const double *u, long long n, double *dst, ReduceBuf rb,
                     cudaStream_t st, const int *gate = nullptr);
-// dst = max |a - b| / (1 + |a|)
-void launch_steplen_diff(const double *a, const double *b, long long n, double *dst,
-                         ReduceBuf rb, cudaStream_t st);
 // fused reductions (one pass each)
 void launch_mgs_first(const double *vk, const double *v0, long long n, double *d_vk2,
                       double *d_h0, ReduceBuf rb, cudaStream_t st);
@@ -379,9 +366,6 @@ void launch_step_norms(const double *f, long long n, double *d_f2, double *d_fma
                        cudaStream_t st);
 void launch_init_norms(const double *u, const double *f, long long n, double *d_u2,
                        double *d_fmax, double *d_f2, ReduceBuf rb, cudaStream_t st);
-// y = y + (sign * (*s)) * x
-void launch_axpy_dev(double *y, const double *x, const double *s, double sign, long long n,
-                     cudaStream_t st);
 // y = a*x + b*y (host scalars)
 void launch_axpby(double *y, const double *x, double a, double b, long long n, cudaStream_t st);
 // difference-quotient J v (KINSpgmrAtimesDQ): the sums and sigma into d[0..4],
