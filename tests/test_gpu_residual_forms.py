@@ -1,9 +1,9 @@
-"""The two launch forms of the residual kernel give the same F bit for bit:
-the gather form (the default: every cell evaluates all six of its faces) and
-the face-once form (PFGPU_RESIDUAL_FACE_ONCE=1: each interior face flux
-evaluated once, shared through shared memory within a tile and through a
-register between planes).  The form is chosen once per process, so each side
-runs in a child process.  The Jacobian launches follow the same switch: the
+"""The two launch forms of the residual kernel give the same F bit for bit: the
+gather form (every cell evaluates all six of its faces) and the march form (a
+warp walks up the planes of 31 columns, each face evaluated once, handed to its
+other cell by a shuffle or a register).  PFGPU_RESIDUAL_FACE_ONCE=0 / 1 forces
+one of them (unset, the size of the grid decides), once per process, so each
+side runs in a child process.  The Jacobian launches follow the same switch: the
 test compares J x and the preconditioner output M^-1 r too."""
 
 import json
@@ -51,10 +51,7 @@ json.dump(out, open(sys.argv[3], "w"))
 def _run(tmp_path, gather):
     path = str(tmp_path / ("gather.json" if gather else "once.json"))
     env = dict(os.environ)
-    if gather:
-        env.pop("PFGPU_RESIDUAL_FACE_ONCE", None)
-    else:
-        env["PFGPU_RESIDUAL_FACE_ONCE"] = "1"
+    env["PFGPU_RESIDUAL_FACE_ONCE"] = "0" if gather else "1"
     subprocess.run([sys.executable, "-c", CHILD, ROOT, json.dumps(NAMES), path], env=env,
                    check=True, timeout=600)
     return json.load(open(path))
