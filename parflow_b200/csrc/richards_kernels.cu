@@ -27,10 +27,13 @@ __device__ __forceinline__ bool launch_ijk(int nx, int ny, int nz, int &i, int &
 // dS/dp (problem_phase_rel_perm.c:1312-1361, problem_saturation.c:342-412).
 // The residual uses kr and S; the Jacobian at the same iterate reuses all four.
 // STEP: the iterate is formed here, pn = u + lam pp (lam from lam_p when
-// given), and written too.  Bound by the latency of its loads (28 % of the
-// issue slots used) over the chain of exponentials and logarithms that follows.
-// 512x512x50: 136 us (memory floor 79 us) against 192 with the logarithms and
-// powers of the reference one by one, a division per reciprocal and per n.
+// given), and written too.  Bound by FP64 arithmetic: two logarithms, two
+// exponentials and a square root per unsaturated cell (k_saturation, with the
+// same ones and half the bytes, takes 161 us of this pass's 190 at 512x512x50;
+// the memory floor is 97 us, 48 B per cell with a field of alpha).  The
+// reference's logarithms and powers one by one, a division per reciprocal and
+// per n, took 197 us there, and the trial step 43 us of its own; with the step
+// in it this pass takes 196.
 // q: 1/(rho g), and m = 1 - 1/n of a uniform n
 struct VGUniform {
   double inv_rg, m;
@@ -51,44 +54,23 @@ __device__ __forceinline__ VGAll vg_cell(const DevProblem &P, const VGUniform &q
   }
   return v;
 }
-// VEC: two cells per thread in 16-byte accesses (every pointer 16-byte
-// aligned), for fields of VG_VEC_CELLS and more: the pass waits on memory, and
-// two cells per thread keep more bytes in flight once the grid is many waves
-// deep.  256x256x50: 31.6 us against 33.7; 197x123x37, where half as many
-// threads leave a worse last wave: 10.1 us against 9.3.
-constexpr long long VG_VEC_CELLS = 2000000;
-template <bool STEP, bool VEC>
-__global__ void __launch_bounds__(256, VEC ? 4 : 5) k_vg_all(DevProblem P, VGUniform q,
+// Six blocks per SM against five: residual with this pass at 256x256x50 107.3 us
+// against 108.3, 512x512x50 380 against 385; two cells per thread in 16-byte
+// accesses 109.9 and 389 (times after a timestep: at zero pressure, where
+// nothing is evaluated, the wider accesses looked better).
+template <bool STEP>
+__global__ void __launch_bounds__(256, 6) k_vg_all(DevProblem P, VGUniform q,
                          const double *__restrict__ p, double *__restrict__ kr,
                          double *__restrict__ dkr, double *__restrict__ sat,
                          double *__restrict__ dsat, const double *__restrict__ pp,
                          const double *lam_p, double lam, double *__restrict__ pn) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long c = VEC ? 2 * t : t;
+  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= P.n) return;
   const VG vg = vg_at(P, c);  // (fields: older than the kernel before this one)
   pdl_enter();
-  const double a = STEP ? (lam_p ? *lam_p : lam) : 0.0;
-  if (VEC && c + 1 < P.n) {
-    double2 pc = reinterpret_cast<const double2 *>(p)[t];
-    if (STEP) {
-      if (a != 0.0) {
-        const double2 d = reinterpret_cast<const double2 *>(pp)[t];
-        pc.x = fma(a, d.x, pc.x);
-        pc.y = fma(a, d.y, pc.y);
-      }
-      reinterpret_cast<double2 *>(pn)[t] = pc;
-    }
-    const VGAll v = vg_cell(P, q, vg, pc.x),
-                w = vg_cell(P, q, vg_at(P, c + 1), pc.y);
-    reinterpret_cast<double2 *>(kr)[t] = make_double2(v.kr, w.kr);
-    reinterpret_cast<double2 *>(dkr)[t] = make_double2(v.dkr, w.dkr);
-    reinterpret_cast<double2 *>(sat)[t] = make_double2(v.s, w.s);
-    reinterpret_cast<double2 *>(dsat)[t] = make_double2(v.ds, w.ds);
-    return;
-  }
-  double pc = p[c];  // (VEC: the last cell of an odd count)
+  double pc = p[c];
   if (STEP) {
+    const double a = lam_p ? *lam_p : lam;
     if (a != 0.0) pc = fma(a, pp[c], pc);
     pn[c] = pc;
   }
@@ -1074,14 +1056,8 @@ template <bool STEP>
 static void vg_launch(const DevProblem &P, const double *p, double *kr, double *dkr, double *sat,
                       double *dsat, const double *pp, const double *lam_p, double lam, double *pn,
                       cudaStream_t st) {
-  const uintptr_t at = (uintptr_t)p | (uintptr_t)kr | (uintptr_t)dkr | (uintptr_t)sat |
-                       (uintptr_t)dsat | (uintptr_t)pp | (uintptr_t)pn;
-  if (P.n >= VG_VEC_CELLS && (at & 15) == 0)
-    launch_pdl(k_vg_all<STEP, true>, dim3(blocks_for((P.n + 1) / 2, 256)), dim3(256), st, P,
-               vg_uniform(P), p, kr, dkr, sat, dsat, pp, lam_p, lam, pn);
-  else
-    launch_pdl(k_vg_all<STEP, false>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P),
-               p, kr, dkr, sat, dsat, pp, lam_p, lam, pn);
+  launch_pdl(k_vg_all<STEP>, dim3(blocks_for(P.n, 256)), dim3(256), st, P, vg_uniform(P), p, kr,
+             dkr, sat, dsat, pp, lam_p, lam, pn);
 }
 void launch_vg_all(const DevProblem &P, const double *p, double *kr, double *dkr, double *sat,
                    double *dsat, cudaStream_t st) {

@@ -1,7 +1,7 @@
 """A timestep of two million cells and one (odd) on the forms that only grids of
-this size take: the trial step formed in the van Genuchten pass two cells per
-thread, march residual and Jacobian, residual and restriction in two launches on
-the finest levels.  Each runs in a child process with one form switched off; the
+this size take: march residual and Jacobian, with the trial step formed in the
+van Genuchten pass, residual and restriction in two launches on the finest
+levels.  Each runs in a child process with one form switched off; the
 pressures are the same bits, and the residual that ended the solve is that of
 the pressure it returned."""
 

@@ -70,9 +70,9 @@ def test_march_equals_gather(tmp_path):
 
 @pytest.mark.parametrize("bottom", (False, True))
 def test_paired_van_genuchten(bottom):
-    """Grids of 2 million cells and more take the van Genuchten pass two cells
-    per thread: its residual equals, bit for bit, that of a smaller grid with
-    the same planes, at either end of an odd number of cells."""
+    """The residual of a grid of 2 million cells equals, bit for bit, that of a
+    smaller grid with the same planes, at either end of an odd number of cells:
+    a van Genuchten pass whose form depends on the size or pairs cells shows."""
     import numpy as np
 
     from parflow_b200 import configs
