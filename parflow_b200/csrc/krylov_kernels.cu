@@ -875,11 +875,15 @@ __device__ bool reorthogonalise(const VecList &V, double *vk, long long n, unsig
 __global__ void __launch_bounds__(FIN_THREADS) k_gmres_finish(
     VecList V, double *vk, long long n, unsigned items, long long chunk, double *partial,
     double *S, int l, int lmax, NkState *St, NkConds C, int *kerr) {
-  pdl_enter();
   const GS g = gs_view(S, lmax);
   const double *sc = g.sc;
   const int k = l + 1, t = threadIdx.x;
   __shared__ double h[NK_MAX_KRYLOV + 1], giv[2 * NK_MAX_KRYLOV];
+  if (t < 2 * l) giv[t] = g.giv[t];  // (older than the kernel before this one)
+  pdl_enter();
+  // (the column is asked for together with the norms: one round trip)
+  const double *column = g.H + t * lmax + k - 1;
+  double ht = t < k ? __ldcg(column) : 0.0;
   double hk = sqrt(sc[SC_NEWNORM2]);
   if (cancelled(sqrt(sc[SC_VKNORM2]), hk)) {
     ReorthCtl *ctl = reinterpret_cast<ReorthCtl *>(g.sc + SCI_COUNT);
@@ -887,14 +891,14 @@ __global__ void __launch_bounds__(FIN_THREADS) k_gmres_finish(
     const double nn2 = __ldcg(&ctl->nn2);
     if (nn2 != 0.0) hk = reorth_norm(hk, nn2);
     if (*(volatile int *)kerr) hk = nan("");
+    if (t < k) ht = __ldcg(column);
     __syncthreads();
     for (int q = t; q < (int)(sizeof(ReorthCtl) / 4); q += FIN_THREADS)
       reinterpret_cast<unsigned *>(ctl)[q] = 0u;
   } else if (blockIdx.x != 0) {
     return;
   }
-  if (t < k) h[t] = __ldcg(g.H + t * lmax + k - 1);
-  if (t < 2 * l) giv[t] = g.giv[t];
+  if (t < k) h[t] = ht;
   __syncthreads();
   if (t != 0) return;
   h[k] = hk;
