@@ -27,13 +27,13 @@ __device__ __forceinline__ bool launch_ijk(int nx, int ny, int nz, int &i, int &
 // dS/dp (problem_phase_rel_perm.c:1312-1361, problem_saturation.c:342-412).
 // The residual uses kr and S; the Jacobian at the same iterate reuses all four.
 // STEP: the iterate is formed here, pn = u + lam pp (lam from lam_p when
-// given), and written too.  Bound by FP64 arithmetic: two logarithms, two
-// exponentials and a square root per unsaturated cell (k_saturation, with the
-// same ones and half the bytes, takes 161 us of this pass's 190 at 512x512x50;
-// the memory floor is 97 us, 48 B per cell with a field of alpha).  The
-// reference's logarithms and powers one by one, a division per reciprocal and
-// per n, took 197 us there, and the trial step 43 us of its own; with the step
-// in it this pass takes 196.
+// given), and written too.  Bound by instruction issue and FP64 arithmetic (84 %
+// of the slots, the FP64 pipe active 55 %): two logarithms, two exponentials and
+// a square root per unsaturated cell (k_saturation, with the same ones and half
+// the bytes, takes four fifths of the time).  512x512x50 after a timestep: 181
+// us (memory floor 97 us, 48 B per cell with a field of alpha), with the step 185;
+// the reference's logarithms and powers one by one, a division per reciprocal
+// and per n, took 191 us there, and the trial step 43 us of its own.
 // q: 1/(rho g), and m = 1 - 1/n of a uniform n
 struct VGUniform {
   double inv_rg, m;
@@ -290,7 +290,7 @@ __device__ __forceinline__ void residual_cell(const DevProblem &P, int i, int j,
 
 // Gather form: every cell evaluates all six of its face fluxes (a face shared
 // by two cells is evaluated by both, with the same operands in the same
-// order).  The default launch form.
+// order).
 template <bool SURF, bool VEL = false>
 __global__ void __launch_bounds__(256, 5) k_residual(DevProblem P, const double *__restrict__ p,
                            const double *__restrict__ p_old, const double *__restrict__ s_old,
@@ -359,15 +359,16 @@ __global__ void __launch_bounds__(256, 5) k_residual(DevProblem P, const double 
 // in a register as the lower one of the next plane: four faces per cell instead
 // of six and half the loads, with no barrier and no shared memory.  Every flux
 // is the same function of the same operands as in the gather form.
-// Bound by instruction issue (two thirds of the slots) and the latency its
-// occupancy leaves: the four faces are evaluated without a branch between them
-// and an inner cell meets one test for the boundary patches.  512x512x50: 211
-// us, 230 with a branch per face and per patch, gather form 311 (memory floor
-// 112 us, 56 B per cell).
-// Four blocks of 64 registers per SM; three (five) give 267 (250) us; with the
-// slopes of a terrain-following grid, which need more registers, three give 45
-// us at 256x256x20, four 51, gather 54.  Two rows per warp (3.6 faces per cell,
-// 96 registers) were slower than gather: 20 warps per SM hide too little.
+// Bound by instruction issue (62 % of the slots, 368 instructions per cell) and
+// the latency its occupancy leaves: the four faces are evaluated without a branch
+// between them and an inner cell meets one test for the boundary patches.
+// 512x512x50: 211 us, gather form 295 (memory floor 114 us, 56 B per cell).
+// Four blocks of 64 registers per SM: with the van Genuchten pass, 197x123x37
+// 33.9 us; three 36.8, five 41.4.  With the slopes of a terrain-following grid,
+// which need more registers, three give 52.5 us at 256x256x20, four 57.2, gather
+// 67.2.  Two rows per warp (3.6 faces per cell, 96 registers) were slower than
+// gather: 20 warps per SM hide too little.
+
 // a column's value of one plane
 struct MCell {
   double p, k, kr;
@@ -921,9 +922,10 @@ __global__ void __launch_bounds__(128, 8) k_jacobian(DevProblem P, const double 
 // The gather form converts every operand of every face to the face arithmetic
 // (103 conversions and reciprocals per cell on a pipe of 16 lanes), this one a
 // cell's values once per thread that needs them, and evaluates the four faces
-// without a branch between them.  512x512x50, FP32: 293 us against 449 (343
-// with the branches).  Blocks per SM, FP64 512x512x50 with the van Genuchten pass:
-// three (80 registers) 559 us, two (128) 588; 197x123x37 48.0 and 47.1.
+// without a branch between them.  512x512x50, FP32: 293 us against 439, FP64 474
+// against 519.  Blocks per SM in FP64, with the van Genuchten pass: three (80
+// registers) 512x512x50 640 us and 24x500x50 34.2; two (128) 622 and 41.1, whose
+// smaller waves leave more of the last one empty (2 % slower over 122 shapes).
 template <typename TJ, typename TP, bool SURF>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, sizeof(TJ) == 8 || SURF ? 3 : 4)
     k_jacobian_march(
