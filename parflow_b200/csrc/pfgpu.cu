@@ -1966,21 +1966,28 @@ static int mg_level0_on_grid(pfgpu_handle *h, MG<T> &mg) {
 
 // FullJacobian storage for a hierarchy: W S L on level 0, the S / L ghost
 // planes on every level, level 0 taken out of the fused / wavefront smoothers
-// and the single-block kernels (their kernels assume a symmetric operator)
+// and the single-block kernels (their kernels assume a symmetric operator).
+// W S L of level 0 switch the multigrid over, so they go in last: an allocation
+// that fails leaves the handle as it was.
 template <typename T>
 static int mg_enable_full(pfgpu_handle *h, MG<T> &mg) {
   const int nl = (int)mg.L.size();
   MGLevel<T> &L0 = mg.L[0];
-  if (!L0.lo[0])
-    for (int s = 0; s < 3; s++)
-      if (dalloc(&L0.lo[s], L0.n)) return PFGPU_ERR_NOMEM;
   for (int l = 0; l < nl; l++) {
     MGLevel<T> &L = mg.L[l];
-    if (!L.sg && (dalloc(&L.sg, (long long)L.nx * L.nz) || dalloc(&L.lg, (long long)L.nx * L.ny)))
+    if ((!L.sg && dalloc(&L.sg, (long long)L.nx * L.nz)) ||
+        (!L.lg && dalloc(&L.lg, (long long)L.nx * L.ny)))
       return PFGPU_ERR_NOMEM;
     CK(cudaMemset(L.sg, 0, (long long)L.nx * L.nz * sizeof(T)));
     CK(cudaMemset(L.lg, 0, (long long)L.nx * L.ny * sizeof(T)));
   }
+  T *lo[3] = {nullptr, nullptr, nullptr};
+  for (int s = 0; s < 3; s++)
+    if (dalloc(&lo[s], L0.n)) {
+      for (T *q : lo) cudaFree(q);
+      return PFGPU_ERR_NOMEM;
+    }
+  std::copy(lo, lo + 3, L0.lo);
   L0.zc = -1;
   return mg_level0_on_grid(h, mg);
 }

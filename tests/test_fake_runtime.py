@@ -18,9 +18,11 @@ RUNTIME = r"""
 #include <stdlib.h>
 #include <string.h>
 #include <stddef.h>
-int fake_fail_malloc, fake_mallocs, fake_frees;
+// fake_fail_after: allocations that still succeed (-1: all)
+int fake_fail_after = -1, fake_mallocs, fake_frees, fake_graphs;
 int cudaMalloc(void **p, size_t n) {
-  if (fake_fail_malloc) return 2;
+  if (fake_fail_after == 0) return 2;
+  if (fake_fail_after > 0) fake_fail_after--;
   fake_mallocs++;
   return (*p = calloc(1, n)) ? 0 : 2;
 }
@@ -37,8 +39,29 @@ int cudaGetDevice(int *d) { *d = 0; return 0; }
 int cudaPointerGetAttributes(void *a, const void *p) { return 1; }
 const char *cudaGetErrorString(int e) { return "fake"; }
 int cudaStreamCreateWithFlags(void **s, unsigned f) { *s = (void *)1; return 0; }
+int cudaStreamGetCaptureInfo_v2(void *s, int *st, unsigned long long *id, void **g, void **deps,
+                                size_t *n) {
+  *st = 1;
+  if (g) *g = (void *)1;
+  if (deps) *deps = NULL;
+  if (n) *n = 0;
+  return 0;
+}
 int cudaStreamEndCapture(void *s, void **g) { *g = (void *)1; return 0; }
-int cudaGraphInstantiate(void **e, void *g, unsigned long long f) { *e = (void *)1; return 0; }
+// (type, reserved, then of a conditional node: handle, type, size, bodies out)
+struct node { int type, reserved[3]; unsigned long long handle; int kind; unsigned size; void **out; };
+int cudaGraphAddNode(void **n, void *g, void *d, size_t nd, struct node *p) {
+  static void *body = (void *)1;
+  p->out = &body;
+  *n = (void *)1;
+  return 0;
+}
+int cudaGraphInstantiate(void **e, void *g, unsigned long long f) {
+  fake_graphs++;
+  *e = (void *)1;
+  return 0;
+}
+int cudaGraphExecDestroy(void *e) { fake_graphs--; return 0; }
 int cudaEventCreate(void **e) { *e = (void *)1; return 0; }
 int cudaOccupancyMaxPotentialClusterSize(int *n, const void *f, const void *c) { *n = 1; return 0; }
 int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *f, int t, size_t s,
@@ -77,25 +100,64 @@ def fake(tmp_path_factory):
     return lib
 
 
+def _count(fake, name):
+    return C.c_int.in_dll(fake, name).value
+
+
+def _fail_after(fake, n):
+    C.c_int.in_dll(fake, "fake_fail_after").value = n
+
+
+@pytest.fixture
+def handle(fake, monkeypatch):
+    """Makes a handle of a grid that is all tail."""
+    monkeypatch.setattr(L, "_lib", fake)
+
+    def make(precision):
+        return RichardsGPU(configs.box(nx=12, ny=10, nz=8, nsteps=1), precision=precision)
+
+    yield make
+    _fail_after(fake, -1)
+
+
 @pytest.mark.parametrize("precision, change", [("fp64", "max_iter"), ("mixed", "max_iter"),
                                                ("mixed16", "max_iter"), ("fp64", "full_jacobian")])
-def test_level_leaves_the_tail_without_memory(fake, monkeypatch, precision, change):
+def test_level_leaves_the_tail_without_memory(fake, handle, precision, change):
     """A grid that is all tail: MGSemi.MaxIter 2 and FullJacobian take level 0
     out of the single-block kernel.  The V-cycle graph of the moment points to
     that kernel's packed operators, so they must not be freed before it goes;
     a change that cannot allocate leaves them alone."""
-    monkeypatch.setattr(L, "_lib", fake)
-    g = RichardsGPU(configs.box(nx=12, ny=10, nz=8, nsteps=1), precision=precision)
-    count = lambda name: C.c_int.in_dll(fake, name).value
-    frees = count("fake_frees")
-    C.c_int.in_dll(fake, "fake_fail_malloc").value = 1
-    try:
-        if change == "max_iter":
-            assert fake.pfgpu_set_mg_max_iter(g.h, 2) == 0
-            assert fake.pfgpu_set_mg_max_iter(g.h, 1) == 0
-        else:  # its own arrays are missing: refused, nothing changed
-            assert fake.pfgpu_set_pc_matrix(g.h, 1) < 0
-        assert count("fake_frees") == frees
-    finally:
-        C.c_int.in_dll(fake, "fake_fail_malloc").value = 0
+    g = handle(precision)
+    frees = _count(fake, "fake_frees")
+    _fail_after(fake, 0)
+    if change == "max_iter":
+        assert fake.pfgpu_set_mg_max_iter(g.h, 2) == 0
+        assert fake.pfgpu_set_mg_max_iter(g.h, 1) == 0
+    else:  # its own arrays are missing: refused, nothing changed
+        assert fake.pfgpu_set_pc_matrix(g.h, 1) < 0
+    assert _count(fake, "fake_frees") == frees
+    _fail_after(fake, -1)
+    g.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_full_jacobian_allocates_all_or_nothing(fake, handle, precision):
+    """FullJacobian's arrays, with the allocator failing at each of them in
+    turn: the call is refused, a later one completes the set, and none leaks."""
+    live = lambda: _count(fake, "fake_mallocs") - _count(fake, "fake_frees")
+    before = live()
+    g = handle(precision)
+    assert fake.pfgpu_set_pc_matrix(g.h, 1) == 0
+    full = live() - before
+    needed = 3 + 2 * len(g.mg_levels())
+    g.close()
+    assert live() == before
+    for n in range(needed):
+        g = handle(precision)
+        _fail_after(fake, n)
+        assert fake.pfgpu_set_pc_matrix(g.h, 1) < 0
+        _fail_after(fake, -1)
+        assert fake.pfgpu_set_pc_matrix(g.h, 1) == 0
+        assert live() - before == full, n
         g.close()
+        assert live() == before
