@@ -1992,8 +1992,11 @@ static int mg_enable_full(pfgpu_handle *h, MG<T> &mg) {
   return mg_level0_on_grid(h, mg);
 }
 template <typename T>
-static int mg_disable_full(MG<T> &mg) {
+static int mg_disable_full(pfgpu_handle *h, MG<T> &mg) {
   MGLevel<T> &L0 = mg.L[0];
+  // (captured solves hold W S L, and would be found again by their key when
+  // FullJacobian returns with other buffers)
+  solve_graphs_forget(h);
   for (int s = 0; s < 3; s++) {
     cudaFree(L0.lo[s]);
     L0.lo[s] = nullptr;
@@ -3343,7 +3346,7 @@ int pfgpu_set_pc_matrix(pfgpu_handle *h, int type) {
     }
     rc = h->mixed ? mg_enable_full<float>(h, h->mgf) : mg_enable_full<double>(h, h->mgd);
   } else {
-    rc = h->mixed ? mg_disable_full<float>(h->mgf) : mg_disable_full<double>(h->mgd);
+    rc = h->mixed ? mg_disable_full<float>(h, h->mgf) : mg_disable_full<double>(h, h->mgd);
   }
   if (rc != PFGPU_OK) return rc;
   // the host-driven V-cycle graph holds the old level-0 path

@@ -161,3 +161,20 @@ def test_full_jacobian_allocates_all_or_nothing(fake, handle, precision):
         assert live() - before == full, n
         g.close()
         assert live() == before
+
+
+def test_captured_solves_go_with_the_arrays_they_hold(fake, handle):
+    """Back from FullJacobian the W, S and L of level 0 are freed: a solve
+    captured with them must not be kept for its return."""
+    base = _count(fake, "fake_graphs")
+    g = handle("fp64")
+    one = _count(fake, "fake_graphs") - base  # the V-cycle
+    stats = L.Stats()
+    for _ in range(2):
+        assert fake.pfgpu_set_pc_matrix(g.h, 1) == 0
+        fake.pfgpu_advance(g.h, C.c_double(0.1), 1, C.byref(stats))
+        assert _count(fake, "fake_graphs") - base == one + 1  # and the solve
+        assert fake.pfgpu_set_pc_matrix(g.h, 0) == 0
+        assert _count(fake, "fake_graphs") - base == one
+    g.close()
+    assert _count(fake, "fake_graphs") == base

@@ -111,3 +111,35 @@ def test_tail_setup_matches_oracle(solver, monkeypatch, shape):
     mg.setup(orc.jacobian(p, prob.dt, symm=1))
     want = mg.apply(r)
     assert np.abs(z - want).max() <= 1e-12 * np.abs(want).max()
+
+
+def test_full_jacobian_comes_and_goes(solver, monkeypatch):
+    """FullJacobian, back, and again: the second solve is not a captured one that
+    holds the first one's arrays; its pressures are a new handle's."""
+    for k in ENV:
+        monkeypatch.delenv(k, raising=False)
+    prob = configs.box(nx=20, ny=14, nz=9, nsteps=1)
+    t, dt = prob.time_plan()[0]
+    p0 = prob.initial_pressure()
+
+    def step(s):
+        s.set_time(t)
+        s.set_pressure(p0)
+        s.advance(1, dt)
+        return s.get_pressure()
+
+    s = solver.RichardsGPU(prob)
+    symmetric = step(s)
+    got = []
+    for _ in range(2):
+        assert s.lib.pfgpu_set_pc_matrix(s.h, 1) == 0
+        got.append(step(s))
+        assert s.lib.pfgpu_set_pc_matrix(s.h, 0) == 0
+        # (level 0 stays out of the tail: equal up to the V-cycle's rounding)
+        assert np.abs(step(s) - symmetric).max() <= 1e-9 * np.abs(symmetric).max()
+    s.close()
+    fresh = solver.RichardsGPU(prob)
+    assert fresh.lib.pfgpu_set_pc_matrix(fresh.h, 1) == 0
+    want = step(fresh)
+    fresh.close()
+    assert np.array_equal(got[0], want) and np.array_equal(got[1], want)
