@@ -434,7 +434,7 @@ __device__ __forceinline__ float ldro_h(const __half *p) {
 // EARLY: the operator, and b when b_early says that the kernel before this one
 // does not write it, are loaded ahead of the wait on that kernel.  On levels
 // whose blocks are all resident at once a sweep is a launch latency, and the
-// loads drop out of it (V-cycle of 64x64x32 in FP64: 103 us against 117); on
+// loads drop out of it (V-cycle of 64x64x32 in FP64: 116 us against 127); on
 // larger levels the loads kept in registers cost more than they hide (colour
 // sweep of 512x512x50, scaled FP16: 47 us against 31).
 template <typename T, bool H, bool EARLY>
@@ -781,7 +781,7 @@ __global__ void __launch_bounds__(256) k_mg_residual_pair(MGLevel<T> L, const T 
 // thread evaluates a residual at f or f+1; the f-1 one comes from the
 // neighbouring lane (D = x) or is evaluated too (half the threads).  With the
 // operators loaded ahead of the wait a level's leg is one launch shorter: V-cycle
-// of 64x64x32 (FP64) 117 us against 123.  On the finest level of 512x512x50 the
+// of 64x64x32 (FP64) 116 us against 124.  On the finest level of 512x512x50 the
 // second evaluation costs more than the stored residual: 107 us against 78.
 // init: the zero-guess red sweep x = b / a0 of the coarse level too.
 template <typename T, bool H, int D>

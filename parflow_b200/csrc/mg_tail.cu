@@ -22,9 +22,9 @@
 //    barriers over power-of-two groups of warps, __syncwarp once one warp is
 //    enough (levels of at most 64 cells, half of all levels).
 // The generic tail (k_vcycle_tail_smem: nine barriers of 1024 threads per level,
-// two level descriptors copied per thread and leg) took 82 us in FP64 at
-// 64x64x32 and 84 us with the scaled FP16 operator at 512x512x50; this one
-// takes 28 and 23 us.  V-cycle of a 12x10x8 grid, all tail: 33 us against 90.
+// two level descriptors copied per thread and leg) took 85 us in FP64 and 83 us
+// with the scaled FP16 operator at 512x512x50; this one takes 23.5 and 23 us.
+// V-cycle graph of a 12x10x8 grid, all tail: 43 us against 103.
 // Spreading levels of up to 8192 cells over a cluster of eight blocks (iterate
 // in distributed shared memory) did not pay: a phase cost 2000 cycles there
 // (470 of them the release / acquire barrier of 512-thread blocks, the rest

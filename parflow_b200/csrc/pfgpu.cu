@@ -98,9 +98,11 @@ struct MG {
 //                     shared memory (default 1024)
 //   PFGPU_TAIL_SMEM   0 runs the V-cycle tail from global memory
 //   PFGPU_FUSE_CELLS  grid levels at or below this many cells take residual
-//                     and restriction in one launch (default 400000: at
-//                     256x256x50 the V-cycle is 305 us there, 321 with none
-//                     and 311 with 1000000)
+//                     and restriction in one launch (default 2000000.  V-cycle
+//                     with 0, 400000, 2000000, 4000000, FP16 operator: 256x256x50
+//                     298, 287, 282, 283 us; 512x512x50 701, 691, 683, 687;
+//                     197x123x37 197, 182, 180, 180; FP64 256x256x50 437, 423,
+//                     415, 424)
 //   PFGPU_MID_CELLS   grid levels at or below this many cells run, with the
 //                     tail, inside one thread-block-cluster kernel (default 0:
 //                     none; on B200 each of its phases waits about as long on
@@ -1836,7 +1838,7 @@ static int alloc_mg(pfgpu_handle *h, MG<T> &mg) {
     }
   tail_form<T>(mg);
   if (tail_image_alloc<T>(h, mg)) return PFGPU_ERR_NOMEM;
-  mg.fuse_cells = env_ll("PFGPU_FUSE_CELLS", 400000);
+  mg.fuse_cells = env_ll("PFGPU_FUSE_CELLS", 2000000);
   mg.flip = env_ll("PFGPU_FLIP", 1) != 0;
   // middle levels: the grid levels at or below PFGPU_MID_CELLS cells just
   // above the tail, when the device can co-schedule a cluster for them
